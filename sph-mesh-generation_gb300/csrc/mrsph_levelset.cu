@@ -392,8 +392,8 @@ struct VmWarp {
   int c[3][32];
 };
 
-// Pass 2b, one warp per cut sub-cube: get_subvolume(0, 1/8, cor) (3D) or
-// get_face(0, 1/4, cor) (2D), geometry_calculator.cpp:450-570, in units of
+// Pass 2b of 2D levels, one warp per cut sub-square: get_face(0, 1/4, cor)
+// (3D: get_subvolume(0, 1/8, cor), k_vm_columns), geometry_calculator.cpp:450-570, in units of
 // 2^-23 of the cell, added to the cell's units.  Every partial volume of the
 // bisection is a multiple of 2^-23 (weights 8^-k or 4^-k, times 1/4, 1/2 or
 // 3/4 at the last level, k <= 7), so the FP64 sum is exact in any order and
@@ -558,6 +558,206 @@ __global__ void __launch_bounds__(128) k_vm_walk(const int* __restrict__ item_ce
   }
   for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(FULL, acc, o);
   if (lane == 0 && acc) atomicAdd(units + item_cell[it], acc);
+}
+
+// Pass 2b in 3D, one warp per cut sub-cube.  The bisection's result can be
+// read off its finest lattice, 64^3 leaves: a leaf counts 4 units (of 2^-23 of
+// the cell) when its eight corners are positive, 0 when they are negative and
+// 3, 2 or 1 by the sign of its corner sum when it is cut.  (A node with all
+// corners positive has only such leaves, midpoints of positive values being
+// positive, and likewise for negative ones.)  The refined values are the
+// trilinear interpolant of the root's corners, linear along a lattice line:
+// a line changes sign once, so its positive (and negative) leaves form an
+// interval that starts or ends at an end of the line, a column's full (and
+// empty) leaves are the intersection of its four lines' intervals, and the
+// corner sum, linear too, splits the column's leaves at one place.  With F
+// full, E empty, P leaves of positive and N of negative corner sum a column
+// counts 4 F + 3 (P - F) + (N - E) + 2 (64 - P - N) = F - E + P - N + 128, so
+// it costs one root per line and one for the sum instead of a visit of the
+// 8^6 tree's cut nodes (some 12,000 per sub-cube): 8.7 ms for the 517,000 cut
+// sub-cubes of the benchmark torus, where visiting the tree breadth-first by
+// one warp each took 46.2 ms.  Both are bound by FP32 and integer issue.  In
+// 2D a sub-square has 64 columns only and the walk (k_vm_walk) stays.
+//
+// Signs are those of the reference's FP64 refinement.  With M the largest
+// |corner| and u = 2^-24, the FP32 values of this kernel lie within 11 u M of
+// the exact interpolant (one rounding per corner, three interpolations of at
+// most 3 u M each), their sums of four within 60 u M, and the refinement's
+// FP64 values within 18 * 2^-53 M (three rounded midpoints in six levels).  A
+// line's lattice value beyond 16 u M = 2^-20 M, and a sum of four beyond
+// 2^-17 M (half the corner sum), therefore has the reference's sign.  Inside
+// that band the value is interpolated directly in FP64 (within 11 * 2^-53 M)
+// and decides beyond 2^-46 M (2^-44 M for the sum); inside that one the
+// column's leaves are refined along their paths as the reference does
+// (gc_path64).
+struct VmLine {
+  float a, e;   // values at the ends (z = 0, 64)
+  unsigned P;   // positive leaves: first | 64 - end << 16
+  unsigned N;   // negative leaves
+};
+
+// direct interpolation at (x, y, z) in units of 1/128 of the sub-cube
+__device__ __noinline__ double vm_point64(const double* c, int x, int y, int z) {
+  const double tx = x * 0x1p-7, ty = y * 0x1p-7, tz = z * 0x1p-7;
+  double v[4];
+  for (int q = 0; q < 4; q++) v[q] = c[q] + tx * (c[4 + q] - c[q]);
+  const double w0 = v[0] + ty * (v[2] - v[0]), w1 = v[1] + ty * (v[3] - v[1]);
+  return w0 + tz * (w1 - w0);
+}
+
+// A line (or, scaled by its four lines, a column's half corner sum) that FP32
+// cannot split: ends ga, ge, positions 0..last (in steps of 2/128 from z0/128),
+// f(k) its FP32 value, band th, exact(k) its FP64 value, band th64.  Returns
+// the last position with the sign of position 0 (last when none differs) and
+// that sign; ok = false when FP64 cannot decide either.
+template <class F32, class F64>
+__device__ __noinline__ int vm_split(F32 f, F64 exact, int guess, int last, float th, double th64, int& sign0,
+                                     bool& ok) {
+  auto sgn = [&](int k) -> int {
+    const float v = f(k);
+    if (fabsf(v) > th) return v > 0.f ? 1 : -1;
+    const double w = exact(k);
+    return fabs(w) > th64 ? (w > 0.0 ? 1 : -1) : 0;
+  };
+  sign0 = sgn(0);
+  const int s1 = sgn(last);
+  ok = sign0 != 0 && s1 != 0;
+  if (!ok || sign0 == s1) return last;
+  int k = max(0, min(guess, last - 1));
+  for (int it = 0; it < 8; it++) {  // the guess is off by one at most unless the line is nearly flat
+    const int s0 = k == 0 ? sign0 : sgn(k), sn = k + 1 == last ? s1 : sgn(k + 1);
+    if (s0 == 0 || sn == 0) break;
+    if (s0 == sign0 && sn == s1) return k;
+    if (s0 != sign0) k--;
+    else k++;
+    if (k < 0 || k >= last) break;
+  }
+  ok = false;
+  return last;
+}
+
+constexpr int kVmWarps = 4;  // sub-cubes per block
+__global__ void __launch_bounds__(32 * kVmWarps) k_vm_columns(const int* __restrict__ item_cell,
+                                                              const double* __restrict__ item_cor, long long nitem,
+                                                              unsigned* __restrict__ units) {
+  constexpr unsigned FULL = 0xffffffffu;
+  __shared__ double s_cor[kVmWarps][8];
+  const int wid = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const long long it = (long long)blockIdx.x * kVmWarps + wid;
+  if (it >= nitem) return;  // whole warps
+  double* cor = s_cor[wid];
+  if (lane < 8) cor[lane] = item_cor[it * 8 + lane];  // [x][y][z]
+  __syncwarp();
+  float c[8], M = 0.f;
+  for (int q = 0; q < 8; q++) {
+    c[q] = (float)cor[q];
+    M = fmaxf(M, fabsf(c[q]));
+  }
+  // M rounded up, so that the bands hold for the FP64 corners
+  M *= 1.000001f;
+  const float th = M * 0x1p-20f + 1.e-37f, thc = M * 0x1p-17f + 1.e-37f;
+  // (corners near FP32's smallest numbers: no FP64 decision, M being inexact)
+  const double th64 = M > 1.e-30f ? (double)M * 0x1p-46 : 1.e300, thc64 = M > 1.e-30f ? (double)M * 0x1p-44 : 1.e300;
+  // lane l: columns x = 2l, 2l + 1, lines x = 2l, 2l + 1, 2l + 2; per line the
+  // values at y = 0 and their change to y = 64, at both ends in z
+  float b0[3], d0[3], b1[3], d1[3];
+  for (int i = 0; i < 3; i++) {
+    const float tx = (float)(2 * lane + i) * 0x1p-6f;
+    const float v00 = fmaf(tx, c[4] - c[0], c[0]), v01 = fmaf(tx, c[5] - c[1], c[1]);
+    const float v10 = fmaf(tx, c[6] - c[2], c[2]), v11 = fmaf(tx, c[7] - c[3], c[3]);
+    b0[i] = v00; d0[i] = v10 - v00;
+    b1[i] = v01; d1[i] = v11 - v01;
+  }
+  VmLine prev[3];
+  unsigned prev_bad = 0;  // bit i: line i of the previous row is not decided
+  int acc = 0;
+  for (int y = 0; y <= 64; y++) {
+    const float ty = (float)y * 0x1p-6f;
+    VmLine cur[3];
+    unsigned bad = 0;
+#pragma unroll
+    for (int i = 0; i < 3; i++) {
+      const float a = fmaf(ty, d0[i], b0[i]), e = fmaf(ty, d1[i], b1[i]), g = e - a;
+      const bool cross = (a > 0.f) != (e > 0.f);
+      int k0 = min(max((int)__fdividef(-64.f * a, g), 0), 63);
+      const float fk = (float)k0 * 0x1p-6f;
+      const float f0 = cross ? fmaf(fk, g, a) : a, f1 = cross ? fmaf(fk + 0x1p-6f, g, a) : e;
+      int kk = cross ? k0 : 64;  // the last lattice point with the sign of the first
+      bool pos = a > 0.f;
+      if (!(fminf(fabsf(f0), fabsf(f1)) > th)) {
+        bool ok;
+        int s0;
+        const int x = 2 * lane + i;
+        kk = vm_split([&](int k) { return fmaf((float)k * 0x1p-6f, g, a); },
+                      [&](int k) { return vm_point64(cor, 2 * x, 2 * y, 2 * k); }, k0, 64, th, th64, s0, ok);
+        pos = s0 > 0;
+        if (!ok) bad |= 1u << i;
+      }
+      const unsigned w0 = (unsigned)(64 - kk) << 16, w1 = (unsigned)(kk + 1);
+      cur[i].a = a;
+      cur[i].e = e;
+      cur[i].P = pos ? w0 : w1;
+      cur[i].N = pos ? w1 : w0;
+    }
+    if (y > 0) {
+      bool exact[2];
+#pragma unroll
+      for (int i = 0; i < 2; i++) {
+        const unsigned P = __vmaxu2(__vmaxu2(prev[i].P, prev[i + 1].P), __vmaxu2(cur[i].P, cur[i + 1].P));
+        const unsigned N = __vmaxu2(__vmaxu2(prev[i].N, prev[i + 1].N), __vmaxu2(cur[i].N, cur[i + 1].N));
+        const int nf = max(0, 64 - (int)(P & 0xffffu) - (int)(P >> 16));
+        const int ne = max(0, 64 - (int)(N & 0xffffu) - (int)(N >> 16));
+        // half the corner sum of leaf k: the four lines at k + 1/2
+        const float A = (prev[i].a + prev[i + 1].a) + (cur[i].a + cur[i + 1].a);
+        const float E = (prev[i].e + prev[i + 1].e) + (cur[i].e + cur[i + 1].e);
+        const float g = E - A;
+        const float s0 = fmaf(0x1p-7f, g, A), s63 = fmaf(1.f - 0x1p-7f, g, A);
+        const bool cross = (s0 > 0.f) != (s63 > 0.f);
+        const int k0 = min(max((int)floorf(__fdividef(-64.f * A, g) - 0.5f), 0), 62);
+        const float fk = fmaf((float)k0, 0x1p-6f, 0x1p-7f);
+        const float f0 = cross ? fmaf(fk, g, A) : s0, f1 = cross ? fmaf(fk + 0x1p-6f, g, A) : s63;
+        int kk = cross ? k0 : 63;
+        bool pos = s0 > 0.f, ok = true;
+        exact[i] = (((bad | prev_bad) >> i) & 3u) != 0;
+        if (!exact[i] && !(fminf(fabsf(f0), fabsf(f1)) > thc)) {
+          int sg;
+          const int x = 2 * lane + i;
+          kk = vm_split([&](int k) { return fmaf(fmaf((float)k, 0x1p-6f, 0x1p-7f), g, A); },
+                        [&](int k) { return 4.0 * vm_point64(cor, 2 * x + 1, 2 * y - 1, 2 * k + 1); }, k0, 63, thc,
+                        thc64, sg, ok);
+          pos = sg > 0;
+          exact[i] = !ok;
+        }
+        const int diff = 2 * (kk + 1) - 64;
+        if (!exact[i]) acc += nf - ne + (pos ? diff : -diff) + 128;
+      }
+      // columns FP64 interpolation cannot decide either: the warp refines their
+      // leaves, two per lane, as the reference does
+      for (int i = 0; i < 2; i++) {
+        unsigned todo = __ballot_sync(FULL, exact[i]);
+        while (todo) {
+          const int x = 2 * (__ffs(todo) - 1) + i, yy = y - 1;
+          todo &= todo - 1u;
+          for (int k = lane; k < 64; k += 32) {
+            int path[6];
+            for (int l = 0; l < 6; l++)
+              path[l] = (((x >> (5 - l)) & 1) << 2) | (((yy >> (5 - l)) & 1) << 1) | ((k >> (5 - l)) & 1);
+            double leaf[8];
+            gc_path64<3>(cor, path, 6, leaf);
+            const int f = gc_mark(leaf, 8);
+            double cv = 0.0;
+            for (int q = 0; q < 8; q++) cv += leaf[q];
+            acc += f == 1 ? 4 : (f == 0 ? 0 : (cv > 0.0 ? 3 : (cv == 0.0 ? 2 : 1)));
+          }
+        }
+      }
+    }
+#pragma unroll
+    for (int i = 0; i < 3; i++) prev[i] = cur[i];
+    prev_bad = bad;
+  }
+  acc = __reduce_add_sync(FULL, acc);
+  if (lane == 0 && acc) atomicAdd(units + item_cell[it], (unsigned)acc);
 }
 
 // Polygonise_MQ::VertexInterp at isolevel 0 (polygonise.cpp:74-92), one axis
@@ -962,7 +1162,7 @@ cudaError_t ls_volume_mass(const LsSet& ls, int level, int D, double* cvol, doub
         (e = cudaStreamSynchronize(s)) == cudaSuccess) {
       if (ni > 0) {
         const long long nbi = ((long long)ni + 3) / 4;  // one warp per cut sub-cube
-        if (D == 3) k_vm_walk<3><<<(unsigned)nbi, 128, 0, s>>>(item_cell, item_cor, (long long)ni, units);
+        if (D == 3) k_vm_columns<<<(unsigned)nbi, 32 * kVmWarps, 0, s>>>(item_cell, item_cor, (long long)ni, units);
         else k_vm_walk<2><<<(unsigned)nbi, 128, 0, s>>>(item_cell, item_cor, (long long)ni, units);
       }
       k_vm_finish<<<(unsigned)((nl + 255) / 256), 256, 0, s>>>(list, nl, units, mark, dv, cvol);
