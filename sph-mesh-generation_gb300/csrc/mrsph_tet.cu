@@ -130,7 +130,7 @@ __device__ __noinline__ int orient_x(const Pt& a, const Pt& b, const Pt& c, cons
   const BI det = bi_add(bi_add(bi_mul(bi_from(adx), m1), bi_mul(bi_from(bdx), m2)), bi_mul(bi_from(cdx), m3));
   return bi_sign(det);
 }
-__device__ int orient3d(const Pt& a, const Pt& b, const Pt& c, const Pt& d, double ig) {
+__device__ __noinline__ int orient3d(const Pt& a, const Pt& b, const Pt& c, const Pt& d, double ig) {
   const double adx = a.x - d.x, ady = a.y - d.y, adz = a.z - d.z;
   const double bdx = b.x - d.x, bdy = b.y - d.y, bdz = b.z - d.z;
   const double cdx = c.x - d.x, cdy = c.y - d.y, cdz = c.z - d.z;
@@ -166,7 +166,7 @@ __device__ __noinline__ int insphere_x(const Pt& a, const Pt& b, const Pt& c, co
                         bi_sub(bi_mul(lift(bex, bey, bez), cda), bi_mul(lift(aex, aey, aez), bcd)));
   return bi_sign(det);
 }
-__device__ int insphere(const Pt& a, const Pt& b, const Pt& c, const Pt& d, const Pt& e, double ig) {
+__device__ __noinline__ int insphere(const Pt& a, const Pt& b, const Pt& c, const Pt& d, const Pt& e, double ig) {
   const double aex = a.x - e.x, aey = a.y - e.y, aez = a.z - e.z;
   const double bex = b.x - e.x, bey = b.y - e.y, bez = b.z - e.z;
   const double cex = c.x - e.x, cey = c.y - e.y, cez = c.z - e.z;
@@ -208,7 +208,7 @@ __device__ inline void cross3(const double* u, const double* v, double* w) {
 }
 __device__ inline double dot3(const double* u, const double* v) { return u[0] * v[0] + u[1] * v[1] + u[2] * v[2]; }
 
-__device__ void tet_geo(const Pt* P, TetGeo& g) {
+__device__ __noinline__ void tet_geo(const Pt* P, TetGeo& g) {
   const double* p3 = &P[3].x;
   for (int k = 0; k < 3; k++) {
     const double* pk = &P[k].x;
@@ -251,6 +251,7 @@ struct TetIn {
   const double* x;  // snapped positions (n x 3)
   const int* type;
   const double* h;
+  const float* rf;  // FP32 radius of the certificate ball, cutoff h (1 - 1e-6)
   const int* rows;  // n x cap ids (list order; self may appear)
   const int* cnt;
   double inv_g;  // 1 / grid
@@ -297,154 +298,235 @@ constexpr int kMaxOut = kMaxStar;  // tets emitted by one particle (at most its 
 
 constexpr unsigned kFull = 0xffffffffu;
 
-// FP32 pre-tests relative to particle i (w = d - x_i): they decide a
-// candidate only when the FP32 value clears a bound far above its rounding
-// error (and above the FP64 error of the circumcentre they use); the rest
-// go to the exact predicates, so every decision equals the exact one.
-struct Rel {
-  float x, y, z, n;  // w and |w|
+// ------------------------------------------------------------ FP32 geometry
+// The star is walked in FP32 relative to particle i (w = x_j - x_i, rounded
+// once, kept in shared memory for the whole star), with an error bound beside
+// every value: a decision is taken from FP32 only when it clears its bound, and
+// from the exact predicates otherwise, so every decision equals the exact one.
+// FP64 runs at 1/60 of the FP32 rate on this part: with the candidates' FP64
+// differences, an FP64 circumcentre per tet and a second scan of the row per
+// tet the pass took 142.9 ms for 150,001 particles (830,000 tets); in this
+// form it takes 7.5 ms, bound by instruction issue and latency.
+constexpr float kE = 0x1p-24f;
+constexpr int kRowS = 256;  // row entries kept in shared memory; longer rows read the rest from the positions
+
+struct V3 {
+  float x, y, z;
 };
-__device__ inline Rel rel(const Pt& p, const Pt& pi) {
-  const float x = (float)(p.x - pi.x), y = (float)(p.y - pi.y), z = (float)(p.z - pi.z);
-  return Rel{x, y, z, sqrtf(x * x + y * y + z * z)};
+__device__ inline V3 vcross(const V3& a, const V3& b) {
+  return V3{a.y * b.z - a.z * b.y, a.z * b.x - a.x * b.z, a.x * b.y - a.y * b.x};
 }
-// Centre c (relative to i) of the sphere through i, a, b, d, and whether it
-// is well enough conditioned (|det| >= 1e-3 |A||B||C|) for the pre-test.
-__device__ bool sphere_rel(const Pt& pi, const Pt& pa, const Pt& pb, const Pt& pd, float* c, float* cn) {
-  const double A[3] = {pa.x - pi.x, pa.y - pi.y, pa.z - pi.z}, B[3] = {pb.x - pi.x, pb.y - pi.y, pb.z - pi.z};
-  const double C[3] = {pd.x - pi.x, pd.y - pi.y, pd.z - pi.z};
-  double bc[3], ca[3], ab[3];
-  cross3(B, C, bc);
-  cross3(C, A, ca);
-  cross3(A, B, ab);
-  const double det = dot3(A, bc);
-  const double la = dot3(A, A), lb = dot3(B, B), lc = dot3(C, C);
-  if (!(fabs(det) >= 1.e-3 * sqrt(la) * sqrt(lb) * sqrt(lc))) return false;
-  double q = 0.0;
-  for (int k = 0; k < 3; k++) {
-    const double v = (la * bc[k] + lb * ca[k] + lc * ab[k]) / (2.0 * det);
-    c[k] = (float)v;
-    q += v * v;
+__device__ inline float vdot(const V3& a, const V3& b) { return fmaf(a.z, b.z, fmaf(a.y, b.y, a.x * b.x)); }
+
+struct Star {  // one warp's particle
+  float4 w[kRowS];  // (w, |w|); x is NaN for the particle itself
+  int tet[kMaxStar][3];  // row slots
+  float rc2[kMaxStar], band[kMaxStar];  // circumsphere diameter and its error bound
+  int le[kMaxLink][2];
+  unsigned char done[kMaxLink], cert[kMaxStar];
+};
+
+struct StarRow {
+  const TetIn& T;
+  const int* S;  // the row's ids
+  int i, m;
+  Pt pi;
+  const Star& sm;
+  __device__ float4 make(int q) const {
+    const int j = S[q];
+    const Pt p = load_pt(T, j);
+    const float x = (float)(p.x - pi.x), y = (float)(p.y - pi.y), z = (float)(p.z - pi.z);
+    return make_float4(j == i ? __int_as_float(0x7fffffff) : x, y, z, sqrtf(fmaf(z, z, fmaf(y, y, x * x))));
   }
-  *cn = (float)sqrt(q);
-  return true;
+  __device__ float4 at(int q) const { return q < kRowS ? sm.w[q] : make(q); }
+  __device__ Pt pt(int q) const { return load_pt(T, S[q]); }
+};
+
+// Orders floats as ints do (for __reduce_min_sync).
+__device__ inline int ford(float v) {
+  const int b = __float_as_int(v);
+  return b >= 0 ? b : b ^ 0x7fffffff;
 }
-// +1 inside, -1 outside, 0 undecided: the power |w|^2 - 2 w.c of a sphere
-// through i
-__device__ inline int power_test(const Rel& w, const float* c, float cn) {
-  const float p = w.n * w.n - 2.0f * (w.x * c[0] + w.y * c[1] + w.z * c[2]);
-  const float sl = 1.e-5f * (w.n * w.n + 2.0f * w.n * cn);
-  return p > sl ? -1 : (p < -sl ? 1 : 0);
+__device__ inline float funord(int b) { return __int_as_float(b >= 0 ? b : b ^ 0x7fffffff); }
+
+struct Face {  // the pencil of spheres through i, u, v: centres c0 + sigma t n
+  V3 n, c0;
+  float sigma, nn, cO, cP, dc0, L;  // |n|; bounds per |w| of n . w and of the power; of c0; |A| + |B|
+};
+// Bounds, with e = 2^-24, k = |A||B| / |n| and L = |A| + |B|: n is off by at most
+// 4 e |A||B|, c0 by 22 e k^2 L (its formula's rounding 14, the rounding of A and
+// B 8), n . w by 8 e |A||B||w|, the power |w|^2 - 2 w . c0 by e (8 |w|^2 + 48 k^2 L |w|).
+// The constants below are at least a third larger.
+__device__ inline Face face_of(const float4& A4, const float4& B4, float sigma) {
+  Face F;
+  const V3 A{A4.x, A4.y, A4.z}, B{B4.x, B4.y, B4.z};
+  F.n = vcross(A, B);
+  const float n2 = vdot(F.n, F.n), a2 = A4.w * A4.w, b2 = B4.w * B4.w;
+  const V3 p = vcross(B, F.n), q = vcross(F.n, A);
+  const float inv = 0.5f / n2;
+  F.c0 = V3{(a2 * p.x + b2 * q.x) * inv, (a2 * p.y + b2 * q.y) * inv, (a2 * p.z + b2 * q.z) * inv};
+  F.sigma = sigma;
+  F.nn = sqrtf(n2);
+  const float ab = A4.w * B4.w, k = ab / F.nn;
+  F.L = A4.w + B4.w;
+  F.cO = 16.f * kE * ab;
+  F.cP = 64.f * kE * k * k * F.L;
+  F.dc0 = 32.f * kE * k * k * F.L;
+  return F;
 }
 
-// Gift-wraps the face (i, a, b) to side s (s * orient3d(i, a, b, d) > 0),
-// one warp over the row: the candidate whose sphere through i, a, b holds
-// no other candidate.  Along the pencil of spheres through the face's
-// circle, "e inside the sphere of d" orders the candidates, so each lane
-// takes the first of its share and a shuffle reduction the first of all.
-// Returns -1 (on every lane) when no row particle lies on that side.
-__device__ int wrap(const TetIn& T, const int* S, int m, const Pt& pi, const Pt& pa, const Pt& pb, int i, int a,
-                    int b, int s, int lane) {
-  // orient3d(i, a, b, d) = -((a - i) x (b - i)) . (d - i)
-  float nf[3], nfn;
-  {
-    const double A[3] = {pa.x - pi.x, pa.y - pi.y, pa.z - pi.z}, B[3] = {pb.x - pi.x, pb.y - pi.y, pb.z - pi.z};
-    double n[3];
-    cross3(A, B, n);
-    nf[0] = (float)n[0]; nf[1] = (float)n[1]; nf[2] = (float)n[2];
-    nfn = (float)sqrt(dot3(n, n));
+struct Wrap {
+  int d;         // row slot of the winner, -1 when no row particle lies on the side
+  float t, et;   // its place on the pencil, and the bound
+  float o;       // sigma n . w
+  bool tie;      // another row particle lies on its sphere
+};
+
+// Gift-wraps the face (i, u, v) to side s (s * orient3d(i, u, v, d) > 0), one
+// warp over the row: the candidate whose sphere through i, u, v holds no other
+// candidate.  Along the pencil "e inside the sphere of d" is t_e < t_d, t =
+// power / (2 sigma n . w), so the winner is the smallest t.  FP32 gives each
+// candidate an interval; when only one reaches below the smallest upper end it
+// has won, else the exact insphere signs decide among those that do.
+__device__ Wrap wrap(const StarRow& R, const Face& F, int u, int v, int s, int lane) {
+  const float INF = __int_as_float(0x7f800000);
+  float lo1 = INF, lo2 = INF, H = INF;
+  int q1 = -1;
+  // interval of candidate q; false when it lies on the other side
+  auto interval = [&](int q, float& lo, float& hi) -> bool {
+    if (q == u || q == v) return false;
+    const float4 w = R.at(q);
+    const V3 w3{w.x, w.y, w.z};
+    const float o = F.sigma * vdot(F.n, w3), eo = F.cO * w.w;
+    if (!(o > -eo)) {
+      if (o <= -eo || w.x != w.x) return false;  // certainly beyond the face; the particle itself
+    }
+    if (!(o > 2.f * eo)) {
+      if (w.x != w.x) return false;
+      const Pt pu = R.pt(u), pv = R.pt(v), pd = R.pt(q);
+      if (s * orient3d(R.pi, pu, pv, pd, R.T.inv_g) <= 0) return false;
+      lo = -INF;
+      hi = INF;
+      return true;
+    }
+    const float n2 = w.w * w.w;
+    const float p = fmaf(-2.f, vdot(w3, F.c0), n2);
+    const float r = __fdividef(0.5f, o);
+    const float t = p * r;
+    const float et = 2.f * (fmaf(16.f * kE, n2, F.cP * w.w) * r + 2.f * fabsf(t) * eo * r) + 4.f * kE * fabsf(t);
+    lo = t - et;
+    hi = t + et;
+    if (!(lo <= hi)) { lo = -INF; hi = INF; }  // no usable bound (a face too thin for FP32)
+    return true;
+  };
+  for (int q = lane; q < R.m; q += 32) {
+    float lo, hi;
+    if (!interval(q, lo, hi)) continue;
+    if (q1 < 0 || lo < lo1) { lo2 = q1 < 0 ? INF : lo1; lo1 = lo; q1 = q; }
+    else lo2 = fminf(lo2, lo);
+    H = fminf(H, hi);
   }
-  int best = -1;
-  Pt pbest{0, 0, 0};
-  float c[3] = {0.f, 0.f, 0.f}, cn = 0.f;
-  bool hc = false;
-  for (int q = lane; q < m; q += 32) {
-    const int d = S[q];
-    if (d == i || d == a || d == b) continue;
-    const Pt pd = load_pt(T, d);
-    const Rel w = rel(pd, pi);
-    const float o = nf[0] * w.x + nf[1] * w.y + nf[2] * w.z, ob = 1.e-5f * nfn * w.n;
-    const int side = o > ob ? -1 : (o < -ob ? 1 : orient3d(pi, pa, pb, pd, T.inv_g));
-    if (s * side <= 0) continue;
-    bool take = best < 0;
-    if (!take) {
-      const int pt = hc ? power_test(w, c, cn) : 0;
-      take = pt != 0 ? pt > 0 : s * insphere(pi, pa, pb, pbest, pd, T.inv_g) > 0;
-    }
-    if (take) {
-      best = d;
-      pbest = pd;
-      hc = sphere_rel(pi, pa, pb, pd, c, &cn);
+  Wrap W;
+  W.tie = false;
+  const float Hm = funord(__reduce_min_sync(kFull, ford(H)));
+  const unsigned cand = __ballot_sync(kFull, q1 >= 0 && lo1 <= Hm);
+  const bool more = __any_sync(kFull, lo2 <= Hm && q1 >= 0 && lo2 < INF);
+  if (!cand) {
+    W.d = -1;
+    return W;
+  }
+  int best;
+  if (__popc(cand) == 1 && !more) {
+    best = __shfl_sync(kFull, q1, __ffs(cand) - 1);
+  } else {
+    // exact: every candidate that reaches below the smallest upper end, in row order
+    best = -1;
+    const Pt pu = R.pt(u), pv = R.pt(v);
+    for (int q0 = 0; q0 < R.m; q0 += 32) {
+      const int q = q0 + lane;
+      float lo = INF, hi;
+      bool in = q < R.m && interval(q, lo, hi);
+      in = in && lo <= Hm;
+      unsigned mask = __ballot_sync(kFull, in);
+      while (mask) {
+        const int d = q0 + __ffs(mask) - 1;
+        mask &= mask - 1u;
+        if (best < 0) {
+          best = d;
+          continue;
+        }
+        const int sg = s * insphere(R.pi, pu, pv, R.pt(best), R.pt(d), R.T.inv_g);
+        if (sg > 0) { best = d; W.tie = false; }
+        else if (sg == 0) W.tie = true;
+      }
     }
   }
-  // shuffle reduction; a lane whose partner lies past the warp gets its own
-  // candidate back, which is never compared with itself
-  for (int off = 16; off > 0; off >>= 1) {
-    const int ob = __shfl_down_sync(kFull, best, off);
-    const Pt po{__shfl_down_sync(kFull, pbest.x, off), __shfl_down_sync(kFull, pbest.y, off),
-                __shfl_down_sync(kFull, pbest.z, off)};
-    const float oc0 = __shfl_down_sync(kFull, c[0], off), oc1 = __shfl_down_sync(kFull, c[1], off);
-    const float oc2 = __shfl_down_sync(kFull, c[2], off), ocn = __shfl_down_sync(kFull, cn, off);
-    const bool ohc = __shfl_down_sync(kFull, (int)hc, off) != 0;
-    if (ob < 0 || ob == best) continue;
-    bool take = best < 0;
-    if (!take) {
-      const int pt = hc ? power_test(rel(po, pi), c, cn) : 0;
-      take = pt != 0 ? pt > 0 : s * insphere(pi, pa, pb, pbest, po, T.inv_g) > 0;
-    }
-    if (take) {
-      best = ob;
-      pbest = po;
-      c[0] = oc0; c[1] = oc1; c[2] = oc2; cn = ocn; hc = ohc;
-    }
-  }
-  return __shfl_sync(kFull, best, 0);
+  W.d = best;
+  const float4 w = R.at(best);
+  const V3 w3{w.x, w.y, w.z};
+  const float eo = F.cO * w.w, n2 = w.w * w.w;
+  W.o = F.sigma * vdot(F.n, w3);
+  const float r = __fdividef(0.5f, W.o);
+  W.t = fmaf(-2.f, vdot(w3, F.c0), n2) * r;
+  W.et = W.o > 2.f * eo
+             ? 2.f * (fmaf(16.f * kE, n2, F.cP * w.w) * r + 2.f * fabsf(W.t) * eo * r) + 4.f * kE * fabsf(W.t)
+             : INF;
+  return W;
 }
 
-// Status of tet (i, a, b, d) for particle i: 0 when a row particle lies
-// inside or on its sphere (or the four are coplanar), 1 when none does (a
-// tet of the row's Delaunay tetrahedralisation), 2 when moreover the sphere
-// lies inside i's ball and the tet is not flat (certified: a Delaunay tet
-// of all particles).  *degen is set when row particles lie on the sphere
-// and none inside it.  Warp-uniform result.
-__device__ int tet_status(const TetIn& T, const int* S, int m, int i, int a, int b, int d, const double* xi,
-                          double hi, bool* degen, int lane) {
-  int v[4] = {i, a, b, d};
-  sort4(v);
+// Whether the circumsphere of (i, u, v, d) lies inside i's ball and the tet is
+// not flat (certified: a Delaunay tet of all particles once its sphere is
+// empty); rc2, band: the sphere's diameter and its error bound.  All lanes
+// agree.  The sphere passes through i, so it lies inside the ball when its
+// diameter does not exceed the radius.  FP32 decides outside its bound, else
+// the canonical FP64 evaluation (tet_in_ball) that the emission uses as well.
+__device__ bool certified(const StarRow& R, const Face& F, const Wrap& W, int u, int v, float Ri, float& rc2,
+                          float& band) {
+  const float4 w = R.at(W.d);
+  const float tn = W.t * F.nn, c2 = vdot(F.c0, F.c0);
+  const float rc = sqrtf(fmaf(tn, tn, c2));
+  rc2 = 2.f * rc;
+  band = 2.f * (F.dc0 + F.nn * W.et + fabsf(W.t) * F.cO + 8.f * kE * rc) + 4.e-6f * Ri;
+  const float Lm = fmaxf(F.L, w.w);
+  const bool solid = W.o - F.cO * w.w > 1.e-5f * Lm * Lm * Lm;  // |det| above 1e-6 of the longest possible edge product
+  if (solid && rc2 + band < Ri) return true;
+  if (solid && rc2 - band > Ri) return false;
+  int id[4] = {R.i, R.S[u], R.S[v], R.S[W.d]};
+  sort4(id);
   Pt P[4];
-  for (int k = 0; k < 4; k++) P[k] = load_pt(T, v[k]);
+  for (int k = 0; k < 4; k++) P[k] = load_pt(R.T, id[k]);
   TetGeo g;
   tet_geo(P, g);
-  const int o = orient3d(P[0], P[1], P[2], P[3], T.inv_g);
-  if (o == 0) return 0;
-  // the sphere's centre relative to i (the pre-test needs |det| >= 1e-3 of the edge product)
-  const bool hc = fabs(g.det) >= 1.e-3 * g.vol_scale;
-  float c[3];
-  double cq = 0.0;
-  for (int k = 0; k < 3; k++) {
-    const double* p3 = &P[3].x;
-    const double v3 = p3[k] + g.c[k] - xi[k];
-    c[k] = (float)v3;
-    cq += v3 * v3;
-  }
-  const float cn = (float)sqrt(cq);
-  const Pt pi{xi[0], xi[1], xi[2]};
+  if (!solid) band = __int_as_float(0x7f800000);  // the emission decides in FP64 as well
+  const double xi[3] = {R.pi.x, R.pi.y, R.pi.z};
+  return tet_in_ball(g, P, xi, R.T.h[R.i], R.T.cutoff);
+}
+
+// No row particle inside or on the sphere of the star's first tet (i, u, v, d)
+// (the faces of later tets border an empty sphere, see k_tet_star); *degen is
+// set when row particles lie on it and none inside.
+__device__ bool first_empty(const StarRow& R, const Face& F, const Wrap& W, int u, int v, int s, bool* degen, int lane) {
+  const float st = F.sigma * W.t;
+  const V3 c{fmaf(st, F.n.x, F.c0.x), fmaf(st, F.n.y, F.c0.y), fmaf(st, F.n.z, F.c0.z)};
+  const float cn = sqrtf(vdot(c, c));
+  const float dc = F.dc0 + F.nn * W.et + fabsf(W.t) * F.cO + 8.f * kE * cn;
+  const Pt pu = R.pt(u), pv = R.pt(v), pd = R.pt(W.d);
   bool inside = false, on = false;
-  for (int q = lane; q < m && !inside; q += 32) {
-    const int e = S[q];
-    if (e == v[0] || e == v[1] || e == v[2] || e == v[3]) continue;
-    const Pt pe = load_pt(T, e);
-    const int pt = hc ? power_test(rel(pe, pi), c, cn) : 0;
-    const int sg = pt != 0 ? pt : o * insphere(P[0], P[1], P[2], P[3], pe, T.inv_g);
+  for (int q = lane; q < R.m && !inside; q += 32) {
+    if (q == u || q == v || q == W.d) continue;
+    const float4 w = R.at(q);
+    if (w.x != w.x) continue;
+    const V3 w3{w.x, w.y, w.z};
+    const float n2 = w.w * w.w, p = fmaf(-2.f, vdot(w3, c), n2);
+    const float e = 16.f * kE * n2 + 2.f * w.w * (dc + 8.f * kE * cn);
+    // insphere(i, u, v, d) is positive inside when orient3d(i, u, v, d) > 0, that is s > 0
+    const int sg = p > e ? -1 : (p < -e ? 1 : s * insphere(R.pi, pu, pv, pd, R.pt(q), R.T.inv_g));
     if (sg > 0) inside = true;
     else if (sg == 0) on = true;
   }
   const bool any_in = __any_sync(kFull, inside), any_on = __any_sync(kFull, on);
-  if (any_in || any_on) {
-    if (!any_in) *degen = true;
-    return 0;
-  }
-  return tet_in_ball(g, P, xi, hi, T.cutoff) ? 2 : 1;
+  if (any_on && !any_in) *degen = true;
+  return !any_in && !any_on;
 }
 
 constexpr int kStarWarps = 4;  // warps (particles) per block of k_tet_star
@@ -453,83 +535,127 @@ constexpr int kStarWarps = 4;  // warps (particles) per block of k_tet_star
 // emits (ascending ids, in star order) into out[i * kMaxOut ...], their
 // number into count[i].  stats: [0] open stars, [1] deleted tets, [2] ties,
 // [3] stars cut at the per-particle limits.
-__global__ void __launch_bounds__(32 * kStarWarps) k_tet_star(TetIn T, int* __restrict__ out,
+//
+// A tet's sphere is scanned for row particles only once, for the first tet.
+// Every later one is wrapped from a face of a tet whose sphere holds no row
+// particle inside or on it: on the far side of the face the new sphere lies
+// inside that one, on the near side no candidate lies inside the winner's, and
+// one lies on it exactly when the wrap saw a tie.
+//
+// Four blocks of four warps per SM (128 registers): 7.5 ms for 150,001
+// particles, 10.6 ms at six blocks (spills), 7.9 ms at three.
+__global__ void __launch_bounds__(32 * kStarWarps, 4) k_tet_star(TetIn T, int* __restrict__ out,
                                                               int* __restrict__ count, unsigned long long* stats,
                                                               unsigned* flags) {
-  __shared__ int s_star[kStarWarps][kMaxStar][3];
-  __shared__ int s_le[kStarWarps][kMaxLink][2];
-  __shared__ unsigned char s_done[kStarWarps][kMaxLink];
-  __shared__ unsigned char s_cert[kStarWarps][kMaxStar];
+  __shared__ Star s_star[kStarWarps];
   const int wib = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  int(*star)[3] = s_star[wib];
-  unsigned char* cert = s_cert[wib];
-  int(*le)[2] = s_le[wib];
-  unsigned char* ldone = s_done[wib];
+  Star& sm = s_star[wib];
   const long long nwarps = (long long)gridDim.x * kStarWarps;
   for (long long i64 = (long long)blockIdx.x * kStarWarps + wib; i64 < T.n; i64 += nwarps) {
     const int i = (int)i64;
-    const int* S = T.rows + i64 * T.cap;
-    const int m = T.cnt[i];
-    const Pt pi = load_pt(T, i);
-    const double xi[3] = {pi.x, pi.y, pi.z};
-    const double hi = T.h[i];
+    const StarRow R{T, T.rows + i64 * T.cap, i, T.cnt[i], load_pt(T, i), sm};
+    const int m = R.m;
+    const float Ri = T.rf[i];
     bool degen = false, open = false, trunc = false;
     int ns = 0, nl = 0;
+    for (int q = lane; q < min(m, kRowS); q += 32) sm.w[q] = R.make(q);
+    __syncwarp();
     // 1. nearest neighbour a (ties: lower id) and the third point c of the
-    // smallest circumcircle through i and a (ties: lower id)
-    double best = 1.e300;
-    int a = 0x7fffffff;
+    // smallest circumcircle through i and a (ties: lower id), by FP64
+    // values, which only the candidates near the FP32 minimum need
+    const float INF = __int_as_float(0x7f800000);
+    float dm = INF;
     for (int q = lane; q < m; q += 32) {
-      const int j = S[q];
-      if (j == i) continue;
+      const float4 w = R.at(q);
+      if (w.x == w.x) dm = fminf(dm, w.w);
+    }
+    dm = __int_as_float(__reduce_min_sync(kFull, __float_as_int(dm)));
+    double best = 1.e300;
+    int a = 0x7fffffff, qa = -1;
+    for (int q = lane; q < m; q += 32) {
+      const float4 w = R.at(q);
+      if (!(w.x == w.x) || w.w > dm * (1.f + 0x1p-18f)) continue;
+      const int j = R.S[q];
       const Pt pj = load_pt(T, j);
-      const double dx = pj.x - pi.x, dy = pj.y - pi.y, dz = pj.z - pi.z;
+      const double dx = pj.x - R.pi.x, dy = pj.y - R.pi.y, dz = pj.z - R.pi.z;
       const double d2 = dx * dx + dy * dy + dz * dz;
-      if (d2 < best || (d2 == best && j < a)) { a = j; best = d2; }
+      if (d2 < best || (d2 == best && j < a)) { a = j; best = d2; qa = q; }
     }
     for (int off = 16; off > 0; off >>= 1) {
       const double ob = __shfl_down_sync(kFull, best, off);
-      const int oa = __shfl_down_sync(kFull, a, off);
-      if (ob < best || (ob == best && oa < a)) { a = oa; best = ob; }
+      const int oa = __shfl_down_sync(kFull, a, off), oq = __shfl_down_sync(kFull, qa, off);
+      if (ob < best || (ob == best && oa < a)) { a = oa; best = ob; qa = oq; }
     }
-    a = __shfl_sync(kFull, a, 0);
-    int c = 0x7fffffff;
-    if (a != 0x7fffffff) {
-      const Pt pa = load_pt(T, a);
-      const double u[3] = {pa.x - pi.x, pa.y - pi.y, pa.z - pi.z};
+    qa = __shfl_sync(kFull, qa, 0);
+    int c = 0x7fffffff, qc = -1;
+    if (qa >= 0) {
+      const float4 u4 = R.at(qa);
+      const V3 u3{u4.x, u4.y, u4.z};
+      // squared circumradius |u|^2 |v|^2 |v - u|^2 / (4 |u x v|^2), at least a
+      // quarter of the longest edge's square; its relative error is below
+      // 40 e |u||v| / |u x v|
+      auto radius = [&](int q, float& lo, float& hi) -> bool {
+        if (q == qa) return false;
+        const float4 w = R.at(q);
+        if (w.x != w.x) return false;
+        const V3 v3{w.x, w.y, w.z}, d3{w.x - u4.x, w.y - u4.y, w.z - u4.z};
+        const V3 x = vcross(u3, v3);
+        const float xx = vdot(x, x), dd = vdot(d3, d3), vv = w.w * w.w, uu = u4.w * u4.w;
+        const float floor_ = 0.25f * fmaxf(vv, fmaxf(uu, dd)) * (1.f - 0x1p-16f);
+        const float r2 = uu * vv * dd / (4.f * xx), rel = 64.f * kE * u4.w * w.w / sqrtf(xx);
+        // |v - u| relative to its own rounding: d3 is off by at most 3 e (|u| + |v|)
+        const float rd = 8.f * kE * (u4.w + w.w) / sqrtf(dd);
+        const float er = rel + 2.f * rd;
+        if (!(er < 0.25f) || !(r2 < 3.e38f)) { lo = floor_; hi = INF; }
+        else { lo = fmaxf(r2 * (1.f - 2.f * er), floor_); hi = r2 * (1.f + 2.f * er); }
+        return true;
+      };
+      float H = INF;
+      for (int q = lane; q < m; q += 32) {
+        float lo, hi;
+        if (radius(q, lo, hi)) H = fminf(H, hi);
+      }
+      H = __int_as_float(__reduce_min_sync(kFull, __float_as_int(H)));
+      const Pt pa = R.pt(qa);
+      const double u[3] = {pa.x - R.pi.x, pa.y - R.pi.y, pa.z - R.pi.z};
       const double uu = dot3(u, u);
       double bestr = 1.e300;
       for (int q = lane; q < m; q += 32) {
-        const int j = S[q];
-        if (j == i || j == a) continue;
+        float lo, hi;
+        if (!radius(q, lo, hi) || lo > H) continue;
+        const int j = R.S[q];
         const Pt pj = load_pt(T, j);
-        const double v[3] = {pj.x - pi.x, pj.y - pi.y, pj.z - pi.z}, w[3] = {v[0] - u[0], v[1] - u[1], v[2] - u[2]};
+        const double v[3] = {pj.x - R.pi.x, pj.y - R.pi.y, pj.z - R.pi.z}, w[3] = {v[0] - u[0], v[1] - u[1], v[2] - u[2]};
         double x[3];
         cross3(u, v, x);
         const double xx = dot3(x, x);
         if (!(xx > 0.0)) continue;
         const double r2 = uu * dot3(v, v) * dot3(w, w) / (4.0 * xx);
-        if (r2 < bestr || (r2 == bestr && j < c)) { c = j; bestr = r2; }
+        if (r2 < bestr || (r2 == bestr && j < c)) { c = j; bestr = r2; qc = q; }
       }
       for (int off = 16; off > 0; off >>= 1) {
         const double ob = __shfl_down_sync(kFull, bestr, off);
-        const int oc = __shfl_down_sync(kFull, c, off);
-        if (ob < bestr || (ob == bestr && oc < c)) { c = oc; bestr = ob; }
+        const int oc = __shfl_down_sync(kFull, c, off), oq = __shfl_down_sync(kFull, qc, off);
+        if (ob < bestr || (ob == bestr && oc < c)) { c = oc; bestr = ob; qc = oq; }
       }
-      c = __shfl_sync(kFull, c, 0);
+      qc = __shfl_sync(kFull, qc, 0);
     }
     // 2. first tet: the face (i, a, c) wrapped to either side
-    if (c != 0x7fffffff) {
-      const Pt pa = load_pt(T, a), pc = load_pt(T, c);
+    if (qc >= 0) {
+      const float4 A = R.at(qa), B = R.at(qc);
       for (int s = 1; s >= -1 && ns == 0; s -= 2) {
-        const int d = wrap(T, S, m, pi, pa, pc, i, a, c, s, lane);
-        const int st = d >= 0 ? tet_status(T, S, m, i, a, c, d, xi, hi, &degen, lane) : 0;
-        if (st > 0) {
+        const Face F = face_of(A, B, (float)-s);  // orient3d(i, a, c, d) = -n . w
+        const Wrap W = wrap(R, F, qa, qc, s, lane);
+        if (W.d >= 0 && first_empty(R, F, W, qa, qc, s, &degen, lane)) {
+          float rc2, band;
+          const bool cert = certified(R, F, W, qa, qc, Ri, rc2, band);
           if (lane == 0) {
-            star[0][0] = s > 0 ? a : c;
-            star[0][1] = s > 0 ? c : a;
-            star[0][2] = d;
-            cert[0] = st == 2;
+            sm.tet[0][0] = s > 0 ? qa : qc;
+            sm.tet[0][1] = s > 0 ? qc : qa;
+            sm.tet[0][2] = W.d;
+            sm.cert[0] = cert;
+            sm.rc2[0] = rc2;
+            sm.band[0] = band;
           }
           ns = 1;
         }
@@ -542,58 +668,85 @@ __global__ void __launch_bounds__(32 * kStarWarps) k_tet_star(TetIn T, int* __re
     // whole star is reached): every tet (x, y, z) is stored with
     // orient3d(i, x, y, z) > 0; its link edges (x, y), (y, z), (z, x) lead
     // to the tets across the faces (i, x, y) ...  (warp-uniform; lane 0 writes)
-    int head = 0;
+    int head = 0, first = 0;  // first: no open link edge before it
     while (true) {
-      for (; head < ns; head++) {
+      for (; head < ns && !trunc; head++) {
+        const int t0 = sm.tet[head][0], t1 = sm.tet[head][1], t2 = sm.tet[head][2];
+        const int eu[3] = {t0, t1, t2}, ev[3] = {t1, t2, t0};
+        int at[3] = {-1, -1, -1};  // the tet's link edges already in the list
+        for (int q0 = 0; q0 < nl; q0 += 32) {
+          const int q = q0 + lane;
+          const int x = q < nl ? sm.le[q][0] : -1, y = q < nl ? sm.le[q][1] : -1;
+          for (int k = 0; k < 3; k++) {
+            const unsigned hit = __ballot_sync(kFull, (x == eu[k] && y == ev[k]) || (x == ev[k] && y == eu[k]));
+            if (hit && at[k] < 0) at[k] = q0 + __ffs(hit) - 1;
+          }
+        }
+        __syncwarp();
         for (int k = 0; k < 3; k++) {
-          const int u = star[head][k], v = star[head][(k + 1) % 3];
-          int f = -1;
-          for (int q = 0; q < nl; q++)
-            if ((le[q][0] == u && le[q][1] == v) || (le[q][0] == v && le[q][1] == u)) { f = q; break; }
-          if (f >= 0) {
-            if (lane == 0) ldone[f] = 1;
+          if (at[k] >= 0) {
+            if (lane == 0) sm.done[at[k]] = 1;
           } else if (nl < kMaxLink) {
-            if (lane == 0) { le[nl][0] = u; le[nl][1] = v; ldone[nl] = 0; }
+            if (lane == 0) { sm.le[nl][0] = eu[k]; sm.le[nl][1] = ev[k]; sm.done[nl] = 0; }
             nl++;
           } else {
             trunc = true;
           }
-          __syncwarp();
         }
+        __syncwarp();
       }
       if (trunc) break;
       int f = -1;
-      for (int q = 0; q < nl; q++)
-        if (!ldone[q]) { f = q; break; }
+      for (; first < nl; first += 32) {
+        const int q = first + lane;
+        const unsigned todo = __ballot_sync(kFull, q < nl && !sm.done[q]);
+        if (todo) { f = first + __ffs(todo) - 1; break; }
+        if (first + 32 > nl) break;  // edges appended later may land in this group
+      }
       if (f < 0) break;
-      const int u = le[f][0], v = le[f][1];
+      const int u = sm.le[f][0], v = sm.le[f][1];
       __syncwarp();
-      if (lane == 0) ldone[f] = 1;
+      if (lane == 0) sm.done[f] = 1;
       __syncwarp();
-      const Pt pu = load_pt(T, u), pv = load_pt(T, v);
       // the stored tet (u, v, w) has orient3d(i, u, v, w) > 0: wrap to the other side
-      const int d = wrap(T, S, m, pi, pu, pv, i, u, v, -1, lane);
-      const int st = d >= 0 ? tet_status(T, S, m, i, u, v, d, xi, hi, &degen, lane) : 0;
-      if (st == 0) {
+      const Face F = face_of(R.at(u), R.at(v), 1.f);
+      const Wrap W = wrap(R, F, u, v, -1, lane);
+      if (W.d >= 0 && W.tie) degen = true;
+      if (W.d < 0 || W.tie) {
         open = true;
         continue;
       }
+      const int d = W.d;
       bool dup = false;
-      for (int q = 0; q < ns && !dup; q++) {
-        const int* t = star[q];
-        const bool hu = t[0] == u || t[1] == u || t[2] == u, hv = t[0] == v || t[1] == v || t[2] == v;
-        const bool hd = t[0] == d || t[1] == d || t[2] == d;
-        dup = hu && hv && hd;
+      for (int q0 = 0; q0 < ns && !dup; q0 += 32) {
+        const int q = q0 + lane;
+        bool same = false;
+        if (q < ns) {
+          const int* t = sm.tet[q];
+          same = (t[0] == u || t[1] == u || t[2] == u) && (t[0] == v || t[1] == v || t[2] == v) &&
+                 (t[0] == d || t[1] == d || t[2] == d);
+        }
+        dup = __any_sync(kFull, same);
       }
       if (dup) continue;
       if (ns == kMaxStar) {
         trunc = true;
         break;
       }
-      if (lane == 0) { star[ns][0] = v; star[ns][1] = u; star[ns][2] = d; cert[ns] = st == 2; }  // orient3d(i, v, u, d) > 0
+      float rc2, band;
+      const bool cert = certified(R, F, W, u, v, Ri, rc2, band);
+      if (lane == 0) {  // orient3d(i, v, u, d) > 0
+        sm.tet[ns][0] = v;
+        sm.tet[ns][1] = u;
+        sm.tet[ns][2] = d;
+        sm.cert[ns] = cert;
+        sm.rc2[ns] = rc2;
+        sm.band[ns] = band;
+      }
       ns++;
       __syncwarp();
     }
+    __syncwarp();
     // 4. emit the tets whose lowest-id holding ball is i's (lanes over the
     // star, compacted in star order); apply the deletion rule
     int ne = 0;
@@ -602,24 +755,37 @@ __global__ void __launch_bounds__(32 * kStarWarps) k_tet_star(TetIn T, int* __re
       const int q = base + lane;
       bool emit = false, del = false;
       int v[4] = {0, 0, 0, 0};
-      if (q < ns && cert[q]) {
-        v[0] = i; v[1] = star[q][0]; v[2] = star[q][1]; v[3] = star[q][2];
+      if (q < ns && sm.cert[q]) {
+        v[0] = i; v[1] = R.S[sm.tet[q][0]]; v[2] = R.S[sm.tet[q][1]]; v[3] = R.S[sm.tet[q][2]];
         sort4(v);
-        Pt P[4];
-        for (int k = 0; k < 4; k++) P[k] = load_pt(T, v[k]);
-        TetGeo g;
-        tet_geo(P, g);
+        // every corner lies on the sphere, so its ball holds the sphere when
+        // the diameter is at most its radius
+        const float rc2 = sm.rc2[q], band = sm.band[q];
         int owner = -1;
-        for (int k = 0; k < 4 && owner < 0; k++) {
-          const double xv[3] = {P[k].x, P[k].y, P[k].z};
-          if (tet_in_ball(g, P, xv, T.h[v[k]], T.cutoff)) owner = v[k];
+        bool sure = band < INF;
+        for (int k = 0; k < 4 && owner < 0 && sure; k++) {
+          const float Rk = T.rf[v[k]];
+          if (v[k] == i || rc2 + band < Rk) owner = v[k];
+          else if (!(rc2 - band > Rk)) sure = false;
         }
-        if (owner == i) {
-          const bool all_boundary =
-              T.type[v[0]] != 0 && T.type[v[1]] != 0 && T.type[v[2]] != 0 && T.type[v[3]] != 0;
-          if (all_boundary && tet_aspect(g, P) > T.thres) del = true;
-          else emit = true;
+        bool all_boundary = false;
+        if (!sure || owner == i)
+          all_boundary = T.type[v[0]] != 0 && T.type[v[1]] != 0 && T.type[v[2]] != 0 && T.type[v[3]] != 0;
+        if (!sure || all_boundary) {
+          Pt P[4];
+          for (int k = 0; k < 4; k++) P[k] = load_pt(T, v[k]);
+          TetGeo g;
+          tet_geo(P, g);
+          if (!sure) {
+            owner = -1;
+            for (int k = 0; k < 4 && owner < 0; k++) {
+              const double xv[3] = {P[k].x, P[k].y, P[k].z};
+              if (tet_in_ball(g, P, xv, T.h[v[k]], T.cutoff)) owner = v[k];
+            }
+          }
+          if (owner == i) del = all_boundary && tet_aspect(g, P) > T.thres;
         }
+        emit = owner == i && !del;
       }
       const unsigned em = __ballot_sync(kFull, emit);
       ndel += __popc(__ballot_sync(kFull, del));
@@ -641,9 +807,12 @@ __global__ void __launch_bounds__(32 * kStarWarps) k_tet_star(TetIn T, int* __re
 }
 
 // Snap to the grid: x' = rint(x / g) g (g a power of two, |x / g| < 2^52).
-__global__ void k_tet_snap(long long n3, double* __restrict__ x, double inv_g, double g) {
+// Also the FP32 ball radii (the first n threads).
+__global__ void k_tet_snap(long long n, double* __restrict__ x, double inv_g, double g, const double* __restrict__ h,
+                           double cutoff, float* __restrict__ rf) {
   const long long k = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (k < n3) x[k] = rint(x[k] * inv_g) * g;
+  if (k < 3 * n) x[k] = rint(x[k] * inv_g) * g;
+  if (k < n) rf[k] = (float)(cutoff * h[k] * (1.0 - 1.e-6));
 }
 
 __global__ void k_tet_compact(long long n, const int* __restrict__ src, const int* __restrict__ count,
@@ -657,7 +826,8 @@ __global__ void k_tet_compact(long long n, const int* __restrict__ src, const in
 
 // ------------------------------------------------------------ quality
 struct TetStat {
-  double vol, vmin, vmax, emin2, emax2, amin, amax, asum, rmin, rmax, rsum, dmin, dmax, dsum;
+  double vol, vmin, vmax, emin2, emax2, amin, amax, asum, rmin, rmax, rsum, dsum;
+  double cdmin, cdmax;  // cosines of the smallest and the largest dihedral angle
 };
 struct TetQIn {
   const double* x;
@@ -667,11 +837,14 @@ struct TetQIn {
   const double* cos_small;  // cos(10, 20, 30, 40 degrees)
   unsigned long long* hist;  // aspect 12, radius 56, dihedral 45, small-dihedral 4
 };
+constexpr int kQualHist = 12 + 56 + 45 + 4;
 constexpr int kAspectBins = 12, kRadiusBins = 56, kDihedBins = 45;
 // degrees as the reference converts them: acos(x) / PI * 180 with its PI (glbparam.h:186)
 constexpr double kPiRef = 3.1415926;
 
-__device__ void tet_quality_one(const TetQIn& Q, long long t, TetStat& s) {
+__host__ __device__ inline double dihed_degrees(double c) { return acos(c) / kPiRef * 180.0; }
+
+__device__ void tet_quality_one(const TetQIn& Q, long long t, TetStat& s, unsigned* hist) {
   Pt P[4];
   for (int k = 0; k < 4; k++) {
     const double* p = Q.x + 3 * (long long)Q.tets[4 * t + k];
@@ -724,10 +897,10 @@ __device__ void tet_quality_one(const TetQIn& Q, long long t, TetStat& s) {
   const double tab[11] = {1.5, 2.0, 2.5, 3.0, 4.0, 6.0, 10.0, 15.0, 25.0, 50.0, 100.0};
   int ai = 0;
   while (ai < 11 && aspect > tab[ai]) ai++;
-  atomicAdd(&Q.hist[ai], 1ull);
+  atomicAdd(&hist[ai], 1u);
   const double rq = floor(ratio / 0.02);
   const int ri = rq >= 0.0 ? (rq < kRadiusBins - 1 ? (int)rq : kRadiusBins - 1) : 0;
-  atomicAdd(&Q.hist[kAspectBins + ri], 1ull);
+  atomicAdd(&hist[kAspectBins + ri], 1u);
   // dihedral angles at the six edges: cos = -n_a . n_b
   const int pa[6] = {0, 0, 0, 1, 1, 2}, pb[6] = {1, 2, 3, 2, 3, 3};
   double cmax = -2.0, cmin = 2.0;
@@ -736,51 +909,73 @@ __device__ void tet_quality_one(const TetQIn& Q, long long t, TetStat& s) {
     cs = fmin(1.0, fmax(-1.0, cs));
     cmax = fmax(cmax, cs);  // smallest angle
     cmin = fmin(cmin, cs);  // largest angle
-    int b = 0;
+    // the bin is the number of table cosines at or above cs: an FP32 angle is
+    // within one bin, the FP64 comparisons settle it
+    int b = min(max((int)(acosf((float)cs) * (45.f / 3.14159265f)), 0), kDihedBins - 1);
     while (b < kDihedBins - 1 && cs <= Q.cos_dihed[b + 1]) b++;
-    atomicAdd(&Q.hist[kAspectBins + kRadiusBins + b], 1ull);
+    while (b > 0 && !(cs <= Q.cos_dihed[b])) b--;
+    atomicAdd(&hist[kAspectBins + kRadiusBins + b], 1u);
   }
   for (int k = 0; k < 4; k++)
-    if (cmax > Q.cos_small[k]) atomicAdd(&Q.hist[kAspectBins + kRadiusBins + kDihedBins + k], 1ull);
-  const double dsmall = acos(cmax) / kPiRef * 180.0, dbig = acos(cmin) / kPiRef * 180.0;
-  s.dmin = fmin(s.dmin, dsmall);
-  s.dmax = fmax(s.dmax, dbig);
-  s.dsum += dsmall;
+    if (cmax > Q.cos_small[k]) atomicAdd(&hist[kAspectBins + kRadiusBins + kDihedBins + k], 1u);
+  s.cdmin = fmax(s.cdmin, cmax);
+  s.cdmax = fmin(s.cdmax, cmin);
+  s.dsum += dihed_degrees(cmax);
 }
 
 __device__ inline void stat_init(TetStat& s) {
   s.vol = s.asum = s.rsum = s.dsum = 0.0;
-  s.vmin = s.emin2 = s.amin = s.rmin = s.dmin = 1.e300;
-  s.vmax = s.emax2 = s.amax = s.rmax = s.dmax = 0.0;
+  s.vmin = s.emin2 = s.amin = s.rmin = 1.e300;
+  s.vmax = s.emax2 = s.amax = s.rmax = 0.0;
+  s.cdmin = -2.0;
+  s.cdmax = 2.0;
 }
 __device__ inline void stat_fold(TetStat& a, const TetStat& b) {
   a.vol += b.vol; a.asum += b.asum; a.rsum += b.rsum; a.dsum += b.dsum;
   a.vmin = fmin(a.vmin, b.vmin); a.emin2 = fmin(a.emin2, b.emin2); a.amin = fmin(a.amin, b.amin);
-  a.rmin = fmin(a.rmin, b.rmin); a.dmin = fmin(a.dmin, b.dmin);
+  a.rmin = fmin(a.rmin, b.rmin); a.cdmin = fmax(a.cdmin, b.cdmin);
   a.vmax = fmax(a.vmax, b.vmax); a.emax2 = fmax(a.emax2, b.emax2); a.amax = fmax(a.amax, b.amax);
-  a.rmax = fmax(a.rmax, b.rmax); a.dmax = fmax(a.dmax, b.dmax);
+  a.rmax = fmax(a.rmax, b.rmax); a.cdmax = fmin(a.cdmax, b.cdmax);
 }
 
-// 256 threads, one partial per block folded in thread order (deterministic)
+// 256 threads, one partial per block folded in a fixed order (deterministic).
+// The histograms are counted in shared memory and added once per block: on
+// global memory every tet's nine counts met on a few dozen words.  With that, the
+// search for a dihedral's bin from an FP32 angle and the extreme angles kept
+// as cosines, 830,000 tets take 1.07 ms instead of 1.78; FP64 divisions and
+// square roots bound it.
 __global__ void __launch_bounds__(256) k_tet_quality(TetQIn Q, TetStat* part) {
   __shared__ TetStat sh[256];
+  __shared__ unsigned s_hist[kQualHist];
+  for (int b = threadIdx.x; b < kQualHist; b += blockDim.x) s_hist[b] = 0u;
+  __syncthreads();
   const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   TetStat s;
   stat_init(s);
-  if (t < Q.ntet) tet_quality_one(Q, t, s);
+  if (t < Q.ntet) tet_quality_one(Q, t, s, s_hist);
   sh[threadIdx.x] = s;
   __syncthreads();
+  for (int b = threadIdx.x; b < kQualHist; b += blockDim.x)
+    if (s_hist[b]) atomicAdd(&Q.hist[b], (unsigned long long)s_hist[b]);
   for (int w = 128; w > 0; w >>= 1) {
     if ((int)threadIdx.x < w) stat_fold(sh[threadIdx.x], sh[threadIdx.x + w]);
     __syncthreads();
   }
   if (threadIdx.x == 0) part[blockIdx.x] = sh[0];
 }
-__global__ void k_tet_quality_fold(const TetStat* part, int nblk, TetStat* out) {
+// one block over the partials, in a fixed order (one thread took 2.70 ms for 3,244)
+__global__ void __launch_bounds__(256) k_tet_quality_fold(const TetStat* part, int nblk, TetStat* out) {
+  __shared__ TetStat sh[256];
   TetStat s;
   stat_init(s);
-  for (int b = 0; b < nblk; b++) stat_fold(s, part[b]);
-  *out = s;
+  for (int b = threadIdx.x; b < nblk; b += blockDim.x) stat_fold(s, part[b]);
+  sh[threadIdx.x] = s;
+  __syncthreads();
+  for (int w = 128; w > 0; w >>= 1) {
+    if ((int)threadIdx.x < w) stat_fold(sh[threadIdx.x], sh[threadIdx.x + w]);
+    __syncthreads();
+  }
+  if (threadIdx.x == 0) *out = sh[0];
 }
 
 int tfail(mrsph_handle* h, int code, const std::string& m) {
@@ -819,6 +1014,7 @@ extern "C" int mrsph_tetrahedralize(mrsph_handle* h, int* tets, long long cap, l
   e += 1;
   const double g = std::ldexp(1.0, e - 52), inv_g = std::ldexp(1.0, 52 - e);
   double *d_x = nullptr, *d_phi = nullptr, *d_h = nullptr, *d_cos = nullptr;
+  float* d_rf = nullptr;
   int *d_type = nullptr, *d_rows = nullptr, *d_cnt = nullptr, *d_out = nullptr, *d_count = nullptr;
   int *d_off = nullptr, *d_blk = nullptr, *d_tets = nullptr;
   unsigned* d_flags = nullptr;
@@ -836,7 +1032,7 @@ extern "C" int mrsph_tetrahedralize(mrsph_handle* h, int* tets, long long cap, l
   for (int k = 0; k <= kDihedBins; k++) cosv[k] = std::cos(4.0 * k * kPiRef / 180.0);
   for (int k = 0; k < 4; k++) cosv[46 + k] = std::cos(10.0 * (k + 1) * kPiRef / 180.0);
   if (!A((void**)&d_x, sizeof(double) * 3 * n) || !A((void**)&d_phi, sizeof(double) * n) ||
-      !A((void**)&d_h, sizeof(double) * n) || !A((void**)&d_type, sizeof(int) * n) ||
+      !A((void**)&d_h, sizeof(double) * n) || !A((void**)&d_rf, sizeof(float) * n) || !A((void**)&d_type, sizeof(int) * n) ||
       !A((void**)&d_rows, sizeof(int) * NC) || !A((void**)&d_cnt, sizeof(int) * n) ||
       !A((void**)&d_out, sizeof(int) * 4 * kMaxOut * (size_t)n) || !A((void**)&d_count, sizeof(int) * (n + 1)) ||
       !A((void**)&d_off, sizeof(int) * (n + 1)) || !A((void**)&d_blk, sizeof(int) * scan_blocksums_size(n)) ||
@@ -853,9 +1049,9 @@ extern "C" int mrsph_tetrahedralize(mrsph_handle* h, int* tets, long long cap, l
   if (rc) { h->err = h->eng->err; goto done; }
   {
     const int nbN = (int)std::min<long long>((n + kStarWarps - 1) / kStarWarps, 152LL * 64);
-    k_tet_snap<<<(int)((3 * n + 255) / 256), 256, 0, s>>>(3 * n, d_x, inv_g, g);
+    k_tet_snap<<<(int)((3 * n + 255) / 256), 256, 0, s>>>(n, d_x, inv_g, g, d_h, h->prm.cutoff, d_rf);
     TetIn T;
-    T.n = n; T.cap = rowcap; T.x = d_x; T.type = d_type; T.h = d_h; T.rows = d_rows; T.cnt = d_cnt;
+    T.n = n; T.cap = rowcap; T.x = d_x; T.type = d_type; T.h = d_h; T.rf = d_rf; T.rows = d_rows; T.cnt = d_cnt;
     T.inv_g = inv_g; T.cutoff = h->prm.cutoff; T.thres = 10.0;
     k_tet_star<<<nbN, 32 * kStarWarps, 0, s>>>(T, d_out, d_count, d_stats, d_flags);
     cell_scan(d_count, d_off, d_blk, n, 0, s);
@@ -879,7 +1075,7 @@ extern "C" int mrsph_tetrahedralize(mrsph_handle* h, int* tets, long long cap, l
       TetQIn Q;
       Q.x = d_x; Q.tets = d_tets; Q.ntet = ntet; Q.cos_dihed = d_cos; Q.cos_small = d_cos + 46; Q.hist = d_hist;
       k_tet_quality<<<nbT, 256, 0, s>>>(Q, d_part);
-      k_tet_quality_fold<<<1, 1, 0, s>>>(d_part, nbT, d_tq);
+      k_tet_quality_fold<<<1, 256, 0, s>>>(d_part, nbT, d_tq);
       cudaMemcpyAsync(&tq, d_tq, sizeof(TetStat), cudaMemcpyDeviceToHost, s);
       cudaMemcpyAsync(hist, d_hist, sizeof(hist), cudaMemcpyDeviceToHost, s);
       if (tets && cap >= ntet) cudaMemcpyAsync(tets, d_tets, sizeof(int) * 4 * ntet, cudaMemcpyDeviceToHost, s);
@@ -902,7 +1098,7 @@ extern "C" int mrsph_tetrahedralize(mrsph_handle* h, int* tets, long long cap, l
       q->min_edge = std::sqrt(tq.emin2); q->max_edge = std::sqrt(tq.emax2);
       q->min_aspect = tq.amin; q->max_aspect = tq.amax; q->avg_aspect = tq.asum / ntet;
       q->min_radius_ratio = tq.rmin; q->max_radius_ratio = tq.rmax; q->avg_radius_ratio = tq.rsum / ntet;
-      q->min_dihedral = tq.dmin; q->max_dihedral = tq.dmax; q->avg_min_dihedral = tq.dsum / ntet;
+      q->min_dihedral = dihed_degrees(tq.cdmin); q->max_dihedral = dihed_degrees(tq.cdmax); q->avg_min_dihedral = tq.dsum / ntet;
     }
     for (int k = 0; k < kAspectBins; k++) q->aspect_hist[k] = (long long)hist[k];
     for (int k = 0; k < kRadiusBins; k++) q->radius_hist[k] = (long long)hist[kAspectBins + k];
