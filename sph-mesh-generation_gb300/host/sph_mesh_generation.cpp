@@ -1054,13 +1054,17 @@ std::string Mesh_binary_writer::Output_mesh(int n_out, SPH_mesh_generation& sim,
     update_pvd(outdir_ + "/mesh_tets.pvd", n_out, std::to_string(ts), "./" + pvtu);
     return outdir_ + "/" + piece;
   }
-  long long ntri = 0;
-  int rc = mrsph_triangulate(sim.handle(), nullptr, 0, &ntri, nullptr);
-  if (rc) throw Error(rc, "mrsph_triangulate");
-  std::vector<int> tris(3 * (ntri > 0 ? ntri : 1));
+  // a planar triangulation has fewer than 2n triangles: one pass, a second one only beyond that
+  long long ntri = 0, room = 2 * sim.num_particles();
+  std::vector<int> tris(3 * (room > 0 ? room : 1));
   mrsph_tri_quality q{};
-  rc = mrsph_triangulate(sim.handle(), tris.data(), ntri, &ntri, &q);
+  int rc = mrsph_triangulate(sim.handle(), tris.data(), room, &ntri, &q);
   if (rc) throw Error(rc, "mrsph_triangulate");
+  if (ntri > room) {
+    tris.resize(3 * ntri);
+    rc = mrsph_triangulate(sim.handle(), tris.data(), ntri, &ntri, &q);
+    if (rc) throw Error(rc, "mrsph_triangulate");
+  }
   std::vector<int> type, nn;
   std::vector<double> h, norm;
   sim.Particle_fields(type, h, norm, nn);

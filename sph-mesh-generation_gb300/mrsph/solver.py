@@ -371,10 +371,14 @@ class SPHMeshGeneration:
         graph_mesh.cpp:411-670).  Returns (tris (ntri x 3 ids), quality dict)."""
         q = L.TriQuality()
         nt = C.c_longlong(0)
-        L.check(self.lib.mrsph_triangulate(self.h, None, 0, C.byref(nt), None), self.h, "mrsph_triangulate")
-        tris = np.zeros((max(nt.value, 1), 3), dtype=np.int32)
-        L.check(self.lib.mrsph_triangulate(self.h, _ptr(tris), nt.value, C.byref(nt), C.byref(q)), self.h,
+        # a planar triangulation has fewer than 2n triangles: one pass, a second one only beyond that
+        tris = np.zeros((2 * max(self.n, 1), 3), dtype=np.int32)
+        L.check(self.lib.mrsph_triangulate(self.h, _ptr(tris), len(tris), C.byref(nt), C.byref(q)), self.h,
                 "mrsph_triangulate")
+        if nt.value > len(tris):
+            tris = np.zeros((nt.value, 3), dtype=np.int32)
+            L.check(self.lib.mrsph_triangulate(self.h, _ptr(tris), len(tris), C.byref(nt), C.byref(q)), self.h,
+                    "mrsph_triangulate")
         out = {f: getattr(q, f) for f, _ in L.TriQuality._fields_ if f != "hist"}
         out["hist"] = np.array(q.hist[:], dtype=np.int64)
         return tris[: nt.value], out
