@@ -4,16 +4,18 @@
 // reference's operation order) and mrsph_fp32.cu.
 //
 // One step (SPH_mesh_generation::SPH_run_mesh_generation,
-// sph_mesh_generation.cpp:1371-1463) is 11 launches on one stream, replayed as
-// a CUDA graph:
+// sph_mesh_generation.cpp:1371-1463) is 11 launches on one stream (15 for a
+// large FP32-split handle), replayed as a CUDA graph:
 //   k_begin_step   scalars of the step
 //   k_map          A1 advect + A2 sample + A3 surface map/re-seed + A4 spacing
 //                  + scale/level refresh + cell key + cell histogram
-//   scan x3, scatter, rank      A5 counting sort into (level, cell) order
-//   k_reorder      gather persistent state into the sorted order
-//   k_density      A6 neighbour search over the cell table + A7 kernel sum,
-//                  writes the neighbour list (one row per particle)
-//   k_force<1>     A8 stage 1 + A9 dt/max|v| grid reduction (FP64 bit atomics)
+//   scan, scatter  A5 counting sort into (level, cell) order
+//   k_reorder      rank inside the cell, gather of the persistent state into the
+//                  sorted order, search radii
+//   k_brick_*      the work order of a large handle's list builder
+//   k_density(_group)  A6 neighbour search over the cell table: the neighbour lists
+//   k_force<1>     A7 kernel sum + A8 stage 1 + A9 dt/max|v| grid reduction (FP64
+//                  bit atomics), k_force_spill for particles whose list spilled
 //   k_force<2>     A8 stage 2 + A9 + A10 (stage-1 kick folded in; the stage-2
 //                  kick is folded into the next k_map)
 #pragma once
@@ -71,22 +73,16 @@ struct Work {  // per-step arrays in sorted order
   int cap;
   int* counts;
   unsigned* lhmax;  // [level][level-0 cell]: largest h (FP32 bits, rounded up) this step, 0 if none
+  int* bcount;      // particles per brick, then (bstart) their exclusive sums; the work order
+  int* bstart;
+  int* order;       // storage slots in work order: bricks, Z-order of half cells inside a brick
+  float* rlev;      // [level][particle]: search radius on the level (level_radius), 0 if none
   int* cstart;
   int* perm;
-  int* perm2;
   int* blocksums;
   int* slot_of_id;
-  int* fixq;    // FP32-split: particles whose density phase is re-decided exactly (count sc->nfix)
   int* spillq;  // particles whose list spilled (count sc->nspill)
 };
-
-// Neighbour-list entries: the neighbour's storage slot in the low 30 bits;
-// bits 30-31 carry the surface filter |n_i . n_j| > cos(angle_thres) where
-// the FP32-split density fix-up decided it in FP64 (0: decide in FP32).
-constexpr int NB_IDX = 0x3FFFFFFF;
-constexpr unsigned NB_COS_OK = 1u, NB_COS_NO = 2u;
-__host__ __device__ inline int nb_index(int e) { return e & NB_IDX; }
-__host__ __device__ inline unsigned nb_mark(int e) { return (unsigned)e >> 30; }
 
 // FP32-split decisions.  Three decisions of a step must come out as the
 // reference's FP64 arithmetic on the world positions makes them: the cell of
@@ -140,8 +136,18 @@ struct BatchSlot {
 
 enum { MAP_STEP = 0, MAP_PRE = 1 };
 
-// Tuning of the FP32 map and neighbour passes: resident 256-thread blocks per SM the
-// register allocation must allow, and the unroll of the tile loop.
+// Particles up to which a handle's own neighbour passes take kG lanes per
+// particle (force_particle, list_group) instead of one lane of a full warp
+// (force_particle, list_warp).  Below these counts the chip is not full and a
+// particle's chain of gathers bounds the kernel, above them the instructions do.
+// Measured, group against lane: stage 1 of 20,000 particles in 3D 37 against 67
+// us, of 77,551 in 2D 39 against 26; lists of 77,551 in 2D 71 against 135 us, of
+// 301,270 in 3D (uniform positions, 281 neighbours) 2.12 against 1.16 ms.
+constexpr long long kGroupMax = 40960;
+constexpr long long kListGroupMax = 131072;
+
+// Tuning of the FP32 map and neighbour passes: resident blocks per SM the
+// register allocation must allow (density: of kDensityThreads threads, else 256).
 #ifndef MRSPH_DENSITY_MIN_BLOCKS
 #define MRSPH_DENSITY_MIN_BLOCKS 6
 #endif
@@ -151,26 +157,20 @@ enum { MAP_STEP = 0, MAP_PRE = 1 };
 #ifndef MRSPH_FORCE2_MIN_BLOCKS
 #define MRSPH_FORCE2_MIN_BLOCKS 6
 #endif
-// list entries (indices, pair coefficients) moved per vector access in the force passes: 1 or 4
-#ifndef MRSPH_FORCE_VEC
-#define MRSPH_FORCE_VEC 4
+// the list builder's tile: candidates, and the spread in half cells within which
+// a warp's lanes share it
+#ifndef MRSPH_TILE_SIZE
+#define MRSPH_TILE_SIZE 256
 #endif
-#ifndef MRSPH_MAP_MIN_BLOCKS
-#define MRSPH_MAP_MIN_BLOCKS 4
-#endif
-#ifndef MRSPH_TILE_UNROLL
-#define MRSPH_TILE_UNROLL 1
-#endif
-constexpr int kTileUnroll = MRSPH_TILE_UNROLL;
-// largest spread of a warp's half cells (max - min per axis) for which the
-// warp scans the union of its lanes' rows through shared-memory tiles
 #ifndef MRSPH_TILE_SPAN_X
-#define MRSPH_TILE_SPAN_X 3
+#define MRSPH_TILE_SPAN_X 15
 #endif
 #ifndef MRSPH_TILE_SPAN_YZ
 #define MRSPH_TILE_SPAN_YZ 1
 #endif
-
+#ifndef MRSPH_MAP_MIN_BLOCKS
+#define MRSPH_MAP_MIN_BLOCKS 4
+#endif
 // ---------------------------------------------------------------------------
 // position representations
 // ---------------------------------------------------------------------------
@@ -335,10 +335,9 @@ template <> __device__ inline float4 mk4<float>(float a, float b, float c, float
 
 template <int D, class R>
 __device__ inline R dot3(const R* a, const R* b) {
-  R s = 0;
-  s += a[0] * b[0];
-  s += a[1] * b[1];
-  if (D == 3) s += a[2] * b[2];
+  R s = a[0] * b[0];
+  s = madd(a[1], b[1], s);
+  if (D == 3) s = madd(a[2], b[2], s);
   return s;
 }
 
@@ -368,7 +367,6 @@ __device__ inline void begin_step_body(DevScalars* sc, int inc) {
   sc->remap = 0;
   sc->nsurf = 0;
   sc->maxcnt = 0;
-  sc->nfix = 0;
   sc->nspill = 0;
   for (int l = 0; l < MAX_CL; l++) {
     sc->hmax[l] = 0;
@@ -376,12 +374,11 @@ __device__ inline void begin_step_body(DevScalars* sc, int inc) {
   }
   sc->step += inc;
 }
-static __global__ void k_begin_step(DevScalars* sc, int inc) { begin_step_body(sc, inc); }
-
-// clears n words (a step's per-level h maxima) as block blk of 256 threads
-__device__ inline void fill_block(unsigned* p, long long n, long long blk) {
-  const long long i = blk * blockDim.x + threadIdx.x;
-  if (i < n) p[i] = 0u;
+// scalars of the step, and the step's per-level h maxima (n words) cleared
+static __global__ void k_begin_step(DevScalars* sc, int inc, unsigned* lhmax, long long n) {
+  const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  if (i == 0) begin_step_body(sc, inc);
+  if (i < n) lhmax[i] = 0u;
 }
 
 // Random_particle_distribution, sph_mesh_generation.cpp:1302-1367 (one rank)
@@ -682,17 +679,30 @@ k_map(KCtx c, Buf<R> b, int* counts, unsigned* lhmax, int mode, unsigned max_att
 // Packed record read by the neighbour passes, two V4 words per particle so
 // that one candidate costs one 32-byte sector (FP32):
 //   FP32: w0 = (offset x, y, z, h), w1 = (anchor x, y, z as exact floats, +-1/rho^2)
-//   FP64: w0 = (x, y, z, h),        w1 = (0, 0, 0, +-1/rho^2)
+//   FP64: w0 = (x, y, z, h),        w1 = (box-relative x, y, z, h as four
+//         floats in the first 16 bytes, 0, +-1/rho^2)
 // The sign carries the type: negative for a particle that is not REAL.  1/rho^2 is the
 // neighbour's share of the pair coefficient of the force stages, computed once
 // per particle (as 1 / (rho * rho), the forces' own expression).
 template <int D, class R> struct RecOps;
 template <int D>
 struct RecOps<D, double> {
-  __device__ static void pack(const KCtx&, const double4& p, int, int type, double rho, double4& w0, double4& w1) {
+  __device__ static void pack(const KCtx& c, const double4& p, int, int type, double rho, double4& w0, double4& w1) {
     w0 = p;
     const double vol = r_rcp(rho * rho);
-    w1 = make_double4(0.0, 0.0, 0.0, type != REAL_P ? -vol : vol);
+    const float x = (float)(p.x - c.geo.box_l[0]), y = (float)(p.y - c.geo.box_l[1]);
+    const float z = D == 3 ? (float)(p.z - c.geo.box_l[2]) : 0.f, h = (float)p.w;
+    w1 = make_double4(__hiloint2double(__float_as_int(y), __float_as_int(x)),
+                      __hiloint2double(__float_as_int(h), __float_as_int(z)), 0.0, type != REAL_P ? -vol : vol);
+  }
+  // box-relative position and h in FP32 (the first 16 bytes of w1)
+  __device__ static float4 filter(const double4& w1) {
+    return make_float4(__int_as_float(__double2loint(w1.x)), __int_as_float(__double2hiint(w1.x)),
+                       __int_as_float(__double2loint(w1.y)), __int_as_float(__double2hiint(w1.y)));
+  }
+  template <class LD>
+  __device__ static float4 load_filter(const double4* rec, long long j) {
+    return LD::ld(reinterpret_cast<const float4*>(rec + 2 * j + 1));
   }
   __device__ static void rel(const KCtx&, const double4& a0, const double4&, const double4& b0, const double4&,
                              double* dr) {
@@ -712,9 +722,9 @@ struct RecOps<D, float> {
   }
   __device__ static void rel(const KCtx& c, const float4& a0, const float4& a1, const float4& b0, const float4& b1,
                              float* dr) {
-    dr[0] = (a1.x - b1.x) * c.geo.Af[0] + (a0.x - b0.x);
-    dr[1] = (a1.y - b1.y) * c.geo.Af[1] + (a0.y - b0.y);
-    dr[2] = (D == 3) ? (a1.z - b1.z) * c.geo.Af[2] + (a0.z - b0.z) : 0.f;
+    dr[0] = fmaf(a1.x - b1.x, c.geo.Af[0], a0.x - b0.x);
+    dr[1] = fmaf(a1.y - b1.y, c.geo.Af[1], a0.y - b0.y);
+    dr[2] = (D == 3) ? fmaf(a1.z - b1.z, c.geo.Af[2], a0.z - b0.z) : 0.f;
   }
 };
 
@@ -750,42 +760,81 @@ __device__ __noinline__ bool exact_cos(const KCtx& c, const float* ni, const flo
   return fabs(ca) > c.prm.cos_thres;
 }
 
-template <int D, class R>
-__device__ inline void reorder_block(const Buf<R>& src, const Buf<R>& dst, const KCtx& c, const int* perm2,
-                                     int* slot_of_id, long long n, int partial, long long blk) {
-  long long s = blk * blockDim.x + threadIdx.x;
-  if (s >= n) return;
-  int o = perm2[s];
-  const auto p = src.posh[o];
-  const int key = src.key ? src.key[o] : 0;
-  const auto nr = src.nr[o];
-  const int meta = src.meta[o];
-  dst.posh[s] = p;
-  if (src.key) dst.key[s] = key;
-  dst.nr[s] = nr;
-  dst.meta[s] = meta;
-  typename V4<R>::T w0, w1;
-  RecOps<D, R>::pack(c, p, key, meta & 0xFF, nr.w, w0, w1);
-  dst.rec[2 * s] = w0;
-  dst.rec[2 * s + 1] = w1;
-  int id = src.id[o];
-  dst.id[s] = id;
-  dst.nu[s] = src.nu_next[o];
-  dst.phi[s] = src.phi[o];
-  dst.curv[s] = src.curv[o];
-  dst.cellkey[s] = src.cellkey[o];
-  if (partial) {  // a step that stops before stage 2 keeps these consistent
-    dst.nu_next[s] = src.nu_next[o];
-    dst.v1[s] = src.v1[o];
-    dst.a2[s] = src.a2[o];
-  }
-  slot_of_id[id] = (int)s;
+// ---------------------------------------------------------------- work order
+// Storage is by rows of half cells, so the 32 particles of a warp lie along a
+// row, and where rows are short (a shell of one level, the end of a body) in
+// several of them: 2.2 segments per level on a relaxed torus.  The list builder
+// of a large handle therefore takes its particles in another order, by bricks
+// of 4 half cells per axis and by Z-order of the half cells inside a brick; what
+// is computed for a particle does not depend on it.
+__device__ inline void brick_of(const CellGeo& g, long long t, int& L, int* q) {
+  L = 0;
+  while (L + 1 < g.ncl && t >= g.boff[L + 1]) L++;
+  long long r = t - g.boff[L];
+  q[0] = (int)(r % g.bn[L][0]);
+  r /= g.bn[L][0];
+  q[1] = (int)(r % g.bn[L][1]);
+  q[2] = (int)(r / g.bn[L][1]);
 }
-
-template <int D, class R>
-__global__ void k_reorder(Buf<R> src, Buf<R> dst, KCtx c, const int* __restrict__ perm2,
-                          int* __restrict__ slot_of_id, long long n, int partial) {
-  reorder_block<D, R>(src, dst, c, perm2, slot_of_id, n, partial, blockIdx.x);
+// one thread per brick: its particles, from the start table
+template <int D>
+__global__ void __launch_bounds__(256) k_brick_count(KCtx c, const int* __restrict__ cstart, int* __restrict__ bcount) {
+  const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  if (t >= c.geo.boff[c.geo.ncl]) return;
+  int L, q[3], n = 0;
+  brick_of(c.geo, t, L, q);
+  if (c.sc->lcount[L]) {
+    const int* hn = c.geo.hn[L];
+    const int x0 = 4 * q[0], x1 = min(x0 + 4, hn[0]);
+    for (int z = 4 * q[2]; z < (D == 3 ? min(4 * q[2] + 4, hn[2]) : 1); z++)
+      for (int y = 4 * q[1]; y < min(4 * q[1] + 4, hn[1]); y++) {
+        const long long rb = c.geo.hoff[L] + ((long long)z * hn[1] + y) * hn[0];
+        n += cstart[rb + x1] - cstart[rb + x0];
+      }
+  }
+  bcount[t] = n;
+}
+// one warp per brick with particles: its half cells' particles in Z-order
+template <int D>
+__global__ void __launch_bounds__(256) k_brick_order(KCtx c, const int* __restrict__ cstart,
+                                                     const int* __restrict__ bcount, const int* __restrict__ bstart,
+                                                     int* __restrict__ order) {
+  const int lane = threadIdx.x & 31;
+  const long long base = ((long long)blockIdx.x * blockDim.x + threadIdx.x) & ~31ll, nb = c.geo.boff[c.geo.ncl];
+  const long long mine = base + lane;
+  unsigned todo = __ballot_sync(0xffffffffu, mine < nb && bcount[mine] > 0);
+  while (todo) {
+    const long long t = base + __ffs(todo) - 1;
+    todo &= todo - 1u;
+    int L, q[3];
+    brick_of(c.geo, t, L, q);
+    const int* hn = c.geo.hn[L];
+    int at = bstart[t];
+    for (int z0 = 0; z0 < (D == 3 ? 64 : 16); z0 += 32) {
+      const int zc = z0 + lane;  // Z-order index of the half cell
+      int h[3];
+      bool ok = zc < (D == 3 ? 64 : 16);
+      for (int d = 0; d < 3; d++) {
+        h[d] = d < D ? 4 * q[d] + (((zc >> d) & 1) | (((zc >> (D + d)) & 1) << 1)) : 0;
+        ok = ok && h[d] < hn[d];
+      }
+      int s0 = 0, s1 = 0;
+      if (ok) {
+        const long long cell = c.geo.hoff[L] + ((long long)h[2] * hn[1] + h[1]) * hn[0] + h[0];
+        s0 = cstart[cell];
+        s1 = cstart[cell + 1];
+      }
+      int inc = s1 - s0;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const int v = __shfl_up_sync(0xffffffffu, inc, o);
+        if (lane >= o) inc += v;
+      }
+      int o = at + inc - (s1 - s0);
+      for (int u = s0; u < s1; u++) order[o++] = u;
+      at += __shfl_sync(0xffffffffu, inc, 31);
+    }
+  }
 }
 
 // Largest h of level-L particles (lhmax entries) over the level-0 cells
@@ -818,33 +867,35 @@ template <int D> struct SOrigin<D, float> {
   }
 };
 
-// Level L of the candidate search from origin so with smoothing length hi:
-// R_L = cutoff * max(hi, local h maximum of level L) + 1e-10 with a relative
-// pad (1e-5 FP64, 3e-5 FP32-split; 0 when no level-L particle can pair with the origin), and the
-// origin's half-cell coordinate q + fr on level L.  The local h maximum is
-// the largest lhmax entry over the level-0 cells overlapping the cube of the
-// level-wide bound (every level-L particle that can pair with the origin lies
-// in one of them).  FP64-plain keeps the box-relative FP64 arithmetic;
-// FP32-split works in FP32 relative to the anchor: a level-L cell is
-// 2^(finest - L) anchor cells, so the position inside the origin's level-L
-// (or level-0) cell is (anchor index - cell's first anchor) * A + offset.
+// Level L of the candidate search from origin so with smoothing length hi.
+// level_radius: R_L = cutoff * max(hi, local h maximum of level L) + 1e-10 with
+// a relative pad (1e-5 FP64, 3e-5 FP32-split; 0 when no level-L particle can
+// pair with the origin).  The local h maximum is the largest lhmax entry over
+// the level-0 cells overlapping the cube of the level-wide bound (every level-L
+// particle that can pair with the origin lies in one of them).  level_position:
+// the origin's half-cell coordinate q + fr on level L.
+// FP64-plain keeps the box-relative FP64 arithmetic; FP32-split works in FP32
+// relative to the anchor: a level-L cell is 2^(finest - L) anchor cells, so the
+// position inside the origin's level-L (or level-0) cell is (anchor index -
+// cell's first anchor) * A + offset.
 template <int D, class LD = LdNC>
-__device__ inline float level_origin(const KCtx& c, const unsigned* __restrict__ lhmax, int L,
-                                     const SOrigin<D, double>& so, double hi, bool active, int* q, float* fr) {
+__device__ inline float level_radius(const KCtx& c, const unsigned* __restrict__ lhmax, int L,
+                                     const SOrigin<D, double>& so, double hi) {
   const double hic = hi * c.prm.cutoff;
   const double Rg = (fmax(hic, bitsd(c.sc->hmax[L]) * c.prm.cutoff) + 1.e-10) * (1.0 + 1.e-5);
-  float hloc = 0.f;
-  if (active) {
-    int lo[3] = {0, 0, 0}, up[3] = {0, 0, 0};
-    for (int d = 0; d < D; d++) {
-      const double top = (double)(c.geo.n[0][d] - 1);
-      lo[d] = (int)fmax(0.0, fmin(floor((so.xr[d] - Rg) * c.geo.idc0[d]), top));
-      up[d] = (int)fmax(0.0, fmin(floor((so.xr[d] + Rg) * c.geo.idc0[d]), top));
-    }
-    hloc = lhmax_over<LD>(c, lhmax, L, lo, up);
+  int lo[3] = {0, 0, 0}, up[3] = {0, 0, 0};
+  for (int d = 0; d < D; d++) {
+    const double top = (double)(c.geo.n[0][d] - 1);
+    lo[d] = (int)fmax(0.0, fmin(floor((so.xr[d] - Rg) * c.geo.idc0[d]), top));
+    up[d] = (int)fmax(0.0, fmin(floor((so.xr[d] + Rg) * c.geo.idc0[d]), top));
   }
+  const float hloc = lhmax_over<LD>(c, lhmax, L, lo, up);
   if (!(hloc > 0.f)) return 0.f;
   const double Rw = fmax(hic, (double)hloc * c.prm.cutoff) + 1.e-10;
+  return (float)(Rw * (1.0 + 1.e-5));
+}
+template <int D>
+__device__ inline void level_position(const KCtx& c, int L, const SOrigin<D, double>& so, int* q, float* fr) {
   for (int d = 0; d < D; d++) {
     double u = so.xr[d] / c.geo.hs[L][d];
     u = fmax(-1.0e6, fmin(u, 1.0e9));
@@ -852,29 +903,29 @@ __device__ inline float level_origin(const KCtx& c, const unsigned* __restrict__
     q[d] = (int)fl;
     fr[d] = (float)(u - fl);
   }
-  return (float)(Rw * (1.0 + 1.e-5));
 }
 template <int D, class LD = LdNC>
-__device__ inline float level_origin(const KCtx& c, const unsigned* __restrict__ lhmax, int L,
-                                     const SOrigin<D, float>& so, float hi, bool active, int* q, float* fr) {
+__device__ inline float level_radius(const KCtx& c, const unsigned* __restrict__ lhmax, int L,
+                                     const SOrigin<D, float>& so, float hi) {
   const float cut = c.prm.cutoff_f;
   const float hic = hi * cut;
   const float Rg = (fmaxf(hic, (float)bitsd(c.sc->hmax[L]) * cut) + 1.e-10f) * (1.f + 3.e-5f);
-  float hloc = 0.f;
-  if (active) {
-    const int sh0 = c.geo.ncl - 1;
-    int lo[3] = {0, 0, 0}, up[3] = {0, 0, 0};
-    for (int d = 0; d < D; d++) {
-      const int c0 = so.k[d] >> sh0;
-      const float u0 = fmaf((float)(so.k[d] - (c0 << sh0)), c.geo.Af[d], so.o[d]) * c.geo.idc0_f[d];
-      const float r0 = Rg * c.geo.idc0_f[d];
-      const int top = c.geo.n[0][d] - 1;
-      lo[d] = max(0, min(c0 + (int)floorf(fmaxf(u0 - r0, -1.0e6f)), top));
-      up[d] = max(0, min(c0 + (int)floorf(fminf(u0 + r0, 1.0e6f)), top));
-    }
-    hloc = lhmax_over<LD>(c, lhmax, L, lo, up);
+  const int sh0 = c.geo.ncl - 1;
+  int lo[3] = {0, 0, 0}, up[3] = {0, 0, 0};
+  for (int d = 0; d < D; d++) {
+    const int c0 = so.k[d] >> sh0;
+    const float u0 = fmaf((float)(so.k[d] - (c0 << sh0)), c.geo.Af[d], so.o[d]) * c.geo.idc0_f[d];
+    const float r0 = Rg * c.geo.idc0_f[d];
+    const int top = c.geo.n[0][d] - 1;
+    lo[d] = max(0, min(c0 + (int)floorf(fmaxf(u0 - r0, -1.0e6f)), top));
+    up[d] = max(0, min(c0 + (int)floorf(fminf(u0 + r0, 1.0e6f)), top));
   }
+  const float hloc = lhmax_over<LD>(c, lhmax, L, lo, up);
   if (!(hloc > 0.f)) return 0.f;
+  return (fmaxf(hic, hloc * cut) + 1.e-10f) * (1.f + 3.e-5f);
+}
+template <int D>
+__device__ inline void level_position(const KCtx& c, int L, const SOrigin<D, float>& so, int* q, float* fr) {
   const int sh = c.geo.ncl - 1 - L;
   for (int d = 0; d < D; d++) {
     const int cc = so.k[d] >> sh;
@@ -884,7 +935,94 @@ __device__ inline float level_origin(const KCtx& c, const unsigned* __restrict__
     q[d] = 2 * cc + (int)fl;
     fr[d] = u - fl;
   }
-  return (fmaxf(hic, hloc * cut) + 1.e-10f) * (1.f + 3.e-5f);
+}
+// the half cells the sphere of radius R around q + fr reaches, per axis
+template <int D>
+__device__ inline void level_box(const KCtx& c, int L, float R, const int* q, const float* fr, int* lo, int* up) {
+  for (int d = 0; d < D; d++) {
+    const float rr = R / c.geo.hs_f[L][d];
+    lo[d] = max(q[d] + (int)floorf(fr[d] - rr), 0);
+    up[d] = min(q[d] + (int)floorf(fr[d] + rr), c.geo.hn[L][d] - 1);
+  }
+}
+// Particles [s0, e0) of row (z, y) of level L inside the sphere; false when the
+// row lies outside.
+template <int D, class LD = LdNC>
+__device__ inline bool row_range(const KCtx& c, const int* __restrict__ cstart, int L, float R, const int* q,
+                                 const float* fr, int z, int y, int& s0, int& e0) {
+  const int* hn = c.geo.hn[L];
+  float gz = 0.f;
+  if (D == 3) {
+    const int m = z - q[2];
+    if (z > 0) gz = fmaxf(gz, (float)m - fr[2]);
+    if (z < hn[2] - 1) gz = fmaxf(gz, fr[2] - (float)(m + 1));
+    gz *= c.geo.hs_f[L][2];
+  }
+  const int m = y - q[1];
+  float gy = 0.f;
+  if (y > 0) gy = fmaxf(gy, (float)m - fr[1]);
+  if (y < hn[1] - 1) gy = fmaxf(gy, fr[1] - (float)(m + 1));
+  gy *= c.geo.hs_f[L][1];
+  const float rem = R * R - gy * gy - gz * gz;
+  if (rem < 0.f) return false;
+  const float w = sqrtf(rem) / c.geo.hs_f[L][0];
+  const int xl = max(q[0] + (int)floorf(fr[0] - w), 0);
+  const int xh = min(q[0] + (int)floorf(fr[0] + w), hn[0] - 1);
+  if (xl > xh) return false;
+  const long long rb = c.geo.hoff[L] + ((long long)z * hn[1] + y) * hn[0];
+  s0 = LD::ld(&cstart[rb + xl]);
+  e0 = LD::ld(&cstart[rb + xh + 1]);
+  return true;
+}
+
+// The last step of the counting sort, the gather into storage order and the
+// per-level search radii, one thread per entry of perm: perm holds each cell's
+// particles in arbitrary order, the canonical order inside a cell is ascending
+// id, so the thread counts the lower ids of its cell and writes its particle
+// there.  (A separate ranking pass wrote and read back the permutation: 25 us
+// and a launch for 2.4 M particles.)
+template <int D, class R, class LD = LdNC>
+__device__ inline void reorder_block(const Buf<R>& src, const Buf<R>& dst, const KCtx& c, const Work<R>& w,
+                                     int partial, long long blk) {
+  const long long t = blk * blockDim.x + threadIdx.x;
+  const long long n = c.n;
+  if (t >= n) return;
+  const int o = w.perm[t];
+  const int ck = src.cellkey[o], id = src.id[o];
+  const int c0 = LD::ld(&w.cstart[ck]), c1 = LD::ld(&w.cstart[ck + 1]);
+  long long s = c0;
+  for (int u = c0; u < c1; u++) s += src.id[w.perm[u]] < id ? 1 : 0;
+  const auto p = src.posh[o];
+  const int key = src.key ? src.key[o] : 0;
+  const auto nr = src.nr[o];
+  const int meta = src.meta[o];
+  dst.posh[s] = p;
+  if (src.key) dst.key[s] = key;
+  dst.nr[s] = nr;
+  dst.meta[s] = meta;
+  typename V4<R>::T w0, w1;
+  RecOps<D, R>::pack(c, p, key, meta & 0xFF, nr.w, w0, w1);
+  dst.rec[2 * s] = w0;
+  dst.rec[2 * s + 1] = w1;
+  dst.id[s] = id;
+  dst.nu[s] = src.nu_next[o];
+  dst.phi[s] = src.phi[o];
+  dst.curv[s] = src.curv[o];
+  dst.cellkey[s] = ck;
+  if (partial) {  // a step that stops before stage 2 keeps these consistent
+    dst.nu_next[s] = src.nu_next[o];
+    dst.v1[s] = src.v1[o];
+    dst.a2[s] = src.a2[o];
+  }
+  w.slot_of_id[id] = (int)s;
+  const SOrigin<D, R> so(c, p, key);
+  for (int L = 0; L < c.geo.ncl; L++)
+    w.rlev[(long long)L * n + s] = c.sc->lcount[L] ? level_radius<D, LD>(c, w.lhmax, L, so, p.w) : 0.f;
+}
+
+template <int D, class R>
+__global__ void k_reorder(Buf<R> src, Buf<R> dst, KCtx c, Work<R> w, int partial) {
+  reorder_block<D, R>(src, dst, c, w, partial, blockIdx.x);
 }
 
 // Candidates of particle i over all cell-list levels.  The reference walks
@@ -901,156 +1039,88 @@ __device__ inline float level_origin(const KCtx& c, const unsigned* __restrict__
 // arithmetic (FP64: 1e-5; FP32-split: 3e-5, which also covers the FP32
 // test's acceptance band of 2^-15 on R^2, so the per-lane and the warp-tile
 // scans accept the same candidates); the candidate test decides membership.
-template <int D, class R, class LD = LdNC, class F>
-__device__ inline void scan_candidates(const KCtx& c, const int* __restrict__ cstart,
-                                       const unsigned* __restrict__ lhmax, const SOrigin<D, R>& so, R hi, F&& f) {
-  for (int L = 0; L < c.geo.ncl; L++) {
-    if (c.sc->lcount[L] == 0) continue;
-    int q[3] = {0, 0, 0}, lo[3] = {0, 0, 0}, up[3] = {0, 0, 0}, hn[3];
-    float fr[3] = {0.f, 0.f, 0.f}, hs[3] = {1.f, 1.f, 1.f};
-    const float R = level_origin<D, LD>(c, lhmax, L, so, hi, true, q, fr);
-    if (!(R > 0.f)) continue;
-    for (int d = 0; d < 3; d++) hn[d] = c.geo.hn[L][d];
-    for (int d = 0; d < D; d++) {
-      hs[d] = c.geo.hs_f[L][d];
-      const float rr = R / hs[d];
-      lo[d] = max(q[d] + (int)floorf(fr[d] - rr), 0);
-      up[d] = min(q[d] + (int)floorf(fr[d] + rr), hn[d] - 1);
+// The candidates by a group of kG lanes per particle.  The lanes take the rows of the particle's spheres
+// kG at a time, one row range each; the ranges of up to kRowTile non-empty rows
+// stand in shared memory as one run of candidates, which the lanes then walk
+// kG at a time: visit(j, in) is called by the whole group, in = false past the
+// end.  The search radii come from w.rlev (one thread per particle and level
+// filled them in the reorder pass).
+constexpr int kG = 8;
+constexpr int kRowTile = 48;
+struct RowTile {
+  int off[kRowTile];  // first particle of the row - its place in the run
+  int end[kRowTile];  // end of the row in the run
+};
+struct GroupLanes {
+  unsigned mask, below;
+  int gl, shift;
+  __device__ GroupLanes() {
+    const int lane = threadIdx.x & 31;
+    gl = lane & (kG - 1);
+    shift = lane - gl;
+    mask = ((1u << kG) - 1u) << shift;
+    below = (1u << gl) - 1u;
+  }
+  __device__ unsigned ballot(bool p) const { return (__ballot_sync(mask, p) >> shift) & ((1u << kG) - 1u); }
+};
+template <int D, class R, class LD, class F>
+__device__ inline void group_scan(const KCtx& c, const Work<R>& w, const GroupLanes& g, RowTile& rt, long long i,
+                                  const SOrigin<D, R>& so, F&& visit) {
+  int nrow = 0, T = 0;
+  auto flush = [&]() {
+    __syncwarp(g.mask);
+    int r = 0;
+    for (int t0 = 0; t0 < T; t0 += kG) {
+      const int t = t0 + g.gl;
+      const bool in = t < T;
+      int j = 0;
+      if (in) {
+        while (t >= rt.end[r]) r++;
+        j = rt.off[r] + t;
+      }
+      visit(j, in);
     }
-    const long long base = c.geo.hoff[L];
-    const float R2 = R * R;
-    for (int z = lo[2]; z <= up[2]; z++) {
-      float gz = 0.f;
-      if (D == 3) {
-        const int m = z - q[2];
-        if (z > 0) gz = fmaxf(gz, (float)m - fr[2]);
-        if (z < hn[2] - 1) gz = fmaxf(gz, fr[2] - (float)(m + 1));
-        gz *= hs[2];
+    __syncwarp(g.mask);
+    nrow = 0;
+    T = 0;
+  };
+  for (int L = 0; L < c.geo.ncl; L++) {
+    const float R_ = LD::ld(&w.rlev[(long long)L * c.n + i]);
+    if (!(R_ > 0.f)) continue;  // group-uniform
+    int q[3] = {0, 0, 0}, lo[3] = {0, 0, 0}, up[3] = {0, 0, 0};
+    float fr[3] = {0.f, 0.f, 0.f};
+    level_position<D>(c, L, so, q, fr);
+    level_box<D>(c, L, R_, q, fr, lo, up);
+    const int ny = up[1] - lo[1] + 1, nz = up[2] - lo[2] + 1;
+    if (ny <= 0 || nz <= 0) continue;
+    const int nr = ny * nz;
+    for (int b = 0; b < nr; b += kG) {
+      const int rr = b + g.gl;
+      int s0 = 0, e0 = 0;
+      if (rr < nr) {
+        const int iz = D == 3 ? rr / ny : 0;
+        row_range<D, LD>(c, w.cstart, L, R_, q, fr, lo[2] + iz, lo[1] + rr - iz * ny, s0, e0);
       }
-      for (int y = lo[1]; y <= up[1]; y++) {
-        const int m = y - q[1];
-        float gy = 0.f;
-        if (y > 0) gy = fmaxf(gy, (float)m - fr[1]);
-        if (y < hn[1] - 1) gy = fmaxf(gy, fr[1] - (float)(m + 1));
-        gy *= hs[1];
-        const float rem = R2 - gy * gy - gz * gz;
-        if (rem < 0.f) continue;
-        const float w = sqrtf(rem) / hs[0];
-        const int xl = max(q[0] + (int)floorf(fr[0] - w), 0);
-        const int xh = min(q[0] + (int)floorf(fr[0] + w), hn[0] - 1);
-        if (xl > xh) continue;
-        const long long rb = base + ((long long)z * hn[1] + y) * hn[0];
-        const int s0 = LD::ld(&cstart[rb + xl]), e0 = LD::ld(&cstart[rb + xh + 1]);
-        for (int j = s0; j < e0; j++) f(j);
+      const int len = max(e0 - s0, 0);
+      int inc = len;
+#pragma unroll
+      for (int o = 1; o < kG; o <<= 1) {
+        const int t = __shfl_up_sync(g.mask, inc, o, kG);
+        if (g.gl >= o) inc += t;
       }
+      const unsigned full = g.ballot(len > 0);
+      if (!full) continue;
+      if (nrow + __popc(full) > kRowTile) flush();
+      if (len > 0) {
+        const int at = nrow + __popc(full & g.below);
+        rt.off[at] = s0 - (T + inc - len);
+        rt.end[at] = T + inc;
+      }
+      nrow += __popc(full);
+      T += __shfl_sync(g.mask, inc, kG - 1, kG);
     }
   }
-}
-
-// Warp-cooperative form of scan_candidates, called by all 32 lanes of a warp
-// (inactive lanes pass active = false).  Per level, when the warp's particles
-// sit within a 4 x 2 x 2 block of half cells (dense regions), the warp walks the
-// union of its lanes' rows: each 32-candidate chunk of a row is loaded once,
-// coalesced, into the warp's shared-memory tile and every lane tests the
-// chunk from there.  Otherwise each lane walks its own rows from global
-// memory.  Either way a lane visits its own candidates in the same order
-// (levels, rows, storage order), so its accepted neighbours and their order
-// do not depend on the mode; lanes also see extra candidates of the union,
-// which the candidate test rejects.
-// load(k) builds the tile entry of candidate k (uniform mode),
-// vchunk(t0, m, tile) visits the m candidates t0 .. t0 + m - 1 held in the
-// tile, in that order, vglob(j) visits candidate j straight from global
-// memory (per-lane mode).
-// origin() gives the search origin (built per level from memory rather than
-// held in registers across the scan).
-template <int D, class R, class LD = LdNC, class E, class SO, class FL, class FT, class FG>
-__device__ inline void warp_scan(const KCtx& c, const int* __restrict__ cstart, const unsigned* __restrict__ lhmax,
-                                 bool active, SO&& origin, R hi, E* tile, FL&& load, FT&& vchunk,
-                                 FG&& vglob) {
-  const int lane = threadIdx.x & 31;
-  const unsigned FULL = 0xffffffffu;
-  for (int L = 0; L < c.geo.ncl; L++) {
-    if (c.sc->lcount[L] == 0) continue;
-    int q[3] = {0, 0, 0}, lo[3] = {0, 0, 0}, up[3] = {-1, -1, -1}, hn[3];
-    float fr[3] = {0.f, 0.f, 0.f}, hs[3] = {1.f, 1.f, 1.f};
-    const float R = level_origin<D, LD>(c, lhmax, L, origin(), hi, active, q, fr);
-    const bool need = R > 0.f;
-    if (!__any_sync(FULL, need)) continue;
-    const float R2 = R * R;
-    for (int d = 0; d < 3; d++) hn[d] = c.geo.hn[L][d];
-    if (D == 2) { lo[2] = 0; up[2] = 0; }
-    if (need) {
-      for (int d = 0; d < D; d++) {
-        hs[d] = c.geo.hs_f[L][d];
-        const float rr = R / hs[d];
-        lo[d] = max(q[d] + (int)floorf(fr[d] - rr), 0);
-        up[d] = min(q[d] + (int)floorf(fr[d] + rr), hn[d] - 1);
-      }
-    }
-    // own x range of row (z, y); empty when the row is outside the lane's sphere
-    auto row_range = [&](int z, int y, int& xl, int& xh) {
-      xl = 0x7fffffff;
-      xh = -1;
-      if (!need || z < lo[2] || z > up[2] || y < lo[1] || y > up[1]) return;
-      float gz = 0.f;
-      if (D == 3) {
-        const int m = z - q[2];
-        if (z > 0) gz = fmaxf(gz, (float)m - fr[2]);
-        if (z < hn[2] - 1) gz = fmaxf(gz, fr[2] - (float)(m + 1));
-        gz *= hs[2];
-      }
-      const int m = y - q[1];
-      float gy = 0.f;
-      if (y > 0) gy = fmaxf(gy, (float)m - fr[1]);
-      if (y < hn[1] - 1) gy = fmaxf(gy, fr[1] - (float)(m + 1));
-      gy *= hs[1];
-      const float rem = R2 - gy * gy - gz * gz;
-      if (rem < 0.f) return;
-      const float w = sqrtf(rem) / hs[0];
-      xl = max(q[0] + (int)floorf(fr[0] - w), 0);
-      xh = min(q[0] + (int)floorf(fr[0] + w), hn[0] - 1);
-    };
-    const long long base = c.geo.hoff[L];
-    // warp compactness at this level
-    const int BIG = 0x3fffffff;
-    bool uni = true;
-    for (int d = 0; d < D; d++) {
-      const int qmin = __reduce_min_sync(FULL, need ? q[d] : BIG);
-      const int qmax = __reduce_max_sync(FULL, need ? q[d] : -BIG);
-      uni = uni && (qmax - qmin <= (d == 0 ? MRSPH_TILE_SPAN_X : MRSPH_TILE_SPAN_YZ));
-    }
-    if (uni) {
-      const int zl = __reduce_min_sync(FULL, need ? lo[2] : BIG), zu = __reduce_max_sync(FULL, need ? up[2] : -BIG);
-      const int yl = __reduce_min_sync(FULL, need ? lo[1] : BIG), yu = __reduce_max_sync(FULL, need ? up[1] : -BIG);
-      for (int z = zl; z <= zu; z++)
-        for (int y = yl; y <= yu; y++) {
-          int xl, xh;
-          row_range(z, y, xl, xh);
-          const int ul = __reduce_min_sync(FULL, xl), uh = __reduce_max_sync(FULL, xh);
-          if (ul > uh) continue;
-          const long long rb = base + ((long long)z * hn[1] + y) * hn[0];
-          const int s0 = LD::ld(&cstart[rb + ul]), e0 = LD::ld(&cstart[rb + uh + 1]);
-          for (int t0 = s0; t0 < e0; t0 += 32) {
-            const int k = t0 + lane;
-            if (k < e0) tile[lane] = load(k);
-            __syncwarp();
-            const int m = min(32, e0 - t0);
-            if (need) vchunk(t0, m, (const E*)tile);
-            __syncwarp();
-          }
-        }
-    } else if (need) {
-      for (int z = lo[2]; z <= up[2]; z++)
-        for (int y = lo[1]; y <= up[1]; y++) {
-          int xl, xh;
-          row_range(z, y, xl, xh);
-          if (xl > xh) continue;
-          const long long rb = base + ((long long)z * hn[1] + y) * hn[0];
-          const int s0 = LD::ld(&cstart[rb + xl]), e0 = LD::ld(&cstart[rb + xh + 1]);
-          for (int j = s0; j < e0; j++) vglob(j);
-        }
-    }
-  }
+  if (T > 0) flush();
 }
 
 // Neighbour criterion, level_infor.cpp:491-500.
@@ -1066,10 +1136,9 @@ __device__ inline double force_dist(double d2) { return sqrt(d2); }
 __device__ inline float force_dist(float d2) { return sqrtf(d2); }
 
 template <class R> __device__ inline R d2_of(const R* dr, int D) {
-  R d2 = 0;
-  d2 += dr[0] * dr[0];
-  d2 += dr[1] * dr[1];
-  if (D == 3) d2 += dr[2] * dr[2];
+  R d2 = dr[0] * dr[0];
+  d2 = madd(dr[1], dr[1], d2);
+  if (D == 3) d2 = madd(dr[2], dr[2], d2);
   return d2;
 }
 
@@ -1084,363 +1153,452 @@ __device__ inline int char_pair(int ti, int tj) {
   return tj == SEGMENT_P ? 1 : (tj == SINGULARITY_P ? 2 : 0);
 }
 
-// A6 + A7: Refresh_neighbor_info (level_infor.cpp:469-506) and
-// Get_kernel_summation (particle_mesh_generation.cpp:690-765).  The
-// neighbour list is written in the fixed scan order.
-template <class R> struct RecPair { typename V4<R>::T a, b; };
+// The neighbour criterion of a pair (A6, Refresh_neighbor_info,
+// level_infor.cpp:469-506), decided as the reference's FP64 arithmetic decides
+// it.  FP32-split: in FP32 outside the band, else on the world positions.
+// FP64-plain: in FP32 on box-relative positions (two words of the record) when
+// the distance clears the radius by the rounding of the positions (2^-21 of
+// their magnitude, above the 3.5 * 2^-24 that three coordinate differences can
+// be off by) and of the test (1e-5), else by the FP64 test itself; an FP64
+// instruction costs 60 FP32 ones here, and nearly every candidate clears it.
+template <int D, class R> struct PairTest;
+template <int D> struct PairTest<D, float> {
+  float4 a0, a1;
+  float cut, R2i;
+  __device__ PairTest(const KCtx& c, const float4* rec, long long i) {
+    a0 = rec[2 * i];
+    a1 = rec[2 * i + 1];
+    cut = c.prm.cutoff_f;
+    R2i = (a0.w * cut) * (a0.w * cut);
+  }
+  template <class LD>
+  __device__ bool near(const KCtx& c, const float4* rec, int j) const {
+    float4 b0, b1;
+    LD::rec(rec, j, b0, b1);
+    float dr[3];
+    RecOps<D, float>::rel(c, a0, a1, b0, b1, dr);
+    const float d2 = d2_of(dr, D);
+    const float rj = b0.w * cut;
+    const float Rm = fmaxf(R2i, rj * rj);
+    if (d2 > Rm * kD2Accept) return false;
+    return d2 < Rm * kD2Sure || exact_neighbor<D>(c, a0, a1, b0, b1);
+  }
+};
+template <int D>
+__device__ __noinline__ bool exact_neighbor64(const KCtx& c, const double4* rec, long long i, int j) {
+  const double4 a0 = rec[2 * i], b0 = rec[2 * (long long)j];
+  double dr[3], dist;
+  RecOps<D, double>::rel(c, a0, a0, b0, b0, dr);
+  return nb_test(d2_of(dr, D), a0.w, b0.w, c.prm.cutoff, dist);
+}
+template <int D> struct PairTest<D, double> {
+  float4 f;  // box-relative position, h
+  float cut, pad;
+  long long i;
+  __device__ PairTest(const KCtx& c, const double4* rec, long long i_) : i(i_) {
+    f = RecOps<D, double>::filter(rec[2 * i + 1]);
+    cut = c.prm.cutoff_f;
+    pad = 0x1p-21f * (c.geo.ext_f + fabsf(f.x) + fabsf(f.y) + fabsf(f.z)) + 2.e-10f;
+  }
+  template <class LD>
+  __device__ bool near(const KCtx& c, const double4* rec, int j) const {
+    const float4 q = RecOps<D, double>::template load_filter<LD>(rec, j);
+    const float dx = f.x - q.x, dy = f.y - q.y, dz = D == 3 ? f.z - q.z : 0.f;
+    const float d2 = dx * dx + dy * dy + dz * dz, Rm = fmaxf(f.w, q.w) * cut;
+    const float far = Rm * 1.00001f + pad, sure = Rm * 0.99999f - pad;
+    if (d2 > far * far) return false;
+    return (sure > 0.f && d2 < sure * sure) || exact_neighbor64<D>(c, rec, i, j);
+  }
+};
 
-
-// KK: the kernel kind fixed at compile time (FP32 Wendland C2), or -1
-template <int D, class R, int KK, class LD = LdNC>
-__device__ inline void density_block(const KCtx& c, const Buf<R>& b, const Work<R>& w, long long blk) {
-  using P = PosOps<D, R>;
-  using Q = RecOps<D, R>;
-  using T4 = typename V4<R>::T;
-  constexpr bool F32 = std::is_same<R, float>::value;
-  // FP32 tile entry: position relative to the warp's anchor cell and
-  // (cutoff*h)^2, negative for a particle that is not REAL; FP64: the packed record
-  using E = typename std::conditional<F32, float4, RecPair<R>>::type;
-  __shared__ E s_tile[8][32];
-  long long i = blk * blockDim.x + threadIdx.x;
-  const bool active = i < c.n;
-  unsigned long long pairs = 0;
-  T4 a0 = mk4<R>(0, 0, 0, 0), a1 = mk4<R>(0, 0, 0, 0);
-  int ti = REAL_P;
-  R ni[3] = {0, 0, 0};
-  if (active) {
-    a0 = b.rec[2 * i];
-    a1 = b.rec[2 * i + 1];
-    ti = b.meta[i] & 0xFF;
-    if (!F32 && ti != REAL_P) {
-      const T4 nri = b.nr[i];
-      ni[0] = nri.x; ni[1] = nri.y; ni[2] = nri.z;
-    }
-  }
-  auto origin = [&]() {
-    return SOrigin<D, R>(c, active ? b.posh[i] : mk4<R>(0, 0, 0, 0), (active && b.key) ? b.key[i] : 0);
-  };
-  const R hi = a0.w;
-  const R inv_hi = active ? r_rcp(hi) : (R)0;
-  const int kind = KK >= 0 ? KK : c.prm.kernel;
-  // FP32 Wendland C2: a REAL particle sums (1 - s/2)^4 (1 + 2s), s = r/h,
-  // clamped at s = 2, and applies the normalisation C/h^D once at the end
-  constexpr bool WEN32 = F32 && KK == K_WEN;
-  const R cos_t = pick<R>(c.prm.cos_thres, c.prm.cos_thres_f);
-  const R cut = pick<R>(c.prm.cutoff, c.prm.cutoff_f);
-  R sum = 0;
-  int ncount = 0, cnt = 0;
-  bool unc = false;  // FP32-split: a decision of this particle lies in its band (exact re-decision follows)
-  const R R2i = (hi * cut) * (hi * cut);
-  int* row = w.nbl + nb_slot(active ? i : 0, 0, w.cap);  // entry q at row[(q >> 3) * 256 + (q & 7)]
-  // accepted neighbour j at distance vector dr (i - j), |dr| = dist; char_j:
-  // j is not REAL.  A SEGMENT particle sums in 3D only (:740-759).
-  const bool char_i = ti == SURFACE_P || (D == 3 && ti == SEGMENT_P);
-  auto accept = [&](int j, const R* dr, R dist, bool char_j) {
-    if (cnt < w.cap) row[((cnt >> 3) << 8) + (cnt & 7)] = j;
-    cnt++;
-    if (ti == REAL_P) {
-      if constexpr (WEN32) {
-        const float s = (float)dist * (float)inv_hi;
-        const float t = fmaxf(fmaf(-0.5f, s, 1.f), 0.f), t2 = t * t;
-        sum += (t2 * t2) * fmaf(2.f, s, 1.f);
-      } else {
-        sum += pair_W(kind, D, dist, hi, inv_hi);
-        ncount++;
-      }
-    } else if (char_i && char_j) {  // the tangential kernel sum of a surface or segment particle
-      const int rule = char_pair(ti, b.meta[j] & 0xFF);
-      if (rule == 0) return;
-      if constexpr (F32) {  // the normal is not kept in registers across the scan
-        const T4 nri = b.nr[i];
-        ni[0] = nri.x; ni[1] = nri.y; ni[2] = nri.z;
-      }
-      R dn = dot3<D, R>(dr, ni);
-      R pr[3] = {dr[0] - ni[0] * dn, dr[1] - ni[1] * dn, dr[2] - ni[2] * dn};
-      R pd = pair_dist(dot3<D, R>(pr, pr));
-      bool ok = true;
-      if (rule == 1) {
-        const T4 nrj = b.nr[j];
-        const R nj[3] = {nrj.x, nrj.y, nrj.z};
-        const R ca = r_fabs(dot3<D, R>(ni, nj));
-        if (F32 && fabsf((float)ca - (float)cos_t) <= kBandCos) unc = true;
-        ok = ca > cos_t;
-      }
-      if (ok) {
-        sum += pair_W(kind, ti == SEGMENT_P ? 1 : D - 1, pd, hi, inv_hi);
-        ncount++;
-      }
-    }
-  };
-  if constexpr (F32) {
-    // Positions relative to the warp's anchor (lane 0's anchor cell; lane 0
-    // is active whenever any lane is), in the tile and in the per-lane path
-    // alike, so the particle's own record is not kept across the scan.
-    const float wa[3] = {__shfl_sync(0xffffffffu, (float)a1.x, 0), __shfl_sync(0xffffffffu, (float)a1.y, 0),
-                         __shfl_sync(0xffffffffu, (float)a1.z, 0)};
-    const float pi[3] = {((float)a1.x - wa[0]) * c.geo.Af[0] + (float)a0.x,
-                         ((float)a1.y - wa[1]) * c.geo.Af[1] + (float)a0.y,
-                         D == 3 ? ((float)a1.z - wa[2]) * c.geo.Af[2] + (float)a0.z : 0.f};
-    auto load = [&](int k) {
-      float4 b0, b1;
-      LD::rec(b.rec, k, b0, b1);
-      const float rj = b0.w * (float)cut;
-      const float r2 = rj * rj;
-      return make_float4((b1.x - wa[0]) * c.geo.Af[0] + b0.x, (b1.y - wa[1]) * c.geo.Af[1] + b0.y,
-                         D == 3 ? (b1.z - wa[2]) * c.geo.Af[2] + b0.z : 0.f, b1.w < 0.f ? -r2 : r2);
-    };
-    auto vglob = [&](int j) {
-      const float4 e = load(j);
-      float dr[3] = {pi[0] - e.x, pi[1] - e.y, D == 3 ? pi[2] - e.z : 0.f};
-      const float d2 = d2_of(dr, D);
-      const float Rm = fmaxf((float)R2i, fabsf(e.w));
-      if (d2 > Rm * kD2Accept) return;
-      if (d2 >= Rm * kD2Sure) unc = true;
-      accept(j, (R*)dr, (R)pair_dist(d2), e.w < 0.f);
-    };
-    // A chunk of 32 tile entries in two parts: every entry is tested without
-    // branches into a bit mask, then the lane walks only its own set bits in
-    // ascending order (the candidates' order) to accept them.  Accepting in
-    // the test loop made the whole warp run the accept path for almost every
-    // entry (some lane accepts nearly every candidate), with a third of the
-    // lanes idle.
-    auto test = [&](const float4& e) -> bool {
-      const float dr[3] = {pi[0] - e.x, pi[1] - e.y, D == 3 ? pi[2] - e.z : 0.f};
-      return d2_of(dr, D) <= fmaxf((float)R2i, fabsf(e.w)) * kD2Accept;
-    };
-    auto vchunk = [&](int t0, int m, const float4* tile) {
-      unsigned mask = 0u;
-      if (m == 32) {
-#pragma unroll
-        for (int t = 0; t < 32; t++) mask |= test(tile[t]) ? (1u << t) : 0u;
-      } else {
-        for (int t = 0; t < m; t++) mask |= test(tile[t]) ? (1u << t) : 0u;
-      }
-      while (mask) {
-        const int t = __ffs(mask) - 1;
-        mask &= mask - 1u;
-        const float4 e = tile[t];
-        float dr[3] = {pi[0] - e.x, pi[1] - e.y, D == 3 ? pi[2] - e.z : 0.f};
-        const float d2 = d2_of(dr, D);
-        const float Rm = fmaxf((float)R2i, fabsf(e.w));
-        if (d2 >= Rm * kD2Sure) unc = true;
-        accept(t0 + t, (R*)dr, (R)pair_dist(d2), e.w < 0.f);
-      }
-    };
-    warp_scan<D, R, LD>(c, w.cstart, w.lhmax, active, origin, hi, s_tile[threadIdx.x >> 5], load, vchunk, vglob);
-  } else {
-    auto vglob = [&](int j) {
-      T4 b0, b1;
-      LD::rec(b.rec, j, b0, b1);
-      R dr[3];
-      Q::rel(c, a0, a1, b0, b1, dr);
-      R dist;
-      if (!nb_test(d2_of(dr, D), hi, b0.w, c.prm.cutoff, dist)) return;
-      accept(j, dr, dist, b1.w < (R)0);
-    };
-    auto load = [&](int k) {
-      RecPair<R> e;
-      LD::rec(b.rec, k, e.a, e.b);
-      return e;
-    };
-    auto vchunk = [&](int t0, int m, const RecPair<R>* tile) {
-      for (int t = 0; t < m; t++) {
-        const RecPair<R>& e = tile[t];
-        R dr[3];
-        Q::rel(c, a0, a1, e.a, e.b, dr);
-        R dist;
-        if (!nb_test(d2_of(dr, D), hi, e.a.w, c.prm.cutoff, dist)) continue;
-        accept(t0 + t, dr, dist, e.b.w < (R)0);
-      }
-    };
-    warp_scan<D, R, LD>(c, w.cstart, w.lhmax, active, origin, hi, s_tile[threadIdx.x >> 5], load, vchunk, vglob);
-  }
-  if (active) {
-    if (WEN32 && ti == REAL_P) {
-      sum *= (R)((float)kern_norm(K_WEN, D) * (D == 3 ? inv_hi * inv_hi * inv_hi : inv_hi * inv_hi));
-      ncount = cnt;
-    }
-    if (ncount > 1) sum = (R)1. / (sum + (R)1.e-15);
-    w.sum[i] = sum;
-    w.cnt[i] = cnt;
-    if (cnt > w.cap) atomicOr(&c.sc->flags, (unsigned)FLAG_SPILL);
-    pairs = (unsigned long long)(cnt - 1);
-  }
-  queue_push(active && cnt > w.cap, &c.sc->nspill, w.spillq, (int)i);
-  if (F32) queue_push(active && unc, &c.sc->nfix, w.fixq, (int)i);
-  unsigned mc = (unsigned)(pairs + 1);
-  for (int o = 16; o > 0; o >>= 1) mc = max(mc, __shfl_xor_sync(0xffffffffu, mc, o));
-  if ((threadIdx.x & 31) == 0 && mc > 1) atomicMax(&c.sc->maxcnt, mc);
-  block_sum_u64_to_global(pairs, &c.sc->pairs);
+// Neighbour list of particle i by its group of kG lanes, in the fixed scan
+// order.  Returns the number of neighbours (itself included); the list keeps the
+// first cap.
+template <int D, class R, class LD>
+__device__ inline int list_group(const KCtx& c, const Buf<R>& b, const Work<R>& w, const GroupLanes& g, RowTile& rt,
+                                 long long i) {
+  const PairTest<D, R> pt(c, b.rec, i);
+  const SOrigin<D, R> so(c, b.posh[i], b.key ? b.key[i] : 0);
+  int* row = w.nbl + nb_slot(i, 0, w.cap);  // entry q at row[(q >> 3) * 256 + (q & 7)]
+  int cnt = 0;
+  group_scan<D, R, LD>(c, w, g, rt, i, so, [&](int j, bool in) {
+    const bool ok = in && pt.template near<LD>(c, b.rec, j);
+    const unsigned m = g.ballot(ok);
+    const int pos = cnt + __popc(m & g.below);
+    if (ok && pos < w.cap) row[((pos >> 3) << 8) + (pos & 7)] = j;
+    cnt += __popc(m);
+  });
+  return cnt;
 }
 
-template <int D, class R, int KK>
-__global__ void __launch_bounds__(256, (std::is_same<R, float>::value ? MRSPH_DENSITY_MIN_BLOCKS : 1)) k_density(KCtx c, Buf<R> b, Work<R> w) {
-  density_block<D, R, KK>(c, b, w, blockIdx.x);
+// Neighbour lists of 32 particles by one warp (FP32-split), lane l's particle i.
+// The lanes that sit in neighbouring half cells (a segment: all 32 in the work
+// order, a few groups in storage order) reach nearly the same rows of the
+// sort table.  The lanes take one row each of the segment's bounding box, the
+// rows' particles are loaded once, coalesced, those within reach of the box are
+// put into a tile of 256 candidates in shared memory, and every lane tests
+// the whole tile: with the positions relative to the segment's frame, |p|^2 +
+// |c|^2 - 2 p . c - max(R_i, R_j)^2 takes two candidates at a time (packed FP32:
+// three fused multiply-adds, two additions), and its sign bits shift into a
+// mask.  The expanded form is off by at most 2^-20 (|p|^2 + |c|^2) (four fused
+// operations on values of at most twice that, and the rounding of c); when a
+// candidate of 32 comes closer to zero than that and the criterion's band of
+// 2^-15 R^2, the lane decides the 32 again one by one, else the mask is the
+// decision and the lane appends its set bits.  The tile is kept over rows and
+// levels, so its words are full.  Lanes walking their own rows (430 candidates
+// for 86 neighbours in the relaxed state) ran at a third of the warp's width.
+constexpr int kTile = MRSPH_TILE_SIZE, kTileRows = 64, kSegX = MRSPH_TILE_SPAN_X, kSegYZ = MRSPH_TILE_SPAN_YZ;
+static_assert(kTile % 64 == 0 && kTile <= 1024, "whole mask words, at most 32 of them");
+struct WarpTile {
+  float4 xy[kTile / 2];  // (x0, x1, y0, y1) of two candidates
+  float4 zq[kTile / 2];  // (z0, z1, |c|^2_0, |c|^2_1)
+  float2 nr2[kTile / 2];  // squared cut-off radii, negated
+  int id[kTile];
+  unsigned mask[kTile / 32][32];
+  int off[kTileRows], end[kTileRows];
+};
+__device__ __forceinline__ unsigned long long pack2(float a, float b) {
+  unsigned long long r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+  return r;
+}
+__device__ __forceinline__ unsigned long long fma2(unsigned long long a, unsigned long long b, unsigned long long c) {
+  unsigned long long r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+  return r;
+}
+__device__ __forceinline__ unsigned long long add2(unsigned long long a, unsigned long long b) {
+  unsigned long long r;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+__device__ inline float warp_fmin(float v) {
+  for (int o = 16; o > 0; o >>= 1) v = fminf(v, __shfl_xor_sync(0xffffffffu, v, o));
+  return v;
+}
+__device__ inline float warp_fmax(float v) {
+  for (int o = 16; o > 0; o >>= 1) v = fmaxf(v, __shfl_xor_sync(0xffffffffu, v, o));
+  return v;
 }
 
-// FP32-split density fix-up, one warp per queued particle (grid-stride over
-// warps): every pair of the particle is decided again (FP32 outside the
-// bands, FP64 inside), its list is compacted to the accepted pairs in scan
-// order (the lanes take 32 entries at a time; a ballot gives each accepted
-// entry its new position), surface-filter decisions made in FP64 are marked
-// on their entries (the force passes read the marks), and its kernel sum,
-// count and share of the step's pair total are redone.  The sum has one
-// fixed order whatever the path: the accepted pairs' terms in list order,
-// term p into lane p mod 32's partial sum, the partials folded by a butterfly
-// (xor 16, 8, 4, 2, 1).  The list path stores the terms in the pair
-// coefficient array (which stage 1 overwrites) and sums them strided; a
-// particle whose list spilled re-scans its cells on lane 0, which keeps the
-// 32 partial sums itself and folds them the same way.
-template <int D, int KK, class LD = LdNC>
-__device__ inline void density_fix_items(const KCtx& c, const Buf<float>& b, const Work<float>& w, long long blk,
-                                         long long nblk) {
-  using Q = RecOps<D, float>;
-  constexpr bool WEN = KK == K_WEN;
+template <int D, class LD>
+__device__ inline int list_warp(const KCtx& c, const Buf<float>& b, const Work<float>& w, WarpTile& wt, long long i,
+                                bool act) {
   const unsigned FULL = 0xffffffffu;
-  const unsigned nq = c.sc->nfix;
-  const long long wpb = blockDim.x >> 5;
-  if (blk * wpb >= (long long)nq) return;  // block-uniform: nothing queued for this block
-  const int lane = threadIdx.x & 31;
-  const int kind = KK >= 0 ? KK : c.prm.kernel;
-  const float cut = c.prm.cutoff_f, cos_t = c.prm.cos_thres_f;
-  for (long long t = blk * wpb + (threadIdx.x >> 5); t < nq; t += nblk * wpb) {  // warp-uniform
-    const int i = w.fixq[t];
-    const float4 a0 = b.rec[2 * i], a1 = b.rec[2 * i + 1];
-    const int ti = b.meta[i] & 0xFF;
-    float ni[3] = {0.f, 0.f, 0.f};
-    if (ti != REAL_P) {
-      const float4 q = b.nr[i];
-      ni[0] = q.x; ni[1] = q.y; ni[2] = q.z;
+  const int lane = threadIdx.x & 31, BIG = 0x3fffffff;
+  float4 a0 = make_float4(0.f, 0.f, 0.f, 0.f);
+  int k[3] = {0, 0, 0}, own = 0;
+  if (act) {
+    a0 = b.rec[2 * i];
+    PosOps<D, float>::unpack(b.key[i], k);
+    own = (int)(signed char)((b.meta[i] >> 8) & 0xFF);
+  }
+  const float cut = c.prm.cutoff_f, nR2i = -((a0.w * cut) * (a0.w * cut));
+  const int cap = w.cap;
+  int* row = w.nbl + nb_slot(act ? i : 0, 0, cap);  // entry q at row[(q >> 3) * 256 + (q & 7)]
+  int cnt = 0;
+  unsigned rem = __ballot_sync(FULL, act);
+  while (rem) {
+    // the segment: the lanes within kSegX half cells of the first left, in x,
+    // and kSegYZ in y and z (of its level; anchor cells are 2^-sh of a level's cell)
+    const int seed = __ffs(rem) - 1;
+    bool in = (rem >> lane) & 1u;
+    const int sh = c.geo.ncl - 1 - __shfl_sync(FULL, own, seed);
+    const int span = ((kSegX + 1) << sh) >> 1, span1 = ((kSegYZ + 1) << sh) >> 1;
+    int ks[3];
+    for (int d = 0; d < 3; d++) {
+      ks[d] = __shfl_sync(FULL, k[d], seed);
+      if (d < D) in = in && abs(k[d] - ks[d]) <= (d == 0 ? span : span1);
     }
-    const bool char_i = ti == SURFACE_P || (D == 3 && ti == SEGMENT_P);
-    const float hi = a0.w, inv_hi = r_rcp(hi);
-    const float R2i = (hi * cut) * (hi * cut);
-    const int old = w.cnt[i];
-    const long long base = nb_slot(i, 0, w.cap);
-    int* row = w.nbl + base;
-    float* prow = w.pc + base;
-    // decision of pair (i, j): false if j is no neighbour; else e = j with
-    // the surface-filter mark, term its kernel-sum term and counted whether
-    // it counts towards ncount (generic kernels)
-    auto visit = [&](int j, int& e, float& term, bool& counted) -> bool {
-      float4 b0, b1;
-      LD::rec(b.rec, j, b0, b1);
-      float dr[3];
-      Q::rel(c, a0, a1, b0, b1, dr);
-      const float d2 = d2_of(dr, D);
-      const float rj = b0.w * cut;
-      const float Rm = fmaxf(R2i, rj * rj);
-      if (d2 > Rm * kD2Accept) return false;
-      if (d2 >= Rm * kD2Sure && !exact_neighbor<D>(c, a0, a1, b0, b1)) return false;
-      e = j;
-      term = 0.f;
-      counted = false;
-      const float dist = pair_dist(d2);
-      if (ti == REAL_P) {
-        if (WEN) {
-          const float s = dist * inv_hi;
-          const float tt = fmaxf(fmaf(-0.5f, s, 1.f), 0.f), t2 = tt * tt;
-          term = (t2 * t2) * fmaf(2.f, s, 1.f);
-        } else {
-          term = pair_W(kind, D, dist, hi, inv_hi);
-          counted = true;
+    rem &= ~__ballot_sync(FULL, in);
+    // frame: the middle anchor in x, the seed's in y and z; bounding box
+    ks[0] = (__reduce_min_sync(FULL, in ? k[0] : BIG) + __reduce_max_sync(FULL, in ? k[0] : -1)) >> 1;
+    float p[3] = {0.f, 0.f, 0.f}, lo[3] = {0.f, 0.f, 0.f}, hi[3] = {0.f, 0.f, 0.f};
+    const float ao[3] = {a0.x, a0.y, a0.z};
+    for (int d = 0; d < D; d++) {
+      p[d] = fmaf((float)(k[d] - ks[d]), c.geo.Af[d], ao[d]);
+      lo[d] = warp_fmin(in ? p[d] : 3.e38f);
+      hi[d] = warp_fmax(in ? p[d] : -3.e38f);
+    }
+    const float Rm2 = __int_as_float(__reduce_max_sync(FULL, in ? __float_as_int(-nR2i) : 0));  // largest R_i^2
+    const float fk[3] = {(float)ks[0], (float)ks[1], (float)ks[2]};
+    const float pp = p[0] * p[0] + p[1] * p[1] + p[2] * p[2];
+    const unsigned long long pp2 = pack2(pp, pp);
+    const unsigned long long mx = pack2(-2.f * p[0], -2.f * p[0]), my = pack2(-2.f * p[1], -2.f * p[1]);
+    const unsigned long long mz = pack2(-2.f * p[2], -2.f * p[2]);
+    int tn = 0;         // candidates in the tile
+    float qmax = 0.f;   // this lane's largest |c|^2 and R_j^2 among those it put there
+    float rmax = 0.f;
+    // tests the tile's candidates, appends the hits, empties the tile
+    auto drain = [&]() {
+      const int nw = (tn + 31) >> 5, pad = (nw << 5) - tn;
+      if (lane < pad) {
+        const int t = tn + lane, s2 = 4 * (t >> 1) + (t & 1);
+        float* xy = reinterpret_cast<float*>(wt.xy);
+        float* zq = reinterpret_cast<float*>(wt.zq);
+        xy[s2] = xy[s2 + 2] = zq[s2] = 0.f;
+        zq[s2 + 2] = 3.e38f;  // |c|^2: never in reach
+        reinterpret_cast<float*>(wt.nr2)[t] = 0.f;
+      }
+      const float qm = __int_as_float(__reduce_max_sync(FULL, __float_as_int(qmax)));
+      const float rm = __int_as_float(__reduce_max_sync(FULL, __float_as_int(rmax)));
+      const float band = fmaf(fmaxf(-nR2i, rm), 0x1.1p-15f, 0x1p-20f * (pp + qm));
+      __syncwarp();
+      unsigned slow = 0u, hits = 0u;
+      for (int v = 0; v < nw; v++) {
+        unsigned mask = 0u;
+        float close = 3.e38f;
+#pragma unroll
+        for (int t = 0; t < 16; t++) {
+          const ulonglong2 xy = *reinterpret_cast<const ulonglong2*>(&wt.xy[v * 16 + t]);
+          const ulonglong2 zq = *reinterpret_cast<const ulonglong2*>(&wt.zq[v * 16 + t]);
+          const float2 nr = wt.nr2[v * 16 + t];
+          unsigned long long s = add2(zq.y, pp2);
+          if (D == 3) s = fma2(zq.x, mz, s);
+          s = fma2(xy.y, my, s);
+          s = fma2(xy.x, mx, s);
+          s = add2(s, pack2(fminf(nR2i, nr.x), fminf(nR2i, nr.y)));
+          const unsigned s0 = (unsigned)s, s1 = (unsigned)(s >> 32);
+          mask = __funnelshift_l(s0, mask, 1);
+          mask = __funnelshift_l(s1, mask, 1);
+          close = fminf(close, fminf(fabsf(__uint_as_float(s0)), fabsf(__uint_as_float(s1))));
         }
-      } else if (char_i && b1.w < 0.f) {
-        const int rule = char_pair(ti, b.meta[j] & 0xFF);
-        if (rule == 0) return true;
-        const float dn = dot3<D, float>(dr, ni);
-        float pr[3] = {dr[0] - ni[0] * dn, dr[1] - ni[1] * dn, dr[2] - ni[2] * dn};
-        const float pd = pair_dist(dot3<D, float>(pr, pr));
-        bool ok = true;
-        if (rule == 1) {
-          const float4 q = b.nr[j];
-          const float nj[3] = {q.x, q.y, q.z};
-          const float ca = fabsf(dot3<D, float>(ni, nj));
-          if (fabsf(ca - cos_t) <= kBandCos) {
-            ok = exact_cos<D>(c, ni, nj);
-            e |= (int)((ok ? NB_COS_OK : NB_COS_NO) << 30);
-          } else {
-            ok = ca > cos_t;
+        if (in) {
+          if (close <= band) slow |= 1u << v;
+          if (mask) hits |= 1u << v;
+          wt.mask[v][lane] = mask;
+        }
+      }
+      // a candidate within the band: its 32 again one by one, decided as the reference does
+      while (slow) {
+        const int v = __ffs(slow) - 1;
+        slow &= slow - 1u;
+        const PairTest<D, float> pt(c, b.rec, i);
+        unsigned mask = 0u;
+        for (int t = 0; t < min(32, tn - 32 * v); t++)
+          if (pt.template near<LD>(c, b.rec, wt.id[32 * v + t])) mask |= 0x80000000u >> t;
+        wt.mask[v][lane] = mask;
+        hits = mask ? hits | (1u << v) : hits & ~(1u << v);
+      }
+      __syncwarp();
+      // accept: candidate 32 v + t is bit 31 - t of word v; a lane goes on to its
+      // next word as soon as one is used up
+      unsigned mk = 0u;
+      const int* id = wt.id;
+      while (hits | mk) {
+        if (!mk) {
+          const int v = __ffs(hits) - 1;
+          hits &= hits - 1u;
+          mk = wt.mask[v][lane];
+          id = wt.id + 32 * v;
+        }
+        const int t = __clz(mk);
+        mk &= ~(0x80000000u >> t);
+        if (cnt < cap) row[((cnt >> 3) << 8) + (cnt & 7)] = id[t];
+        cnt++;
+      }
+      __syncwarp();
+      tn = 0;
+      qmax = 0.f;
+      rmax = 0.f;
+    };
+    int nrow = 0, T = 0;
+    // puts the rows' candidates that lie within reach of the box into the tile
+    auto take_rows = [&]() {
+      __syncwarp();
+      int r = 0;
+      for (int t0 = 0; t0 < T; t0 += 32) {
+        const int t = t0 + lane;
+        float e[3] = {0.f, 0.f, 0.f}, rr = 0.f;
+        int j = 0;
+        bool keep = false;
+        if (t < T) {
+          while (t >= wt.end[r]) r++;
+          j = wt.off[r] + t;
+          float4 b0, b1;
+          LD::rec(b.rec, j, b0, b1);
+          e[0] = fmaf(b1.x - fk[0], c.geo.Af[0], b0.x);
+          e[1] = fmaf(b1.y - fk[1], c.geo.Af[1], b0.y);
+          if (D == 3) e[2] = fmaf(b1.z - fk[2], c.geo.Af[2], b0.z);
+          const float rj = b0.w * cut;
+          rr = rj * rj;
+          float d2 = 0.f;
+          for (int d = 0; d < D; d++) {
+            const float gd = fmaxf(fmaxf(lo[d] - e[d], e[d] - hi[d]), 0.f);
+            d2 = fmaf(gd, gd, d2);
+          }
+          keep = d2 <= fmaxf(Rm2, rr) * 1.0002f;
+        }
+        const unsigned m = __ballot_sync(FULL, keep);
+        if (keep) {
+          const int at = tn + __popc(m & ((1u << lane) - 1u)), s2 = 4 * (at >> 1) + (at & 1);
+          const float q = fmaf(e[2], e[2], fmaf(e[1], e[1], e[0] * e[0]));
+          float* xy = reinterpret_cast<float*>(wt.xy);
+          float* zq = reinterpret_cast<float*>(wt.zq);
+          xy[s2] = e[0];
+          xy[s2 + 2] = e[1];
+          zq[s2] = e[2];
+          zq[s2 + 2] = q;
+          reinterpret_cast<float*>(wt.nr2)[at] = -rr;
+          wt.id[at] = j;
+          qmax = fmaxf(qmax, q);
+          rmax = fmaxf(rmax, rr);
+        }
+        tn += __popc(m);
+        if (tn > kTile - 32) drain();
+      }
+      __syncwarp();
+      nrow = 0;
+      T = 0;
+    };
+    for (int L = 0; L < c.geo.ncl; L++) {
+      if (c.sc->lcount[L] == 0) continue;
+      const float R = warp_fmax(in ? LD::ld(&w.rlev[(long long)L * c.n + i]) : 0.f);
+      if (!(R > 0.f)) continue;
+      const float R2 = R * R;
+      // half cell h of axis d covers [(h - h0) hs - f0, + hs) of the frame
+      const int shl = c.geo.ncl - 1 - L;
+      int h0[3] = {0, 0, 0}, r0[3] = {0, 0, 0}, r1[3] = {0, 0, 0};
+      float f0[3] = {0.f, 0.f, 0.f};
+      for (int d = 0; d < D; d++) {
+        if (shl == 0) h0[d] = 2 * ks[d];
+        else {
+          h0[d] = ks[d] >> (shl - 1);
+          f0[d] = (float)(ks[d] & ((1 << (shl - 1)) - 1)) * c.geo.Af[d];
+        }
+        const float ih = c.geo.ihs_f[L][d];
+        r0[d] = max(h0[d] + (int)floorf((lo[d] - R + f0[d]) * ih), 0);
+        r1[d] = min(h0[d] + (int)floorf((hi[d] + R + f0[d]) * ih), c.geo.hn[L][d] - 1);
+      }
+      if (r1[0] < r0[0] || r1[1] < r0[1] || r1[2] < r0[2]) continue;
+      if (w.bstart && (r1[1] - r0[1] + 1) * (r1[2] - r0[2] + 1) > 64) {
+        // many rows (a finer level): cut them to the bricks that hold particles
+        const int b0y = r0[1] >> 2, b0z = r0[2] >> 2;
+        const int nby = (r1[1] >> 2) - b0y + 1, nbz = (r1[2] >> 2) - b0z + 1;
+        int ymin = BIG, ymax = -1, zmin = BIG, zmax = -1;
+        for (int t = lane; t < nby * nbz; t += 32) {
+          const int z = b0z + t / nby, y = b0y + t % nby;
+          const long long at = c.geo.boff[L] + ((long long)z * c.geo.bn[L][1] + y) * c.geo.bn[L][0];
+          if (LD::ld(&w.bstart[at + (r1[0] >> 2) + 1]) > LD::ld(&w.bstart[at + (r0[0] >> 2)])) {
+            ymin = min(ymin, y); ymax = max(ymax, y);
+            zmin = min(zmin, z); zmax = max(zmax, z);
           }
         }
-        if (ok) {
-          term = pair_W(kind, ti == SEGMENT_P ? 1 : D - 1, pd, hi, inv_hi);
-          counted = true;
+        ymax = __reduce_max_sync(FULL, ymax);
+        if (ymax < 0) continue;
+        ymin = __reduce_min_sync(FULL, ymin);
+        r0[1] = max(r0[1], 4 * ymin);
+        r1[1] = min(r1[1], 4 * ymax + 3);
+        if (D == 3) {
+          r0[2] = max(r0[2], 4 * __reduce_min_sync(FULL, zmin));
+          r1[2] = min(r1[2], 4 * __reduce_max_sync(FULL, zmax) + 3);
         }
       }
-      return true;
-    };
-    int cnt = 0, ncount = 0;
-    float sum = 0.f;
-    if (old <= w.cap) {
-      // the list holds every candidate the FP32 test did not certainly
-      // reject; each chunk of 32 entries is read before any of it is written,
-      // and an accepted entry moves to a position <= its own
-      for (int q0 = 0; q0 < old; q0 += 32) {
-        const int q = q0 + lane;
-        int e = 0;
-        float term = 0.f;
-        bool acc = false, counted = false;
-        if (q < old) acc = visit(nb_index(LD::ld(&row[((q >> 3) << 8) + (q & 7)])), e, term, counted);
-        const unsigned m = __ballot_sync(FULL, acc);
-        ncount += __popc(__ballot_sync(FULL, acc && counted));
-        if (acc) {
-          const int pos = cnt + __popc(m & ((1u << lane) - 1u));
-          const int o = ((pos >> 3) << 8) + (pos & 7);
-          row[o] = e;
-          prow[o] = term;
+      const int ny = r1[1] - r0[1] + 1, nr = ny * (r1[2] - r0[2] + 1);
+      for (int rb = 0; rb < nr; rb += 32) {
+        const int rr = rb + lane;
+        int s0 = 0, e0 = 0;
+        if (rr < nr) {
+          const int iz = D == 3 ? rr / ny : 0;
+          const int z = r0[2] + iz, y = r0[1] + rr - iz * ny;
+          float gz = 0.f, gy = 0.f;
+          if (D == 3) {
+            const float zl = fmaf((float)(z - h0[2]), c.geo.hs_f[L][2], -f0[2]);
+            if (z > 0) gz = fmaxf(gz, zl - hi[2]);
+            if (z < c.geo.hn[L][2] - 1) gz = fmaxf(gz, lo[2] - (zl + c.geo.hs_f[L][2]));
+          }
+          const float yl = fmaf((float)(y - h0[1]), c.geo.hs_f[L][1], -f0[1]);
+          if (y > 0) gy = fmaxf(gy, yl - hi[1]);
+          if (y < c.geo.hn[L][1] - 1) gy = fmaxf(gy, lo[1] - (yl + c.geo.hs_f[L][1]));
+          const float left = R2 - gy * gy - gz * gz;
+          if (left >= 0.f) {
+            const float wd = sqrtf(left), ih = c.geo.ihs_f[L][0];
+            const int xl = max(h0[0] + (int)floorf((lo[0] - wd + f0[0]) * ih), 0);
+            const int xh = min(h0[0] + (int)floorf((hi[0] + wd + f0[0]) * ih), c.geo.hn[L][0] - 1);
+            if (xl <= xh) {
+              const long long at = c.geo.hoff[L] + ((long long)z * c.geo.hn[L][1] + y) * c.geo.hn[L][0];
+              s0 = LD::ld(&w.cstart[at + xl]);
+              e0 = LD::ld(&w.cstart[at + xh + 1]);
+            }
+          }
         }
-        cnt += __popc(m);
-        __syncwarp();
-      }
-      for (int p = lane; p < cnt; p += 32) sum += LD::ld(&prow[((p >> 3) << 8) + (p & 7)]);
-      for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(FULL, sum, o);
-    } else {
-      if (lane == 0) {
-        float part[32];
-        for (int l = 0; l < 32; l++) part[l] = 0.f;
-        const SOrigin<D, float> so(c, b.posh[i], b.key[i]);
-        scan_candidates<D, float, LD>(c, w.cstart, w.lhmax, so, hi, [&](int j) {
-          int e = 0;
-          float term = 0.f;
-          bool counted = false;
-          if (!visit(j, e, term, counted)) return;
-          if (cnt < w.cap) row[((cnt >> 3) << 8) + (cnt & 7)] = e;
-          part[cnt & 31] += term;
-          ncount += counted ? 1 : 0;
-          cnt++;
-        });
-        for (int o = 16; o > 0; o >>= 1) {
-          float nxt[32];
-          for (int l = 0; l < 32; l++) nxt[l] = part[l] + part[l ^ o];
-          for (int l = 0; l < 32; l++) part[l] = nxt[l];
+        const int len = max(e0 - s0, 0);
+        const unsigned full = __ballot_sync(FULL, len > 0);
+        if (!full) continue;
+        int inc = len;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+          const int t = __shfl_up_sync(FULL, inc, o);
+          if (lane >= o) inc += t;
         }
-        sum = part[0];
+        if (nrow + __popc(full) > kTileRows) take_rows();
+        if (len > 0) {
+          const int at = nrow + __popc(full & ((1u << lane) - 1u));
+          wt.off[at] = s0 - (T + inc - len);
+          wt.end[at] = T + inc;
+        }
+        nrow += __popc(full);
+        T += __shfl_sync(FULL, inc, 31);
       }
-      cnt = __shfl_sync(FULL, cnt, 0);
-      ncount = __shfl_sync(FULL, ncount, 0);
     }
-    if (lane == 0) {
-      if (WEN && ti == REAL_P) {
-        sum *= (float)kern_norm(K_WEN, D) * (D == 3 ? inv_hi * inv_hi * inv_hi : inv_hi * inv_hi);
-        ncount = cnt;
-      }
-      if (ncount > 1) sum = 1.f / (sum + 1.e-15f);
-      w.sum[i] = sum;
-      w.cnt[i] = cnt;
-      atomicAdd(&c.sc->pairs, (unsigned long long)(long long)(cnt - old));
-    }
-    __syncwarp();
+    if (T > 0) take_rows();
+    if (tn > 0) drain();
+  }
+  return cnt;
+}
+
+// what follows a list: its length, the spill queue, the step's totals
+template <int D, class R>
+__device__ inline void list_done(const KCtx& c, const Work<R>& w, long long i, int cnt, bool lead) {
+  if (lead) {
+    w.cnt[i] = cnt;
+    if (cnt > w.cap) atomicOr(&c.sc->flags, (unsigned)FLAG_SPILL);
+  }
+  queue_push(lead && cnt > w.cap, &c.sc->nspill, w.spillq, (int)i);
+  const unsigned mc = __reduce_max_sync(0xffffffffu, (unsigned)cnt);
+  const unsigned ps = __reduce_add_sync(0xffffffffu, lead ? (unsigned)(cnt - 1) : 0u);
+  if ((threadIdx.x & 31) == 0) {
+    if (mc > 1) atomicMax(&c.sc->maxcnt, mc);
+    if (ps) atomicAdd(&c.sc->pairs, (unsigned long long)ps);
   }
 }
 
-template <int D, int KK>
-__global__ void __launch_bounds__(256) k_density_fix(KCtx c, Buf<float> b, Work<float> w) {
-  density_fix_items<D, KK>(c, b, w, blockIdx.x, gridDim.x);
+// particles [first, first + blockDim.x / kG), a group each
+template <int D, class R, class LD = LdNC>
+__device__ inline void density_group_block(const KCtx& c, const Buf<R>& b, const Work<R>& w, RowTile* tiles,
+                                           long long first) {
+  const GroupLanes g;
+  const long long i = first + threadIdx.x / kG;
+  int cnt = 0;
+  if (i < c.n) cnt = list_group<D, R, LD>(c, b, w, g, tiles[threadIdx.x / kG], i);
+  __syncwarp();
+  list_done<D, R>(c, w, i, cnt, i < c.n && g.gl == 0);
+}
+
+// particles [first, first + blockDim.x), one warp per 32
+template <int D, class LD = LdNC>
+__device__ inline void density_warp_block(const KCtx& c, const Buf<float>& b, const Work<float>& w, WarpTile* tiles,
+                                          long long first) {
+  const long long t = first + threadIdx.x;
+  const bool act = t < c.n;
+  const long long i = act && w.order ? w.order[t] : t;
+  const int cnt = list_warp<D, LD>(c, b, w, tiles[threadIdx.x >> 5], i, act);
+  list_done<D, float>(c, w, i, cnt, act);
+}
+
+constexpr int kDensityThreads = 128;
+template <int D, class R>
+__global__ void __launch_bounds__(kDensityThreads, 10) k_density_group(KCtx c, Buf<R> b, Work<R> w) {
+  __shared__ RowTile tiles[kDensityThreads / kG];
+  density_group_block<D, R>(c, b, w, tiles, (long long)blockIdx.x * (kDensityThreads / kG));
+}
+template <int D>
+__global__ void __launch_bounds__(kDensityThreads, MRSPH_DENSITY_MIN_BLOCKS) k_density(KCtx c, Buf<float> b, Work<float> w) {
+  __shared__ WarpTile tiles[kDensityThreads / 32];
+  density_warp_block<D>(c, b, w, tiles, (long long)blockIdx.x * kDensityThreads);
 }
 
 __device__ inline void accum_pairs_body(DevScalars* sc) { sc->pairs_total += sc->pairs; }
-static __global__ void k_accum_pairs(DevScalars* sc) { accum_pairs_body(sc); }
 
 // four consecutive pair coefficients (16-byte aligned)
 __device__ inline void store4(float* p, const float* v) {
@@ -1461,14 +1619,24 @@ __device__ inline void load4(const double* p, double* v) {
   v[0] = t0.x; v[1] = t0.y; v[2] = t1.x; v[3] = t1.y;
 }
 
-// A8 force stages + A9 timestep (Set_timestep(stage), particle_mesh_generation.cpp:127-145).
-// Stage 1 evaluates each pair's kernel gradient aw and stores, in the
-// neighbour list's layout, the pair coefficient c_ij = aw * (1/rho_i^2 +
-// 1/rho_j^2) (0 for a pair the forces skip), and per particle (a1, eta),
-// eta = nu * rho, negated for a particle that is not REAL.  The stage-2 viscous term
-// of a pair is c_ij * eta_ij * (v_i - v_j) (:1021-1049), so stage 2 reads the
-// coefficient and one vector per neighbour; a particle whose list spilled
-// re-scans its cells and recomputes c_ij in both stages.
+// A7 Get_kernel_summation (particle_mesh_generation.cpp:690-765), A8 force
+// stages, A9 timestep (Set_timestep(stage), :127-145).
+// Stage 1 forms the kernel sum and the pressure force together: the force of a
+// pair is sum_i * c_ij dr_ij with the pair coefficient c_ij = aw * (1/rho_i^2 +
+// 1/rho_j^2), so the inverted sum scales the accumulated force at the end and
+// the distance is computed once.  It stores c_ij in the neighbour list's layout (0
+// for a pair the forces skip), and per particle (a1, eta), eta = nu * rho, negated for a
+// particle that is not REAL.  The stage-2 viscous term of a pair is c_ij * eta_ij *
+// (v_i - v_j) (:1021-1049), so stage 2 reads the coefficient and one vector per
+// neighbour; a particle whose list spilled re-scans its cells and recomputes c_ij
+// in both stages.  Stage 0 forms the kernel sum alone (a step that stops after
+// the density phase).
+// A particle is taken by one thread (G = 1) or by a group of kG lanes (G = kG),
+// which share its entries kG at a time and hand their terms to lanes 0 to 3,
+// one per component, to be added in list order: the sums, and so every bit,
+// are the same.  One thread is the cheaper form once the chip is full; below
+// that a group shortens the chain of gathers that bounds the kernel (see
+// kGroupMax).
 // FP32 Wendland C2 gradient over distance in DK dimensions (0 in 1D, the
 // reference's quirk), Derivative_kernel_function (particle.cpp:732-750):
 // -5 C (1 - s/2)^3 s / h / (r + 1e-15) with C = norm / h^DK and s = r / h,
@@ -1488,226 +1656,290 @@ __device__ inline float wendland_aw(float dist, float h) {
   return dist > 0.f ? (-5.f * (float)kern_norm(K_WEN, DK)) * ihp * (t * t * t) : 0.f;
 }
 
-// One particle of a force stage.  SPILL = false: the particle's list is
-// complete (cnt <= cap); SPILL = true: it spilled and re-scans its cells,
-// making the neighbour and surface-filter decisions as the density pass does
-// (FP32-split: exact inside the bands).  my_dt / my_v take the min / max.
-template <int D, class R, int STAGE, int KK, bool SPILL, class LD = LdNC>
-__device__ inline void force_particle(const KCtx& c, const Buf<R>& b, const Work<R>& w, long long i, double& my_dt,
-                                      double& my_v) {
+// Shared memory of a group of kG lanes.
+template <class R>
+struct GroupTile {
+  RowTile rows;       // the candidate scan of a spilled particle
+  int vlist[2 * kG];  // its neighbours, kG at a time
+  R term[4][kG];      // force components and kernel-sum term of the entries in hand
+};
+
+// One particle of a force stage.  SPILL = false: the particle's list is complete
+// (cnt <= cap); SPILL = true: it spilled, and its cells are scanned for the
+// list's entries in their order, so a spill changes nothing.  my_dt / my_v take
+// the min / max (of the group's first lane).
+template <int D, class R, int STAGE, int KK, int G, bool SPILL, class LD = LdNC>
+__device__ inline void force_particle(const KCtx& c, const Buf<R>& b, const Work<R>& w, const GroupLanes& g,
+                                      GroupTile<R>* gt, long long i, double& my_dt, double& my_v) {
   using Q = RecOps<D, R>;
   constexpr bool F32 = std::is_same<R, float>::value;
   constexpr bool WEN32 = F32 && KK == K_WEN;
+  constexpr bool GEO = STAGE < 2 || SPILL;  // the pair geometry is needed
   using T4 = typename V4<R>::T;
   const T4 a0 = b.rec[2 * i], a1r = b.rec[2 * i + 1];
-  const int mi = b.meta[i];
-  const int ti = mi & 0xFF;
+  const int ti = b.meta[i] & 0xFF;
+  const int kind = KK >= 0 ? KK : c.prm.kernel;
   R ni[3] = {0, 0, 0};
   if (ti != REAL_P) {
     const T4 nri = b.nr[i];
     ni[0] = nri.x; ni[1] = nri.y; ni[2] = nri.z;
   }
   const R rho = b.nr[i].w, h = a0.w;
-  const R cos_t = pick<R>(c.prm.cos_thres, c.prm.cos_thres_f);
-  const R sum = (STAGE == 1) ? w.sum[i] : (R)0;
-  R nu = 0, eta_i = 0;
-  R hdt1 = 0;
+  const R inv_h = STAGE < 2 ? pair_inv(h) : (R)0;
+  R eta_i = 0, hdt1 = 0;
   R vi[3] = {0, 0, 0};
   if (STAGE == 2) {
     hdt1 = (R)(0.5 * bitsd(c.sc->dt1));
-    T4 an = w.a1[i];
-    vi[0] = an.x * hdt1; vi[1] = an.y * hdt1; vi[2] = an.z * hdt1;
+    const T4 an = w.a1[i];
+    vi[0] = rmul(an.x, hdt1); vi[1] = rmul(an.y, hdt1); vi[2] = rmul(an.z, hdt1);
     eta_i = r_fabs(an.w);
-  } else {
-    nu = b.nu[i];
   }
   // FP32-split accumulates a particle's pair forces in groups of four list
-  // entries (a candidate scan groups its accepted neighbours the same way)
-  // and adds each group's sum into F with compensated (Kahan) summation.  The
-  // list is in scan order (levels, then z, y rows), so a plain running sum
-  // first collects every same-signed term of one side and reaches about half
-  // of sum |terms| before the other side cancels it; rounding at that
+  // entries and adds each group's sum into F with compensated (Kahan)
+  // summation.  The list is in scan order (levels, then z, y rows), so a plain
+  // running sum first collects every same-signed term of one side and reaches
+  // about half of sum |terms| before the other side cancels it; rounding at that
   // magnitude, not the terms, dominated the FP32 error.  FP64-plain sums
-  // plainly, in the reference's expression order.
+  // plainly.  G = 1: components 0..2; G = kG: lane d < 3 holds component d in
+  // F[0] (and lane 3 the kernel sum in sum).
   R F[3] = {0, 0, 0}, Fb[3] = {0, 0, 0}, Fc[3] = {0, 0, 0};
+  R sum = 0;
+  int ncount = 0;
   auto accum = [&](int d, R v) {
-    if constexpr (F32) Fb[d] = Fb[d] + v;
+    if constexpr (F32) Fb[d] = radd(Fb[d], v);
     else F[d] = F[d] + v;
   };
-  auto flush = [&]() {
+  auto flush = [&](int d) {
     if constexpr (F32) {
-      for (int d = 0; d < D; d++) {
-        const float y = Fb[d] - Fc[d];
-        const float t = F[d] + y;
-        Fc[d] = (t - F[d]) - y;
-        F[d] = t;
-        Fb[d] = 0.f;
-      }
+      const float y = Fb[d] - Fc[d];
+      const float t = F[d] + y;
+      Fc[d] = (t - F[d]) - y;
+      F[d] = t;
+      Fb[d] = 0.f;
     }
   };
   const R vol_i = (R)1.0 / (rho * rho);
-  // pair (i, j) at relative position vec: the skip rules of :1019-1031 and
-  // :904-920, the direction dr the force acts along and the coefficient.
-  // mark: the surface filter's FP64 decision from the density fix-up (0: none)
-  auto coef = [&](int j, const T4& b0, const T4& b1, const R* vec, R* dr, R& cij, unsigned mark) -> bool {
-    if (j == (int)i) return false;
-    int rule = 0;
-    if (ti != REAL_P) {  // SURFACE or SEGMENT: j must not be REAL
-      if (!(b1.w < (R)0)) return false;
-      rule = char_pair(ti, b.meta[j] & 0xFF);
-      if (rule == 0) return false;
-    }
-    R aw;
+  const R CW = (!F32 && STAGE < 2) ? kernel_C<R>(kind, D, h) : (R)0;
+  // kernel-sum term of a pair at distance r in dim dimensions
+  auto W = [&](int dim, R r) -> R {
+    if constexpr (F32) return kernel_W_fast(kind, dim, (float)r, (float)inv_h);
+    else return dim == D ? kernel_W_C<R>(kind, dim, r, h, CW) : kernel_W<R>(kind, dim, r, h);
+  };
+  // pair (i, j): the skip rules of :717-759, :904-920 and :1019-1031; its
+  // kernel-sum term wt (true when it counts), and the pair coefficient cij and
+  // the direction dr its force acts along (cij = 0: no force)
+  auto pair = [&](int j, R* dr, R& cij, R& wt) -> bool {
+    T4 b0, b1;
+    LD::rec(b.rec, j, b0, b1);
+    Q::rel(c, a0, a1r, b0, b1, dr);
     const R hij = (R)0.5 * (h + b0.w);
+    cij = 0;
+    wt = 0;
     if (ti == REAL_P) {
-      dr[0] = vec[0]; dr[1] = vec[1]; dr[2] = vec[2];
-      R dist = force_dist(dot3<D, R>(dr, dr));
-      if constexpr (WEN32) aw = wendland_aw<D>(dist, hij);
-      else aw = pair_dW(c.prm.kernel, D, dist, hij);
-    } else {
-      R dn = dot3<D, R>(vec, ni);
-      dr[0] = vec[0] - ni[0] * dn; dr[1] = vec[1] - ni[1] * dn; dr[2] = vec[2] - ni[2] * dn;
-      R dist = force_dist(dot3<D, R>(dr, dr));
-      bool ok = true;
-      if (rule == 1) {
-        if (mark == NB_COS_OK) {
-          ok = true;
-        } else if (mark == NB_COS_NO) {
-          ok = false;
+      const R dist = force_dist(dot3<D, R>(dr, dr));
+      if (STAGE < 2) {
+        if constexpr (WEN32) {
+          // (1 - s/2)^4 (1 + 2s), s = r/h, clamped at s = 2; the
+          // normalisation C/h^D comes once at the end
+          const float s = (float)dist * (float)inv_h;
+          const float t = fmaxf(fmaf(-0.5f, s, 1.f), 0.f), t2 = t * t;
+          wt = rmul(t2 * t2, fmaf(2.f, s, 1.f));
         } else {
-          const T4 nrj = b.nr[j];
-          const R nj[3] = {nrj.x, nrj.y, nrj.z};
-          const R ca = r_fabs(dot3<D, R>(ni, nj));
-          ok = ca > cos_t;
-          if constexpr (F32 && SPILL) {
-            if (fabsf(ca - cos_t) <= kBandCos) ok = exact_cos<D>(c, (const float*)ni, (const float*)nj);
-          }
+          wt = W(D, dist);
         }
       }
+      if (STAGE > 0 && j != (int)i) {
+        R aw;
+        if constexpr (WEN32) aw = wendland_aw<D>(dist, hij);
+        else aw = pair_dW(kind, D, dist, hij);
+        cij = aw * (vol_i + r_fabs(b1.w));
+      }
+      return true;
+    }
+    if (!(b1.w < (R)0)) return false;  // SURFACE or SEGMENT: j must not be REAL
+    const int rule = char_pair(ti, b.meta[j] & 0xFF);
+    if (rule == 0) return false;
+    const R dn = dot3<D, R>(dr, ni);
+    for (int d = 0; d < 3; d++) dr[d] = madd(-ni[d], dn, dr[d]);
+    if (rule == 1) {
+      const T4 nrj = b.nr[j];
+      const R nj[3] = {nrj.x, nrj.y, nrj.z};
+      const R ca = r_fabs(dot3<D, R>(ni, nj)), cos_t = pick<R>(c.prm.cos_thres, c.prm.cos_thres_f);
+      bool ok = ca > cos_t;
+      if constexpr (F32) {
+        if (fabsf(ca - cos_t) <= kBandCos) ok = exact_cos<D>(c, (const float*)ni, (const float*)nj);
+      }
       if (!ok) return false;
+    }
+    const R dist = force_dist(dot3<D, R>(dr, dr));
+    if (STAGE > 0 && j != (int)i) {
+      R aw;
       if (ti == SEGMENT_P) {  // the 1D kernel gradient in 3D, none in 2D (:769-879)
         if constexpr (WEN32) aw = wendland_aw<1>(dist, hij);
-        else aw = (D == 3) ? pair_dW(c.prm.kernel, 1, dist, hij) : (R)0;
+        else aw = (D == 3) ? pair_dW(kind, 1, dist, hij) : (R)0;
       } else {
         if constexpr (WEN32) aw = wendland_aw<D - 1>(dist, hij);
-        else aw = pair_dW(c.prm.kernel, D - 1, dist, hij);
+        else aw = pair_dW(kind, D - 1, dist, hij);
       }
+      cij = aw * (vol_i + r_fabs(b1.w));
     }
-    const R vol_ij = vol_i + r_fabs(b1.w);
-    if (STAGE == 1) {
-      const R P_ij = sum * vol_ij;
-      for (int d = 0; d < D; d++) accum(d, (dr[d] * aw) * -P_ij);
-    }
-    cij = aw * vol_ij;
+    if (STAGE == 2 || !(ti == SURFACE_P || D == 3)) return false;  // a SEGMENT particle sums in 3D only (:740-759)
+    wt = W(ti == SEGMENT_P ? 1 : D - 1, dist);
     return true;
   };
-  auto visc = [&](int j, R cij) {
+  // viscous term of neighbour j
+  auto visc = [&](int j, R cij, R* t) {
     const T4 anj = w.a1[j];
     const bool char_j = signbit(anj.w);  // j is not REAL
     R vj[3];
     if (ti == REAL_P && char_j) {
       vj[0] = vi[0] * (R)-1.0; vj[1] = vi[1] * (R)-1.0; vj[2] = vi[2] * (R)-1.0;
     } else {
-      vj[0] = anj.x * hdt1; vj[1] = anj.y * hdt1; vj[2] = anj.z * hdt1;
+      vj[0] = rmul(anj.x, hdt1); vj[1] = rmul(anj.y, hdt1); vj[2] = rmul(anj.z, hdt1);
     }
     const R eta_j = r_fabs(anj.w);
     const R eta_ij = r_div((R)2. * eta_j * eta_i, eta_i + eta_j + (R)1.e-15);
     const R temp0 = cij * eta_ij;
-    for (int d = 0; d < D; d++) accum(d, (vi[d] - vj[d]) * temp0);
+    for (int d = 0; d < D; d++) t[d] = rmul(vi[d] - vj[d], temp0);
   };
-  if (ti != SINGULARITY_P) {  // a SINGULARITY particle has no force
-    if constexpr (!SPILL) {
-      const int cnt = w.cnt[i];
+  // entry j: its force terms t (0 when it has none), its kernel-sum term; cij is
+  // the stored coefficient (read in stage 2, written in stage 1).  Returns
+  // whether it counts towards the kernel sum.
+  auto entry = [&](int j, R& cij, R* t, R& wt) -> bool {
+    bool counts = false;
+    t[0] = t[1] = t[2] = 0;
+    wt = 0;
+    if constexpr (GEO) {
+      R dr[3], cg;
+      counts = pair(j, dr, cg, wt);
+      cij = cg;
+      if (STAGE == 1)
+        for (int d = 0; d < D; d++) t[d] = rmul(dr[d], cij);
+    }
+    if (STAGE == 2 && cij != (R)0) visc(j, cij, t);
+    return counts;
+  };
+  const int cnt = w.cnt[i];
+  if (ti != SINGULARITY_P) {  // a SINGULARITY particle has no kernel sum and no force
+    if constexpr (G == 1) {
+      int q = 0;  // entries taken
+      auto take = [&](int j, R& cij) {
+        R t[3], wt;
+        if (entry(j, cij, t, wt)) {
+          sum = radd(sum, wt);
+          ncount++;
+        }
+        if (STAGE > 0)
+          for (int d = 0; d < D; d++) accum(d, t[d]);
+      };
+      static_assert(!SPILL, "a spilled particle is taken by a group");
       const long long base = nb_slot(i, 0, w.cap);
       const int* row = w.nbl + base;
       R* crow = w.pc + base;
-      if (MRSPH_FORCE_VEC == 4) {
-        // four entries per access: q0 is a multiple of 4, so row + o and
-        // crow + o are 16-byte aligned; entries past cnt inside the group
-        // lie within the particle's cap and are ignored (stage 1 stores 0)
-        for (int q0 = 0; q0 < cnt; q0 += 4) {
-          const int o = ((q0 >> 3) << 8) + (q0 & 7);
-          const int4 j4 = LD::ld(reinterpret_cast<const int4*>(row + o));
-          const int jj[4] = {j4.x, j4.y, j4.z, j4.w};
-          R cc[4];
-          if (STAGE == 1) {
+      // four entries per access: q is a multiple of 4, so row + o and
+      // crow + o are 16-byte aligned; entries past cnt inside the group
+      // lie within the particle's cap and are ignored (stage 1 stores 0)
+      for (; q < cnt; q += 4) {
+        const int o = ((q >> 3) << 8) + (q & 7);
+        const int4 j4 = LD::ld(reinterpret_cast<const int4*>(row + o));
+        const int jj[4] = {j4.x, j4.y, j4.z, j4.w};
+        R cc[4] = {0, 0, 0, 0};
+        if (STAGE == 2) load4<LD>(crow + o, cc);
 #pragma unroll
-            for (int k = 0; k < 4; k++) {
-              cc[k] = 0;
-              if (q0 + k < cnt) {
-                const int j = nb_index(jj[k]);
-                T4 b0, b1;
-                LD::rec(b.rec, j, b0, b1);
-                R vec[3], dr[3];
-                Q::rel(c, a0, a1r, b0, b1, vec);
-                coef(j, b0, b1, vec, dr, cc[k], nb_mark(jj[k]));
-              }
-            }
-            store4(crow + o, cc);
-          } else {
-            load4<LD>(crow + o, cc);
-#pragma unroll
-            for (int k = 0; k < 4; k++)
-              if (q0 + k < cnt && cc[k] != (R)0) visc(nb_index(jj[k]), cc[k]);
-          }
-          flush();
-        }
-      } else {
-        for (int q = 0; q < cnt; q++) {
-          const int o = ((q >> 3) << 8) + (q & 7);
-          if (STAGE == 1) {
-            const int e = LD::ld(&row[o]);
-            const int j = nb_index(e);
-            T4 b0, b1;
-            LD::rec(b.rec, j, b0, b1);
-            R vec[3], dr[3], cij = 0;
-            Q::rel(c, a0, a1r, b0, b1, vec);
-            coef(j, b0, b1, vec, dr, cij, nb_mark(e));
-            crow[o] = cij;
-          } else {
-            const R cij = LD::ld(&crow[o]);
-            if (cij != (R)0) visc(nb_index(LD::ld(&row[o])), cij);
-          }
-          if ((q & 3) == 3 || q == cnt - 1) flush();
-        }
+        for (int k = 0; k < 4; k++)
+          if (q + k < cnt) take(jj[k], cc[k]);
+        if (STAGE == 1) store4(crow + o, cc);
+        for (int d = 0; d < D; d++) flush(d);
       }
     } else {
-      const R cut = pick<R>(c.prm.cutoff, c.prm.cutoff_f);
-      const R R2i = (h * cut) * (h * cut);
-      const SOrigin<D, R> so(c, b.posh[i], b.key ? b.key[i] : 0);
-      int q = 0;  // accepted neighbours so far (the list entries this scan replaces)
-      scan_candidates<D, R, LD>(c, w.cstart, w.lhmax, so, h, [&](int j) {
-        T4 b0, b1;
-        LD::rec(b.rec, j, b0, b1);
-        R vec[3], dr[3], cij = 0;
-        Q::rel(c, a0, a1r, b0, b1, vec);
-        if constexpr (F32) {
-          const float d2 = d2_of(vec, D);
-          const float rj = b0.w * cut;
-          const float Rm = fmaxf(R2i, rj * rj);
-          if (d2 > Rm * kD2Accept) return;
-          if (d2 >= Rm * kD2Sure && !exact_neighbor<D>(c, a0, a1r, b0, b1)) return;
-        } else {
-          R dist;
-          if (!nb_test(d2_of(vec, D), h, b0.w, c.prm.cutoff, dist)) return;
+      // entries q0 .. q0 + kG - 1, this lane's being j (on = false past the end)
+      auto chunk = [&](int q0, int j, bool on, R* crow) {
+        R t[3] = {0, 0, 0}, wt = 0, cij = 0;
+        bool counts = false;
+        if (on) {
+          if (STAGE == 2 && !SPILL) cij = LD::ld(crow);
+          counts = entry(j, cij, t, wt);
+          if (STAGE == 1 && !SPILL) *crow = cij;
         }
-        if (coef(j, b0, b1, vec, dr, cij, 0u) && STAGE == 2 && cij != (R)0) visc(j, cij);
-        if ((q & 3) == 3) flush();
-        q++;
-      });
-      if (q & 3) flush();
+        if (STAGE > 0)
+          for (int d = 0; d < D; d++) gt->term[d][g.gl] = t[d];
+        if (STAGE < 2) {
+          gt->term[3][g.gl] = wt;
+          ncount += __popc(g.ballot(counts));
+        }
+        __syncwarp(g.mask);
+        if (STAGE > 0 && g.gl < D) {
+          const R* v = gt->term[g.gl];
+          for (int k = 0; k < 4; k++) accum(0, v[k]);
+          flush(0);
+          if (q0 + 4 < cnt) {
+            for (int k = 4; k < kG; k++) accum(0, v[k]);
+            flush(0);
+          }
+        }
+        if (STAGE < 2 && g.gl == 3)
+          for (int k = 0; k < kG; k++) sum = radd(sum, gt->term[3][k]);
+        __syncwarp(g.mask);
+      };
+      if constexpr (!SPILL) {
+        const long long base = nb_slot(i, g.gl, w.cap);  // entry q0 + gl at base + 32 q0
+        for (int q0 = 0; q0 < cnt; q0 += kG) {
+          const bool on = q0 + g.gl < cnt;
+          chunk(q0, on ? LD::ld(w.nbl + base + 32 * q0) : 0, on, w.pc + base + 32 * q0);
+        }
+      } else {
+        const PairTest<D, R> pt(c, b.rec, i);
+        const SOrigin<D, R> so(c, b.posh[i], b.key ? b.key[i] : 0);
+        int held = 0, q0 = 0;
+        group_scan<D, R, LD>(c, w, g, gt->rows, i, so, [&](int j, bool in) {
+          const bool ok = in && pt.template near<LD>(c, b.rec, j);
+          const unsigned m = g.ballot(ok);
+          if (ok) gt->vlist[held + __popc(m & g.below)] = j;
+          held += __popc(m);
+          __syncwarp(g.mask);
+          if (held >= kG) {
+            chunk(q0, gt->vlist[g.gl], true, nullptr);
+            q0 += kG;
+            held -= kG;
+            const int rest = g.gl < held ? gt->vlist[kG + g.gl] : 0;
+            __syncwarp(g.mask);
+            if (g.gl < held) gt->vlist[g.gl] = rest;
+            __syncwarp(g.mask);
+          }
+        });
+        if (held > 0) chunk(q0, g.gl < held ? gt->vlist[g.gl] : 0, g.gl < held, nullptr);
+      }
     }
+  }
+  if (G > 1) {
+    if (STAGE > 0) {
+      if constexpr (F32) F[0] = F[0] - Fc[0];
+      F[1] = __shfl_sync(g.mask, F[0], 1, kG);
+      F[2] = __shfl_sync(g.mask, F[0], 2, kG);
+    }
+    if (STAGE < 2) sum = __shfl_sync(g.mask, sum, 3, kG);
+    if (g.gl != 0) return;
+    if (D == 2) F[2] = 0;
+  } else if constexpr (F32) {
+    for (int d = 0; d < D; d++) F[d] = F[d] - Fc[d];
+  }
+  if (STAGE < 2) {
+    if (ti == REAL_P) {
+      if (WEN32) sum = rmul(sum, (R)((float)kern_norm(K_WEN, D) * (D == 3 ? inv_h * inv_h * inv_h : inv_h * inv_h)));
+      ncount = cnt;
+    }
+    if (ncount > 1) sum = (R)1. / radd(sum, (R)1.e-15);
+    w.sum[i] = sum;
+    if (STAGE == 0) return;
   }
   R a[3] = {0, 0, 0};
   if (ti != SINGULARITY_P) {
-    if constexpr (F32)
-      for (int d = 0; d < D; d++) F[d] = F[d] - Fc[d];
-    for (int d = 0; d < D; d++) a[d] = F[d];
+    for (int d = 0; d < D; d++) a[d] = STAGE == 1 ? rmul(F[d], -sum) : F[d];
     if (STAGE == 2)
-      for (int d = 0; d < D; d++) a[d] = a[d] + vi[d] * pick<R>(c.prm.damp_coeff, c.prm.damp_coeff_f);
+      for (int d = 0; d < D; d++) a[d] = madd(vi[d], pick<R>(c.prm.damp_coeff, c.prm.damp_coeff_f), a[d]);
     if (ti == SURFACE_P || ti == SEGMENT_P) {  // Map_surface_particle_force, :1122-1126
       R nf = dot3<D, R>(a, ni);
-      for (int d = 0; d < D; d++) a[d] = a[d] - ni[d] * nf;
+      for (int d = 0; d < D; d++) a[d] = madd(-ni[d], nf, a[d]);
     }
   }
   R U = r_sqrt(dot3<D, R>(vi, vi));
@@ -1716,53 +1948,75 @@ __device__ inline void force_particle(const KCtx& c, const Buf<R>& b, const Work
   ts = AMIN1(ts, h / (R)40. / (U + (R)1.e-15));
   if (STAGE == 2) {
     R nu_new = pick<R>(c.prm.nu_coeff, c.prm.nu_coeff_f) * h * U;
-    ts = AMIN1(ts, (R)0.125 * h * h / (nu_new + (R)1.e-15));
+    ts = AMIN1(ts, (R)0.125 * h * h / radd(nu_new, (R)1.e-15));
     b.nu_next[i] = nu_new;
     b.v1[i] = mk4<R>(vi[0], vi[1], vi[2], U);
     b.a2[i] = mk4<R>(a[0], a[1], a[2], 0);
   } else {
-    const R eta = nu * rho;
+    const R eta = b.nu[i] * rho;
     w.a1[i] = mk4<R>(a[0], a[1], a[2], ti != REAL_P ? -eta : eta);
   }
   my_dt = fmin(my_dt, (double)ts);
   my_v = fmax(my_v, (double)U);
 }
 
-// KK: the kernel kind fixed at compile time (FP32 Wendland C2), or -1.
-// Particles whose list spilled are left to k_force_spill.
-template <int D, class R, int STAGE, int KK, class LD = LdNC>
-__device__ inline void force_block(const KCtx& c, const Buf<R>& b, const Work<R>& w, long long blk) {
-  long long i = blk * blockDim.x + threadIdx.x;
-  double my_dt = 1.e300, my_v = 0.0;
-  if (i < c.n && w.cnt[i] <= w.cap) force_particle<D, R, STAGE, KK, false, LD>(c, b, w, i, my_dt, my_v);
+template <int STAGE>
+__device__ inline void force_reduce(const KCtx& c, double my_dt, double my_v) {
   if (STAGE == 1) block_minmax_to_global(my_dt, my_v, &c.sc->dt1, &c.sc->vmax1);
-  else block_minmax_to_global(my_dt, my_v, &c.sc->dt2, &c.sc->vmax2);
+  if (STAGE == 2) block_minmax_to_global(my_dt, my_v, &c.sc->dt2, &c.sc->vmax2);
+}
+
+// KK: the kernel kind fixed at compile time (FP32 Wendland C2), or -1.
+// The blockDim.x / G particles from first; those whose list spilled are left to
+// k_force_spill.  gt: a GroupTile per group (G = kG).
+template <int D, class R, int STAGE, int KK, int G, class LD = LdNC>
+__device__ inline void force_block(const KCtx& c, const Buf<R>& b, const Work<R>& w, GroupTile<R>* gt,
+                                   long long first) {
+  const GroupLanes g;
+  double my_dt = 1.e300, my_v = 0.0;
+  const long long i = first + threadIdx.x / G;
+  if (i < c.n && w.cnt[i] <= w.cap)
+    force_particle<D, R, STAGE, KK, G, false, LD>(c, b, w, g, G > 1 ? gt + threadIdx.x / G : nullptr, i, my_dt, my_v);
+  __syncwarp();
+  force_reduce<STAGE>(c, my_dt, my_v);
 }
 
 template <int D, class R, int STAGE, int KK>
 __global__ void __launch_bounds__(256, (std::is_same<R, float>::value ? (STAGE == 1 ? MRSPH_FORCE_MIN_BLOCKS : MRSPH_FORCE2_MIN_BLOCKS) : 1)) k_force(KCtx c, Buf<R> b, Work<R> w) {
-  force_block<D, R, STAGE, KK>(c, b, w, blockIdx.x);
+  if (STAGE < 2 && blockIdx.x == 0 && threadIdx.x == 0) accum_pairs_body(c.sc);
+  force_block<D, R, STAGE, KK, 1>(c, b, w, nullptr, (long long)blockIdx.x * 256);
+}
+
+constexpr int kGroupThreads = 128;
+template <int D, class R, int STAGE, int KK>
+__global__ void __launch_bounds__(kGroupThreads, std::is_same<R, float>::value ? 8 : 1) k_force_group(KCtx c, Buf<R> b, Work<R> w) {
+  __shared__ GroupTile<R> gt[kGroupThreads / kG];
+  if (STAGE < 2 && blockIdx.x == 0 && threadIdx.x == 0) accum_pairs_body(c.sc);
+  force_block<D, R, STAGE, KK, kG>(c, b, w, gt, (long long)blockIdx.x * (kGroupThreads / kG));
 }
 
 // The force stage of the particles whose list spilled (queued by the density
-// pass; grid-stride), re-scanning their cells.
+// pass; grid-stride over groups), re-scanning their cells.
 template <int D, class R, int STAGE, int KK, class LD = LdNC>
-__device__ inline void force_spill_items(const KCtx& c, const Buf<R>& b, const Work<R>& w, long long blk,
-                                         long long nblk) {
+__device__ inline void force_spill_items(const KCtx& c, const Buf<R>& b, const Work<R>& w, GroupTile<R>* gt,
+                                         long long blk, long long nblk) {
+  const GroupLanes g;
   double my_dt = 1.e300, my_v = 0.0;
-  const unsigned nq = c.sc->nspill;
-  if (blk * blockDim.x >= (long long)nq) return;  // block-uniform: nothing queued for this block
-  for (long long t = blk * blockDim.x + threadIdx.x; t < nq; t += nblk * blockDim.x) {
+  const long long nq = c.sc->nspill, per = blockDim.x / kG;
+  if (blk * per >= nq) return;  // block-uniform: nothing queued for this block
+  for (long long t = blk * per + threadIdx.x / kG; t < nq; t += nblk * per) {
     const int i = w.spillq[t];
-    if (w.cnt[i] > w.cap) force_particle<D, R, STAGE, KK, true, LD>(c, b, w, i, my_dt, my_v);
+    if (w.cnt[i] > w.cap)
+      force_particle<D, R, STAGE, KK, kG, true, LD>(c, b, w, g, gt + threadIdx.x / kG, i, my_dt, my_v);
   }
-  if (STAGE == 1) block_minmax_to_global(my_dt, my_v, &c.sc->dt1, &c.sc->vmax1);
-  else block_minmax_to_global(my_dt, my_v, &c.sc->dt2, &c.sc->vmax2);
+  __syncwarp();
+  force_reduce<STAGE>(c, my_dt, my_v);
 }
 
 template <int D, class R, int STAGE, int KK>
-__global__ void __launch_bounds__(256) k_force_spill(KCtx c, Buf<R> b, Work<R> w) {
-  force_spill_items<D, R, STAGE, KK>(c, b, w, blockIdx.x, gridDim.x);
+__global__ void __launch_bounds__(kGroupThreads) k_force_spill(KCtx c, Buf<R> b, Work<R> w) {
+  __shared__ GroupTile<R> gt[kGroupThreads / kG];
+  force_spill_items<D, R, STAGE, KK>(c, b, w, gt, blockIdx.x, gridDim.x);
 }
 
 // ----------------------------------------------------------------- taps
@@ -1819,11 +2073,11 @@ __global__ void k_export_tri(KCtx c, Buf<R> b, Work<R> w, double* __restrict__ x
   const int* src = w.nbl + nb_slot(s, 0, w.cap);
   int* dst = rows + k * rowcap;
   if (!sort_rows) {
-    for (int q = 0; q < m; q++) dst[q] = b.id[nb_index(src[((q >> 3) << 8) + (q & 7)])];
+    for (int q = 0; q < m; q++) dst[q] = b.id[src[((q >> 3) << 8) + (q & 7)]];
     return;
   }
   for (int q = 0; q < m; q++) {  // insertion sort by id
-    int v = b.id[nb_index(src[((q >> 3) << 8) + (q & 7)])];
+    int v = b.id[src[((q >> 3) << 8) + (q & 7)]];
     int p = q;
     while (p > 0 && dst[p - 1] > v) { dst[p] = dst[p - 1]; p--; }
     dst[p] = v;
@@ -1931,6 +2185,8 @@ class Engine : public EngineBase {
     kc_.ls.max_curv_f = (float)kc_.ls.max_curv;
     kc_.ls.min_curv_f = (float)kc_.ls.min_curv;
     kc_.geo.max_scale_f = (float)kc_.geo.max_scale;
+    kc_.geo.ext_f = 0.f;
+    for (int d = 0; d < D; d++) kc_.geo.ext_f = std::max(kc_.geo.ext_f, (float)(cfg.prm.box_r[d] - cfg.prm.box_l[d]));
     if (std::is_same<R, float>::value) init_rc_ = anchor_tables();
     int dev = 0;
     if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms_, cudaDevAttrMultiProcessorCount, dev);
@@ -1994,13 +2250,22 @@ class Engine : public EngineBase {
   }
 
   // Graph replay.  The neighbour-list capacity follows the largest list
-  // seen: every 32 steps (and on the first call) the device max count is read
-  // and the list grown, within a memory budget; particles whose list does not
-  // fit are handled by re-scanning their cells in the force kernels.
+  // seen: every 32 steps the device max count is read and the list grown,
+  // within a memory budget; particles whose list does not fit are handled by
+  // re-scanning their cells in the force kernels.  A state's first step is
+  // launched kernel by kernel and settles the capacity before the forces: the
+  // re-scan of every particle of a freshly seeded body took longer than the rest
+  // of the step, and the step graphs were built twice.
   int step(int nsteps) override {
     if (!n_) { err = "no particles"; return MRSPH_ERR_STATE; }
     if (nsteps <= 0) return 0;
     for (int k = 0; k < nsteps; k++) {
+      if (countdown_ <= 0) {  // the first step of a state
+        int rc = launch_step(MRSPH_PHASE_FORCE2, nullptr, true);
+        if (rc) return rc;
+        countdown_ = 32;
+        continue;
+      }
       int rc = build_graphs();
       if (rc) return rc;
       MR_CK(cudaGraphLaunch(graph_[cur_], st_));
@@ -2205,7 +2470,7 @@ class Engine : public EngineBase {
     for (long long k = 0; k < n_; k++) off[k + 1] = off[k] + byid_cnt[k];
     for (long long s = 0; s < n_; s++) {
       long long base = off[ids[s]];
-      for (int q = 0; q < cnt[s]; q++) nb[base + q] = ids[nb_index(nbl[nb_slot(s, q, w_.cap)])];
+      for (int q = 0; q < cnt[s]; q++) nb[base + q] = ids[nbl[nb_slot(s, q, w_.cap)]];
       std::sort(nb + base, nb + base + cnt[s]);
     }
     return 0;
@@ -2286,6 +2551,7 @@ class Engine : public EngineBase {
     std::memcpy((void*)&s.buf[0], (const void*)&buf_[0], sizeof(Buf<float>));
     std::memcpy((void*)&s.buf[1], (const void*)&buf_[1], sizeof(Buf<float>));
     std::memcpy((void*)&s.w, (const void*)&w_, sizeof(Work<float>));
+    s.w.bcount = s.w.bstart = s.w.order = nullptr;  // the batch's phases do not make the work order
     s.ncells = ncells_;
     s.dim = D;
     s.cur = cur_;
@@ -2302,12 +2568,12 @@ class Engine : public EngineBase {
   static unsigned long long dbits_host(double x) { unsigned long long u; std::memcpy(&u, &x, 8); return u; }
   static double bitsd_host(unsigned long long u) { double x; std::memcpy(&x, &u, 8); return x; }
   static int grid(long long n) { return (int)((n + 255) / 256); }
-  // grid of the queue kernels (density fix-up, spilled force stages): the
-  // queues' lengths are known on the device only; two blocks per SM at most
+  // grid of the spilled force stages: the queue's length is known on the
+  // device only; two blocks per SM at most
   int qgrid() const { return std::max(1, std::min(grid(n_), 2 * sms_)); }
 
   int pre_run() {
-    k_begin_step<<<1, 1, 0, st_>>>(kc_.sc, 0);
+    begin_step(0);
     int rc = run_map_and_bin(MAP_PRE);
     if (rc) return rc;
     // Pre_run (sph_mesh_generation.cpp:1010-1050) leaves v = 0 (Reset_particle_force)
@@ -2327,30 +2593,64 @@ class Engine : public EngineBase {
   // map (mode) + counting sort + reorder; swaps cur_.
   int run_map_and_bin(int mode) {
     const long long n = n_;
-    MR_CK(cudaMemsetAsync(w_.lhmax, 0, sizeof(unsigned) * kc_.geo.nc0 * kc_.geo.ncl, st_));
     k_map<D, R><<<grid(n), 256, 0, st_>>>(kc_, buf_[cur_], w_.counts, w_.lhmax, mode, 1000000u);
     MR_CK(cudaGetLastError());
     return bin(1);
+  }
+
+  void begin_step(int inc) {
+    const long long nl = kc_.geo.nc0 * kc_.geo.ncl;
+    k_begin_step<<<grid(nl), 256, 0, st_>>>(kc_.sc, inc, w_.lhmax, nl);
   }
 
   int bin(int partial) {
     const long long n = n_;
     cell_scan(w_.counts, w_.cstart, w_.blocksums, ncells_, (int)n, st_);
     cell_scatter(buf_[cur_].cellkey, w_.counts, w_.cstart, w_.perm, n, st_);
-    cell_rank(buf_[cur_].cellkey, w_.cstart, w_.perm, buf_[cur_].id, w_.perm2, n, st_);
-    k_reorder<D, R><<<grid(n), 256, 0, st_>>>(buf_[cur_], buf_[cur_ ^ 1], kc_, w_.perm2, w_.slot_of_id, n, partial);
+    k_reorder<D, R><<<grid(n), 256, 0, st_>>>(buf_[cur_], buf_[cur_ ^ 1], kc_, w_, partial);
     MR_CK(cudaGetLastError());
     cur_ ^= 1;
     return 0;
   }
 
+  int ggrid(int threads) const { return (int)((n_ + threads / kG - 1) / (threads / kG)); }  // kG lanes per particle
+
+  void launch_lists() {
+    const long long n = n_;
+    bool grouped = true;
+    if constexpr (std::is_same<R, float>::value) {
+      if (n > kListGroupMax) {
+        const long long nb = kc_.geo.boff[kc_.geo.ncl];
+        k_brick_count<D><<<grid(nb), 256, 0, st_>>>(kc_, w_.cstart, w_.bcount);
+        cell_scan(w_.bcount, w_.bstart, w_.blocksums, nb, (int)n, st_);
+        k_brick_order<D><<<grid(nb), 256, 0, st_>>>(kc_, w_.cstart, w_.bcount, w_.bstart, w_.order);
+        k_density<D><<<(int)((n + kDensityThreads - 1) / kDensityThreads), kDensityThreads, 0, st_>>>(kc_, buf_[cur_], w_);
+        grouped = false;
+      }
+    }
+    if (grouped) k_density_group<D, R><<<ggrid(kDensityThreads), kDensityThreads, 0, st_>>>(kc_, buf_[cur_], w_);
+  }
+
+  template <int STAGE, int KK>
+  void launch_force_kind() {
+    if (n_ <= kGroupMax) k_force_group<D, R, STAGE, KK><<<ggrid(kGroupThreads), kGroupThreads, 0, st_>>>(kc_, buf_[cur_], w_);
+    else k_force<D, R, STAGE, KK><<<grid(n_), 256, 0, st_>>>(kc_, buf_[cur_], w_);
+    k_force_spill<D, R, STAGE, KK><<<qgrid(), kGroupThreads, 0, st_>>>(kc_, buf_[cur_], w_);
+  }
+  template <int STAGE>
+  void launch_force() {
+    if (kc_.prm.kernel == K_WEN) launch_force_kind<STAGE, (sizeof(R) == 4 ? K_WEN : -1)>();
+    else launch_force_kind<STAGE, -1>();
+  }
+
   // ev (optional, 8 events) brackets the timer phases MRSPH_TIMER_*.
-  int launch_step(int phase, cudaEvent_t* ev = nullptr) {
+  // settle: the list capacity is made to fit between the lists and the forces
+  // (synchronises).
+  int launch_step(int phase, cudaEvent_t* ev = nullptr, bool settle = false) {
     const long long n = n_;
     auto mark = [&](int k) { if (ev) cudaEventRecord(ev[k], st_); };
     mark(0);
-    k_begin_step<<<1, 1, 0, st_>>>(kc_.sc, 1);
-    MR_CK(cudaMemsetAsync(w_.lhmax, 0, sizeof(unsigned) * kc_.geo.nc0 * kc_.geo.ncl, st_));
+    begin_step(1);
     k_map<D, R><<<grid(n), 256, 0, st_>>>(kc_, buf_[cur_], w_.counts, w_.lhmax, MAP_STEP, 1000000u);
     MR_CK(cudaGetLastError());
     mark(1);
@@ -2361,44 +2661,33 @@ class Engine : public EngineBase {
     cell_scan(w_.counts, w_.cstart, w_.blocksums, ncells_, (int)n, st_);
     mark(2);
     cell_scatter(buf_[cur_].cellkey, w_.counts, w_.cstart, w_.perm, n, st_);
-    cell_rank(buf_[cur_].cellkey, w_.cstart, w_.perm, buf_[cur_].id, w_.perm2, n, st_);
     mark(3);
-    k_reorder<D, R><<<grid(n), 256, 0, st_>>>(buf_[cur_], buf_[cur_ ^ 1], kc_, w_.perm2, w_.slot_of_id, n,
-                                              phase < MRSPH_PHASE_FORCE2 ? 1 : 0);
+    k_reorder<D, R><<<grid(n), 256, 0, st_>>>(buf_[cur_], buf_[cur_ ^ 1], kc_, w_, phase < MRSPH_PHASE_FORCE2 ? 1 : 0);
     MR_CK(cudaGetLastError());
     cur_ ^= 1;
     mark(4);
     if (phase < MRSPH_PHASE_DENSITY) return 0;
-    const bool wen32 = sizeof(R) == 4 && kc_.prm.kernel == K_WEN;
-    if (wen32)
-      k_density<D, R, (sizeof(R) == 4 ? K_WEN : -1)><<<grid(n), 256, 0, st_>>>(kc_, buf_[cur_], w_);
-    else
-      k_density<D, R, -1><<<grid(n), 256, 0, st_>>>(kc_, buf_[cur_], w_);
-    if constexpr (std::is_same<R, float>::value) {
-      // one warp per queued particle: as many warps as particles / 32
-      if (wen32) k_density_fix<D, K_WEN><<<grid(n), 256, 0, st_>>>(kc_, buf_[cur_], w_);
-      else k_density_fix<D, -1><<<grid(n), 256, 0, st_>>>(kc_, buf_[cur_], w_);
+    launch_lists();
+    if (settle) {
+      const int cap = w_.cap;
+      int rc = maybe_grow_cap();
+      if (rc) return rc;
+      if (w_.cap != cap) {  // the same lists again, now whole
+        MR_CK(cudaMemsetAsync(&kc_.sc->pairs, 0, sizeof(kc_.sc->pairs), st_));
+        MR_CK(cudaMemsetAsync(&kc_.sc->nspill, 0, sizeof(kc_.sc->nspill), st_));
+        launch_lists();
+      }
     }
-    k_accum_pairs<<<1, 1, 0, st_>>>(kc_.sc);
     have_work_ = true;
     mark(5);
-    if (phase < MRSPH_PHASE_FORCE1) return 0;
-    if (wen32) {
-      k_force<D, R, 1, (sizeof(R) == 4 ? K_WEN : -1)><<<grid(n), 256, 0, st_>>>(kc_, buf_[cur_], w_);
-      k_force_spill<D, R, 1, (sizeof(R) == 4 ? K_WEN : -1)><<<qgrid(), 256, 0, st_>>>(kc_, buf_[cur_], w_);
-    } else {
-      k_force<D, R, 1, -1><<<grid(n), 256, 0, st_>>>(kc_, buf_[cur_], w_);
-      k_force_spill<D, R, 1, -1><<<qgrid(), 256, 0, st_>>>(kc_, buf_[cur_], w_);
+    if (phase < MRSPH_PHASE_FORCE1) {
+      launch_force<0>();
+      return 0;
     }
+    launch_force<1>();
     mark(6);
     if (phase < MRSPH_PHASE_FORCE2) return 0;
-    if (wen32) {
-      k_force<D, R, 2, (sizeof(R) == 4 ? K_WEN : -1)><<<grid(n), 256, 0, st_>>>(kc_, buf_[cur_], w_);
-      k_force_spill<D, R, 2, (sizeof(R) == 4 ? K_WEN : -1)><<<qgrid(), 256, 0, st_>>>(kc_, buf_[cur_], w_);
-    } else {
-      k_force<D, R, 2, -1><<<grid(n), 256, 0, st_>>>(kc_, buf_[cur_], w_);
-      k_force_spill<D, R, 2, -1><<<qgrid(), 256, 0, st_>>>(kc_, buf_[cur_], w_);
-    }
+    launch_force<2>();
     mark(7);
     MR_CK(cudaGetLastError());
     return 0;
@@ -2531,15 +2820,21 @@ class Engine : public EngineBase {
       rc |= A((void**)&w_.pc, sizeof(R) * (size_t)cap * ((n + 31) / 32 * 32));
       rc |= A((void**)&w_.counts, sizeof(int) * ncells_);
       rc |= A((void**)&w_.lhmax, sizeof(unsigned) * kc_.geo.nc0 * kc_.geo.ncl);
+      rc |= A((void**)&w_.rlev, sizeof(float) * kc_.geo.ncl * n);
       rc |= A((void**)&w_.cstart, sizeof(int) * (ncells_ + 1));
       rc |= A((void**)&w_.perm, sizeof(int) * n);
-      rc |= A((void**)&w_.perm2, sizeof(int) * n);
       rc |= A((void**)&w_.blocksums, sizeof(int) * scan_blocksums_size(ncells_));
       rc |= A((void**)&w_.slot_of_id, sizeof(int) * n);
-      rc |= A((void**)&w_.fixq, sizeof(int) * n);
       rc |= A((void**)&w_.spillq, sizeof(int) * n);
       rc |= A((void**)&stage_, sizeof(double) * 3 * n);
       rc |= A((void**)&kc_.sc, sizeof(DevScalars));
+    }
+    w_.bcount = w_.bstart = w_.order = nullptr;
+    if (!rc && std::is_same<R, float>::value && n > kListGroupMax) {
+      const long long nb = kc_.geo.boff[kc_.geo.ncl];
+      rc |= A((void**)&w_.bcount, sizeof(int) * nb);
+      rc |= A((void**)&w_.bstart, sizeof(int) * (nb + 1));
+      rc |= A((void**)&w_.order, sizeof(int) * n);
     }
     if (rc) { release(); return rc; }
     MR_CK(cudaMemsetAsync(w_.counts, 0, sizeof(int) * ncells_, st_));

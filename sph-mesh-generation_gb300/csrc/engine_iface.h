@@ -89,8 +89,6 @@ cudaError_t ls_volume_mass(const LsSet& ls, int level, int D, double* cvol, doub
 // sort / scan primitives (mrsph_sort.cu)
 void cell_scan(int* counts, int* cstart, int* blocksums, long long ncells, int ntotal, cudaStream_t s);
 void cell_scatter(const int* cellkey, int* cursor, const int* cstart, int* perm, long long n, cudaStream_t s);
-void cell_rank(const int* cellkey, const int* cstart, const int* perm, const int* id, int* perm2, long long n,
-               cudaStream_t s);
 long long scan_blocksums_size(long long ncells);
 
 }  // namespace mrsph

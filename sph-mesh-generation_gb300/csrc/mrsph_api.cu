@@ -71,11 +71,11 @@ static int plan_levels(mrsph_handle* h) {
     ini[d] = (d < D) ? (int)(domain[d] / max_scale) : 1;
     g.box_l[d] = (d < D) ? p.box_l[d] : 0.0;
   }
-  long long off = 0, hoff = 0;
+  long long off = 0, hoff = 0, boff = 0;
   for (int l = 0; l < num_level; l++) {
     double multi = powern_d(2.0, l);
     double sc = 1.e300;
-    long long nc = 1, hc = 1;
+    long long nc = 1, hc = 1, bc = 1;
     for (int d = 0; d < 3; d++) {
       g.n[l][d] = (d < D) ? (int)(ini[d] * multi) : 1;
       g.dcell[l][d] = (d < D) ? domain[d] / g.n[l][d] : 1.0;
@@ -89,6 +89,8 @@ static int plan_levels(mrsph_handle* h) {
       g.ihs_f[l][d] = (float)g.ihs[l][d];
       g.hs_f[l][d] = (float)g.hs[l][d];
       hc *= g.hn[l][d];
+      g.bn[l][d] = (g.hn[l][d] + 3) / 4;
+      bc *= g.bn[l][d];
     }
     // the engine keys levels by exponent: scale = max_scale * 2^-l (sph.cpp:247-276)
     if (std::fabs(sc - std::ldexp(max_scale, -l)) > 1.e-10)
@@ -97,9 +99,12 @@ static int plan_levels(mrsph_handle* h) {
     off += nc;
     g.hoff[l] = hoff;
     hoff += hc;
+    g.boff[l] = boff;
+    boff += bc;
   }
   g.off[num_level] = off;
   g.hoff[num_level] = hoff;
+  g.boff[num_level] = boff;
   g.nc0 = (long long)g.n[0][0] * g.n[0][1] * g.n[0][2];
   // cell keys are 32-bit: the half-cell table (counts + starts, 8 bytes per
   // entry; 1.06 G entries for four levels down to 480^3 cells) must index in int

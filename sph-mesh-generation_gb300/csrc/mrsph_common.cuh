@@ -63,6 +63,7 @@ struct CellGeo {
   double box_l[3];
   double max_scale, min_scale;
   float max_scale_f;
+  float ext_f;  // largest box length
   int n[MAX_CL][3];
   double dcell[MAX_CL][3];
   long long off[MAX_CL + 1];
@@ -78,6 +79,9 @@ struct CellGeo {
   int hn[MAX_CL][3];
   double hs[MAX_CL][3];  // half-cell size = dcell / 2
   long long hoff[MAX_CL + 1];
+  // bricks of 4 x 4 (x 4) half cells, row-major per level (the work order of large handles)
+  int bn[MAX_CL][3];
+  long long boff[MAX_CL + 1];
 };
 
 struct Params {
@@ -99,7 +103,6 @@ struct DevScalars {
   unsigned int remap, nsurf, flags, spill;
   unsigned int step;
   unsigned int maxcnt;  // largest neighbour count of the last density phase
-  unsigned int nfix;    // FP32-split: particles queued for the exact re-decision of the density phase
   unsigned int nspill;  // particles whose neighbour list spilled (re-scanned by the force fix-up launches)
   unsigned long long hmax[MAX_CL];  // FP64 bits of the largest h per level (this step)
   unsigned int lcount[MAX_CL];      // particles per level (this step)
@@ -157,50 +160,67 @@ __device__ inline double bitsd(unsigned long long b) { return __longlong_as_doub
 // ---------------------------------------------------------------- SPH kernels
 // particle.cpp:31-807 restated.  D = kernel dimension.  dW returns
 // dW/dr / dist (Derivative_kernel_function convention).
+// The normalisation C of W(., h): constant over a particle's neighbours.
 template <class R>
-__device__ inline R kernel_W(int kind, int D, R dist, R h) {
+__device__ inline R kernel_C(int kind, int D, R h) {
   const R PI = (R)PI_REF;
-  R s = dist / h, C = 0, val = 0;
   if (kind == K_WEN) {
     if (D == 1) return 0;
-    if (D == 2) C = (R)1.0 / PI / powern(h, 2) * (R)7. / (R)4.;
-    else C = (R)1.0 / PI / powern(h, 3) * (R)21. / (R)16.;
-    if (s < 2) val = C * powern(((R)1. - (R)0.5 * s), 4) * ((R)1. + (R)2. * s);
-    return val;
+    if (D == 2) return (R)1.0 / PI / powern(h, 2) * (R)7. / (R)4.;
+    return (R)1.0 / PI / powern(h, 3) * (R)21. / (R)16.;
   }
   if (kind == K_HYP) {
-    if (D == 1) C = (R)1.0 / (R)7.0 / powern(h, 1);
-    else if (D == 2) C = (R)1.0 / ((R)3.0 * PI) / powern(h, 2);
-    else C = (R)15.0 / ((R)62.0 * PI) / powern(h, 3);
-    if (s < 1) val = C * ((R)6.0 - (R)6.0 * s + s * s * s);
-    else if (s < 2) val = C * (2 - s) * (2 - s) * (2 - s);
-    return val;
+    if (D == 1) return (R)1.0 / (R)7.0 / powern(h, 1);
+    if (D == 2) return (R)1.0 / ((R)3.0 * PI) / powern(h, 2);
+    return (R)15.0 / ((R)62.0 * PI) / powern(h, 3);
   }
   if (kind == K_CUB) {
-    if (D == 1) C = (R)0.666666667 / powern(h, 1);
-    else if (D == 2) C = (R)0.454728408 / powern(h, 2);
-    else C = (R)0.318309886 / powern(h, 3);
-    if (s < 1) val = C * (1 - (R)1.5 * s * s + (R)0.75 * s * s * s);
-    else if (s < 2) val = C / (R)4.0 * (2 - s) * (2 - s) * (2 - s);
-    return val;
+    if (D == 1) return (R)0.666666667 / powern(h, 1);
+    if (D == 2) return (R)0.454728408 / powern(h, 2);
+    return (R)0.318309886 / powern(h, 3);
   }
   if (kind == K_GAU) {
     R fac = (R)0.5 * 2 / r_sqrt(PI);
     if (D > 1) fac *= (R)0.5 * 2 / r_sqrt(PI);
     if (D > 2) fac *= (R)0.5 * 2 / r_sqrt(PI);
-    if (D == 1) C = fac / h;
-    else C = fac / powern(h, D);
+    return D == 1 ? fac / h : fac / powern(h, D);
+  }
+  if (D == 1) return (R)1.0 / (R)120. / powern(h, 1);
+  if (D == 2) return (R)1.0 / PI * (R)7. / (R)478. / powern(h, 2);
+  return (R)1.0 / PI * (R)3. / (R)359. / powern(h, 3);
+}
+// W given C = kernel_C(kind, D, h)
+template <class R>
+__device__ inline R kernel_W_C(int kind, int D, R dist, R h, R C) {
+  R s = dist / h, val = 0;
+  if (kind == K_WEN) {
+    if (D == 1) return 0;
+    if (s < 2) val = C * powern(((R)1. - (R)0.5 * s), 4) * ((R)1. + (R)2. * s);
+    return val;
+  }
+  if (kind == K_HYP) {
+    if (s < 1) val = C * ((R)6.0 - (R)6.0 * s + s * s * s);
+    else if (s < 2) val = C * (2 - s) * (2 - s) * (2 - s);
+    return val;
+  }
+  if (kind == K_CUB) {
+    if (s < 1) val = C * (1 - (R)1.5 * s * s + (R)0.75 * s * s * s);
+    else if (s < 2) val = C / (R)4.0 * (2 - s) * (2 - s) * (2 - s);
+    return val;
+  }
+  if (kind == K_GAU) {
     if (s < 3) val = r_exp((R)-1. * s * s) * C;
     return val;
   }
   // quintic
-  if (D == 1) C = (R)1.0 / (R)120. / powern(h, 1);
-  else if (D == 2) C = (R)1.0 / PI * (R)7. / (R)478. / powern(h, 2);
-  else C = (R)1.0 / PI * (R)3. / (R)359. / powern(h, 3);
   if (s < 1) val = C * (powern(((R)3. - s), 5) - (R)6. * powern(((R)2. - s), 5) + (R)15. * powern(((R)1. - s), 5));
   else if (s < 2) val = C * (powern(((R)3. - s), 5) - (R)6. * powern(((R)2. - s), 5));
   else if (s < 3) val = C * (powern(((R)3. - s), 5));
   return val;
+}
+template <class R>
+__device__ inline R kernel_W(int kind, int D, R dist, R h) {
+  return kernel_W_C<R>(kind, D, dist, h, kernel_C<R>(kind, D, h));
 }
 
 template <class R>
@@ -270,6 +290,8 @@ template <class R> __host__ __device__ inline R pick(double d, float f);
 template <> __host__ __device__ inline double pick<double>(double d, float) { return d; }
 template <> __host__ __device__ inline float pick<float>(double, float f) { return f; }
 
+__device__ inline double pair_inv(double x) { return 1.0 / x; }
+__device__ inline float pair_inv(float x) { return __frcp_rn(x); }  // 1 / h of a kernel sum
 __device__ inline double r_rcp(double x) { return 1.0 / x; }
 __device__ inline float r_rcp(float x) { return __fdividef(1.0f, x); }
 __device__ inline double r_div(double a, double b) { return a / b; }
@@ -289,9 +311,20 @@ __host__ __device__ constexpr double kern_norm(int kind, int D) {
        : 0.0;
 }
 
+// a * b + c: one fused operation in FP32 (written out, so that every kernel that
+// evaluates a pair rounds alike, whatever the compiler contracts), the
+// reference's two roundings in FP64
+__device__ inline float madd(float a, float b, float c) { return fmaf(a, b, c); }
+__device__ inline double madd(double a, double b, double c) { return a * b + c; }
+// a sum and a product that are not contracted with what surrounds them
+__device__ inline float radd(float a, float b) { return __fadd_rn(a, b); }
+__device__ inline double radd(double a, double b) { return a + b; }
+__device__ inline float rmul(float a, float b) { return __fmul_rn(a, b); }
+__device__ inline double rmul(double a, double b) { return a * b; }
+
 // FP32 W(dist, h) given inv_h = 1/h
 __device__ inline float kernel_W_fast(int kind, int D, float dist, float inv_h) {
-  const float s = dist * inv_h;
+  const float s = __fmul_rn(dist, inv_h);  // not contracted into 2 - s
   float ih = inv_h, C;
   float hD = ih;
   if (D >= 2) hD *= ih;
@@ -301,18 +334,18 @@ __device__ inline float kernel_W_fast(int kind, int D, float dist, float inv_h) 
     C = (float)kern_norm(K_WEN, 2) * hD;
     if (D == 3) C = (float)kern_norm(K_WEN, 3) * hD;
     if (!(s < 2.f)) return 0.f;
-    const float t = 1.f - 0.5f * s, t2 = t * t;
-    return C * (t2 * t2) * (1.f + 2.f * s);
+    const float t = fmaf(-0.5f, s, 1.f), t2 = t * t;
+    return C * (t2 * t2) * fmaf(2.f, s, 1.f);
   }
   if (kind == K_HYP) {
     C = (float)(D == 1 ? kern_norm(K_HYP, 1) : D == 2 ? kern_norm(K_HYP, 2) : kern_norm(K_HYP, 3)) * hD;
-    if (s < 1.f) return C * (6.f - 6.f * s + s * s * s);
+    if (s < 1.f) return C * fmaf(s * s, s, fmaf(-6.f, s, 6.f));
     if (s < 2.f) { const float t = 2.f - s; return C * t * t * t; }
     return 0.f;
   }
   if (kind == K_CUB) {
     C = (float)(D == 1 ? kern_norm(K_CUB, 1) : D == 2 ? kern_norm(K_CUB, 2) : kern_norm(K_CUB, 3)) * hD;
-    if (s < 1.f) return C * (1.f - 1.5f * s * s + 0.75f * s * s * s);
+    if (s < 1.f) return C * fmaf(s * s, fmaf(0.75f, s, -1.5f), 1.f);
     if (s < 2.f) { const float t = 2.f - s; return C * 0.25f * t * t * t; }
     return 0.f;
   }
@@ -327,8 +360,8 @@ __device__ inline float kernel_W_fast(int kind, int D, float dist, float inv_h) 
   C = (float)(D == 1 ? kern_norm(K_QUI, 1) : D == 2 ? kern_norm(K_QUI, 2) : kern_norm(K_QUI, 3)) * hD;
   const float a = 3.f - s, b = 2.f - s, c = 1.f - s;
   const float a5 = a * a * a * a * a, b5 = b * b * b * b * b, c5 = c * c * c * c * c;
-  if (s < 1.f) return C * (a5 - 6.f * b5 + 15.f * c5);
-  if (s < 2.f) return C * (a5 - 6.f * b5);
+  if (s < 1.f) return C * fmaf(15.f, c5, fmaf(-6.f, b5, a5));
+  if (s < 2.f) return C * fmaf(-6.f, b5, a5);
   if (s < 3.f) return C * a5;
   return 0.f;
 }
@@ -340,21 +373,21 @@ __device__ inline float kernel_W_fast(int kind, int D, float dist, float inv_h) 
 // h and not average out of a near-balanced force sum.
 __device__ inline float kernel_dW_fast(int kind, int D, float dist, float h) {
   const float ih = __frcp_rn(h);
-  const float s = dist * ih;
+  const float s = __fmul_rn(dist, ih);
   float hD = ih;
   if (D >= 2) hD *= ih;
   if (D >= 3) hD *= ih;
   if (kind == K_WEN) {
     if (D == 1 || !(s < 2.f)) return 0.f;
     const float C = (float)(D == 2 ? kern_norm(K_WEN, 2) : kern_norm(K_WEN, 3)) * hD;
-    const float t = 1.f - 0.5f * s;
+    const float t = fmaf(-0.5f, s, 1.f);
     return -5.f * C * (t * t * t) * s * ih * __frcp_rn(dist + 1.e-15f);
   }
   if (kind == K_HYP) {
     const float C = (float)(D == 1 ? kern_norm(K_HYP, 1) : D == 2 ? kern_norm(K_HYP, 2) : kern_norm(K_HYP, 3)) *
                     hD * ih;
     float v = 0.f;
-    if (s < 1.f) v = C * (-6.f + 3.f * s * s);
+    if (s < 1.f) v = C * fmaf(3.f * s, s, -6.f);
     else if (s < 2.f) { const float t = 2.f - s; v = C * -3.f * t * t; }
     return v * __frcp_rn(dist + 1.e-20f);
   }
@@ -362,7 +395,7 @@ __device__ inline float kernel_dW_fast(int kind, int D, float dist, float h) {
     const float C = (float)(D == 1 ? kern_norm(K_CUB, 1) : D == 2 ? kern_norm(K_CUB, 2) : kern_norm(K_CUB, 3)) *
                     hD * ih;
     float v = 0.f;
-    if (s < 1.f) v = 3.f * C * (-s + 0.75f * s * s);
+    if (s < 1.f) v = 3.f * C * fmaf(0.75f * s, s, -s);
     else if (s < 2.f) { const float t = 2.f - s; v = -0.75f * C * t * t; }
     return v * __frcp_rn(dist + 1.e-20f);
   }
@@ -378,8 +411,8 @@ __device__ inline float kernel_dW_fast(int kind, int D, float dist, float h) {
   const float a = 3.f - s, b = 2.f - s, c = 1.f - s;
   const float a4 = a * a * a * a, b4 = b * b * b * b, c4 = c * c * c * c;
   float v;
-  if (s < 1.f) v = C * (-5.f * a4 + 30.f * b4 - 75.f * c4);
-  else if (s < 2.f) v = C * (-5.f * a4 + 30.f * b4);
+  if (s < 1.f) v = C * fmaf(-75.f, c4, fmaf(30.f, b4, -5.f * a4));
+  else if (s < 2.f) v = C * fmaf(30.f, b4, -5.f * a4);
   else if (s < 3.f) v = C * (-5.f * a4);
   else return 0.f;
   return v * ih * __frcp_rn(dist + 1.e-15f);

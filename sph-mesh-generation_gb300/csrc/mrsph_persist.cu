@@ -4,7 +4,7 @@
 // The reference relaxes one geometry per run (SPH_run_mesh_generation,
 // sph_mesh_generation.cpp:1371-1463, driven by Solver::SPH_Mesh_Generation_
 // Solver, solver.cpp:257-321).  Here each phase of a step (begin, map, the
-// three scan passes, scatter, rank, reorder, density, its fix-up, the two
+// three scan passes, scatter, reorder, density, the two
 // force stages with their spilled particles) is a work list of (geometry,
 // block) items over all geometries of a batch: blocks of 256 particles,
 // blocks of 4096 cells for the scans, or one item per geometry.  Every item
@@ -23,7 +23,7 @@
 //     Buffers read in one phase were written by other blocks earlier in the
 //     same launch, so the persistent kernel reads through coherent loads
 //     (LdPlain), never the read-only path.
-//   * phases: one launch per phase (14 per step) with one block per item,
+//   * phases: one launch per phase (12 per step) with one block per item,
 //     each phase its own kernel (own register allocation, read-only loads).
 #include <cuda_runtime.h>
 
@@ -48,8 +48,8 @@ constexpr int kBatchThreads = 256;
 constexpr int kBatchScanCells = kBatchThreads * SCAN_ITEMS;  // cells per scan item
 
 enum BatchPhase {
-  BP_BEGIN = 0, BP_MAP, BP_SCAN_REDUCE, BP_SCAN_TOP, BP_SCAN_DOWN, BP_SCATTER, BP_RANK, BP_REORDER,
-  BP_DENSITY, BP_FIX, BP_FORCE1, BP_SPILL1, BP_FORCE2, BP_SPILL2, BP_COUNT
+  BP_BEGIN = 0, BP_MAP, BP_SCAN_REDUCE, BP_SCAN_TOP, BP_SCAN_DOWN, BP_SCATTER, BP_REORDER,
+  BP_DENSITY, BP_FORCE1, BP_SPILL1, BP_FORCE2, BP_SPILL2, BP_COUNT
 };
 
 // A force stage's listed and spilled particles are independent of each
@@ -61,14 +61,13 @@ __host__ __device__ inline bool barrier_after(int ph) { return ph != BP_FORCE1 &
 // per-handle kernels' tuning
 __host__ __device__ constexpr int phase_min_blocks(int ph) {
   return ph == BP_MAP ? MRSPH_MAP_MIN_BLOCKS
-         : ph == BP_DENSITY ? MRSPH_DENSITY_MIN_BLOCKS
+         : ph == BP_DENSITY ? 4
          : ph == BP_FORCE1 ? MRSPH_FORCE_MIN_BLOCKS
          : ph == BP_FORCE2 ? MRSPH_FORCE2_MIN_BLOCKS : 1;
 }
 
 // item lists: 0 one item per geometry, 1 particle blocks, 2 scan blocks,
-// 3 queue blocks (the density fix-up and the spilled force stages, whose
-// queues hold a few per cent of a geometry's particles at most: one item per
+// 3 queue blocks (the spilled force stages, whose queues hold a few per cent of a geometry's particles at most: one item per
 // MRSPH_BATCH_QUEUE_DIV particle blocks, at least one per geometry, each
 // striding over the geometry's queue)
 constexpr int kBatchLists = 4;
@@ -78,7 +77,7 @@ constexpr int kBatchLists = 4;
 __host__ __device__ inline int phase_list(int ph) {
   return (ph == BP_BEGIN || ph == BP_SCAN_TOP) ? 0
          : (ph == BP_SCAN_REDUCE || ph == BP_SCAN_DOWN) ? 2
-         : (ph == BP_FIX || ph == BP_SPILL1 || ph == BP_SPILL2) ? 3 : 1;
+         : (ph == BP_SPILL1 || ph == BP_SPILL2) ? 3 : 1;
 }
 
 // items a block claims at a time from a phase's work queue
@@ -158,8 +157,13 @@ __device__ inline void load_slot(const BatchPlan& P, int g, BatchSlot& s_slot, i
   __syncthreads();
 }
 
+union PhaseTiles {  // shared memory of the phases that scan cells
+  WarpTile tile[kBatchThreads / 32];
+  GroupTile<float> spill[kBatchThreads / kG];
+};
+
 template <int D, int KK, class LD>
-__device__ inline void run_item_d(const BatchSlot& S, int ph, long long blk, long long nblk, int cur) {
+__device__ inline void run_item_d(const BatchSlot& S, int ph, long long blk, long long nblk, int cur, PhaseTiles& sm) {
   const Buf<float>& b0 = S.buf[cur];      // the step's state before the reorder
   const Buf<float>& b1 = S.buf[cur ^ 1];  // after it
   switch (ph) {
@@ -174,22 +178,21 @@ __device__ inline void run_item_d(const BatchSlot& S, int ph, long long blk, lon
     case BP_SCAN_TOP: scan_top_block(S.w.blocksums, (S.ncells + kBatchScanCells - 1) / kBatchScanCells); break;
     case BP_SCAN_DOWN: scan_down_block(S.w.counts, S.ncells, S.w.blocksums, S.w.cstart, (int)S.c.n, blk); break;
     case BP_SCATTER: scatter_block(b0.cellkey, S.w.counts, S.w.cstart, S.w.perm, S.c.n, blk); break;
-    case BP_RANK: rank_block(b0.cellkey, S.w.cstart, S.w.perm, b0.id, S.w.perm2, S.c.n, blk); break;
-    case BP_REORDER: reorder_block<D, float>(b0, b1, S.c, S.w.perm2, S.w.slot_of_id, S.c.n, 0, blk); break;
-    case BP_DENSITY: density_block<D, float, KK, LD>(S.c, b1, S.w, blk); break;
-    case BP_FIX: density_fix_items<D, KK, LD>(S.c, b1, S.w, blk, nblk); break;
+    case BP_REORDER: reorder_block<D, float, LD>(b0, b1, S.c, S.w, 0, blk); break;
+    case BP_DENSITY: density_warp_block<D, LD>(S.c, b1, S.w, sm.tile, blk * kBatchThreads); break;
     case BP_FORCE1:
       if (blk == 0 && threadIdx.x == 0) accum_pairs_body(S.c.sc);
-      force_block<D, float, 1, KK, LD>(S.c, b1, S.w, blk);
+      force_block<D, float, 1, KK, 1, LD>(S.c, b1, S.w, nullptr, blk * kBatchThreads);
       break;
-    case BP_SPILL1: force_spill_items<D, float, 1, KK, LD>(S.c, b1, S.w, blk, nblk); break;
-    case BP_FORCE2: force_block<D, float, 2, KK, LD>(S.c, b1, S.w, blk); break;
-    case BP_SPILL2: force_spill_items<D, float, 2, KK, LD>(S.c, b1, S.w, blk, nblk); break;
+    case BP_SPILL1: force_spill_items<D, float, 1, KK, LD>(S.c, b1, S.w, sm.spill, blk, nblk); break;
+    case BP_FORCE2: force_block<D, float, 2, KK, 1, LD>(S.c, b1, S.w, nullptr, blk * kBatchThreads); break;
+    case BP_SPILL2: force_spill_items<D, float, 2, KK, LD>(S.c, b1, S.w, sm.spill, blk, nblk); break;
   }
 }
 
 template <int KK, class LD>
-__device__ inline void run_item(const BatchPlan& P, int ph, long long it, int step, BatchSlot& s_slot, int& s_g) {
+__device__ inline void run_item(const BatchPlan& P, int ph, long long it, int step, BatchSlot& s_slot, int& s_g,
+                                PhaseTiles& sm) {
   const int list = phase_list(ph);
   const long long* off = P.off + list * (P.ng + 1);
   const int g = item_geometry(off, P.ng, it);
@@ -202,11 +205,11 @@ __device__ inline void run_item(const BatchPlan& P, int ph, long long it, int st
   // so its results stay those of stepping it alone
   const bool wen = KK < 0 && s_slot.c.prm.kernel == K_WEN;
   if (s_slot.dim == 2) {
-    if (wen) run_item_d<2, K_WEN, LD>(s_slot, ph, blk, nblk, cur);
-    else run_item_d<2, KK, LD>(s_slot, ph, blk, nblk, cur);
+    if (wen) run_item_d<2, K_WEN, LD>(s_slot, ph, blk, nblk, cur, sm);
+    else run_item_d<2, KK, LD>(s_slot, ph, blk, nblk, cur, sm);
   } else {
-    if (wen) run_item_d<3, K_WEN, LD>(s_slot, ph, blk, nblk, cur);
-    else run_item_d<3, KK, LD>(s_slot, ph, blk, nblk, cur);
+    if (wen) run_item_d<3, K_WEN, LD>(s_slot, ph, blk, nblk, cur, sm);
+    else run_item_d<3, KK, LD>(s_slot, ph, blk, nblk, cur, sm);
   }
 }
 
@@ -214,6 +217,7 @@ template <int KK>
 __global__ void __launch_bounds__(kBatchThreads, MRSPH_BATCH_MIN_BLOCKS) k_batch_persist(BatchPlan P) {
   __shared__ BatchSlot s_slot;
   __shared__ int s_g;
+  __shared__ PhaseTiles sm;
   if (threadIdx.x == 0) s_g = -1;
   __syncthreads();
   __shared__ long long s_it;
@@ -231,7 +235,7 @@ __global__ void __launch_bounds__(kBatchThreads, MRSPH_BATCH_MIN_BLOCKS) k_batch
         __syncthreads();
         if (it0 >= n) break;
         const long long it1 = it0 + MRSPH_BATCH_CHUNK < n ? it0 + MRSPH_BATCH_CHUNK : n;
-        for (long long it = it0; it < it1; it++) run_item<KK, LdPlain>(P, ph, it, P.step0 + st, s_slot, s_g);
+        for (long long it = it0; it < it1; it++) run_item<KK, LdPlain>(P, ph, it, P.step0 + st, s_slot, s_g, sm);
       }
       if (barrier_after(ph) && !grid_barrier(P.bar, P.err, ++epoch, P.limit_ns)) return;
     }
@@ -242,9 +246,10 @@ template <int KK, int PH>
 __global__ void __launch_bounds__(kBatchThreads, phase_min_blocks(PH)) k_batch_phase(BatchPlan P) {
   __shared__ BatchSlot s_slot;
   __shared__ int s_g;
+  __shared__ PhaseTiles sm;
   if (threadIdx.x == 0) s_g = -1;
   __syncthreads();
-  run_item<KK, LdNC>(P, PH, blockIdx.x, P.step0, s_slot, s_g);
+  run_item<KK, LdNC>(P, PH, blockIdx.x, P.step0, s_slot, s_g, sm);
 }
 
 // A barrier that one block never reaches: the others give up after limit_ns.
@@ -295,10 +300,8 @@ cudaError_t launch_phases(const BatchPlan& P, cudaStream_t s) {
   if (e == cudaSuccess) e = L(k_batch_phase<KK, BP_SCAN_TOP>, BP_SCAN_TOP);
   if (e == cudaSuccess) e = L(k_batch_phase<KK, BP_SCAN_DOWN>, BP_SCAN_DOWN);
   if (e == cudaSuccess) e = L(k_batch_phase<KK, BP_SCATTER>, BP_SCATTER);
-  if (e == cudaSuccess) e = L(k_batch_phase<KK, BP_RANK>, BP_RANK);
   if (e == cudaSuccess) e = L(k_batch_phase<KK, BP_REORDER>, BP_REORDER);
   if (e == cudaSuccess) e = L(k_batch_phase<KK, BP_DENSITY>, BP_DENSITY);
-  if (e == cudaSuccess) e = L(k_batch_phase<KK, BP_FIX>, BP_FIX);
   if (e == cudaSuccess) e = L(k_batch_phase<KK, BP_FORCE1>, BP_FORCE1);
   if (e == cudaSuccess) e = L(k_batch_phase<KK, BP_SPILL1>, BP_SPILL1);
   if (e == cudaSuccess) e = L(k_batch_phase<KK, BP_FORCE2>, BP_FORCE2);

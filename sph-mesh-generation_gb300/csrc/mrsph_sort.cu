@@ -26,11 +26,6 @@ __global__ void k_scatter(const int* __restrict__ cellkey, int* cursor, const in
   scatter_block(cellkey, cursor, cstart, perm, n, blockIdx.x);
 }
 
-__global__ void k_rank(const int* __restrict__ cellkey, const int* __restrict__ cstart,
-                       const int* __restrict__ perm, const int* __restrict__ id, int* __restrict__ perm2,
-                       long long n) {
-  rank_block(cellkey, cstart, perm, id, perm2, n, blockIdx.x);
-}
 }  // namespace
 
 // block totals of the smallest chunk (the batch kernels' 256-thread scans)
@@ -46,12 +41,6 @@ void cell_scan(int* counts, int* cstart, int* blocksums, long long ncells, int n
 void cell_scatter(const int* cellkey, int* cursor, const int* cstart, int* perm, long long n, cudaStream_t s) {
   int nb = (int)((n + 255) / 256);
   k_scatter<<<nb, 256, 0, s>>>(cellkey, cursor, cstart, perm, n);
-}
-
-void cell_rank(const int* cellkey, const int* cstart, const int* perm, const int* id, int* perm2, long long n,
-               cudaStream_t s) {
-  int nb = (int)((n + 255) / 256);
-  k_rank<<<nb, 256, 0, s>>>(cellkey, cstart, perm, id, perm2, n);
 }
 
 }  // namespace mrsph

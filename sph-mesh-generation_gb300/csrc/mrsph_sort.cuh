@@ -8,7 +8,7 @@
 //   counts[key]++            (atomic, inside the map kernel)
 //   cstart = exclusive_scan(counts), cstart[ncells] = n
 //   perm[cstart[key] + --counts[key]] = i   (atomic; leaves counts at zero)
-//   rank inside each cell by particle id -> perm2 (canonical, deterministic)
+//   reorder (engine.cuh): rank inside each cell by particle id (canonical, deterministic)
 //
 // cstart doubles as the dense lower-bound table used by the neighbour scan:
 // every (empty or not) cell has a start, so a run of cells in a row is one
@@ -149,20 +149,6 @@ __device__ inline void scatter_block(const int* cellkey, int* cursor, const int*
   int c = cellkey[i];
   int slot = cstart[c] + atomicSub(&cursor[c], 1) - 1;
   if (slot >= 0 && slot < n) perm[slot] = (int)i;  // a histogram out of step with the keys cannot write outside
-}
-
-// Canonical order inside a cell: ascending particle id.
-__device__ inline void rank_block(const int* cellkey, const int* cstart, const int* perm, const int* id, int* perm2,
-                                  long long n, long long blk) {
-  long long s = blk * blockDim.x + threadIdx.x;
-  if (s >= n) return;
-  int o = perm[s];
-  int c = cellkey[o];
-  int b = cstart[c], e = cstart[c + 1];
-  int my = id[o];
-  int r = 0;
-  for (int t = b; t < e; t++) r += (id[perm[t]] < my) ? 1 : 0;
-  perm2[b + r] = o;
 }
 
 }  // namespace mrsph

@@ -1,9 +1,8 @@
 """Autotuner of the neighbour passes' tile shapes and per-block work splits.
 
-The FP32 density and force kernels take their shared-memory tile criterion
-(MRSPH_TILE_SPAN_X / _YZ: the largest spread of a warp's half cells for which
-it scans through shared-memory tiles), the unroll of the tile loop
-(MRSPH_TILE_UNROLL) and their resident blocks per SM, i.e. registers per
+The FP32 list and force kernels take their shared-memory tile (MRSPH_TILE_SIZE
+candidates; MRSPH_TILE_SPAN_X / _YZ: the spread in half cells within which a
+warp's particles share one) and their resident blocks per SM, i.e. registers per
 thread and work per SM (MRSPH_DENSITY_MIN_BLOCKS, MRSPH_FORCE_MIN_BLOCKS,
 MRSPH_FORCE2_MIN_BLOCKS, MRSPH_MAP_MIN_BLOCKS), as compile-time macros; the
 persistent batch kernel its resident blocks per SM (MRSPH_BATCH_MIN_BLOCKS)
@@ -31,12 +30,12 @@ from . import build as _build
 
 # the engine's defaults (csrc/engine.cuh) and the values tried per macro
 DEFAULTS: Dict[str, int] = {"DENSITY_MIN_BLOCKS": 6, "FORCE_MIN_BLOCKS": 5, "FORCE2_MIN_BLOCKS": 6,
-                            "MAP_MIN_BLOCKS": 4, "TILE_UNROLL": 1, "TILE_SPAN_X": 3, "TILE_SPAN_YZ": 1}
+                            "MAP_MIN_BLOCKS": 4, "TILE_SIZE": 256, "TILE_SPAN_X": 15, "TILE_SPAN_YZ": 1}
 BATCH_DEFAULTS: Dict[str, int] = {"BATCH_MIN_BLOCKS": 4, "BATCH_CHUNK": 2}
 BATCH_SPACE: Dict[str, List[int]] = {"BATCH_MIN_BLOCKS": [2, 3, 4, 5, 6], "BATCH_CHUNK": [1, 2, 4, 8]}
-SPACE: Dict[str, List[int]] = {"DENSITY_MIN_BLOCKS": [4, 5, 6], "FORCE_MIN_BLOCKS": [4, 5, 6],
+SPACE: Dict[str, List[int]] = {"DENSITY_MIN_BLOCKS": [5, 6, 7], "FORCE_MIN_BLOCKS": [4, 5, 6],
                                "FORCE2_MIN_BLOCKS": [5, 6, 8], "MAP_MIN_BLOCKS": [3, 4],
-                               "TILE_UNROLL": [1, 4], "TILE_SPAN_X": [3, 5, 7], "TILE_SPAN_YZ": [0, 1, 2]}
+                               "TILE_SIZE": [128, 192, 256], "TILE_SPAN_X": [7, 15, 31], "TILE_SPAN_YZ": [1, 3]}
 
 WORKLOADS = {
     "torus_3d": "cases.torus_3d(precision='fp32')",
