@@ -78,7 +78,8 @@ struct Work {  // per-step arrays in sorted order
   int* order;       // storage slots in work order: bricks, Z-order of half cells inside a brick
   float* rlev;      // [level][particle]: search radius on the level (level_radius), 0 if none
   int* cstart;
-  int* perm;
+  int* perm;  // the counting sort's particles, cells in order, and their ids
+  int* pid;
   int* blocksums;
   int* slot_of_id;
   int* spillq;  // particles whose list spilled (count sc->nspill)
@@ -376,6 +377,7 @@ __device__ inline void begin_step_body(DevScalars* sc, int inc) {
 }
 // scalars of the step, and the step's per-level h maxima (n words) cleared
 static __global__ void k_begin_step(DevScalars* sc, int inc, unsigned* lhmax, long long n) {
+  chain_wait();
   const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (i == 0) begin_step_body(sc, inc);
   if (i < n) lhmax[i] = 0u;
@@ -673,6 +675,7 @@ __device__ inline void map_block(const KCtx& c, const Buf<R>& b, int* counts, un
 template <int D, class R>
 __global__ void __launch_bounds__(256, (std::is_same<R, float>::value ? MRSPH_MAP_MIN_BLOCKS : 1))
 k_map(KCtx c, Buf<R> b, int* counts, unsigned* lhmax, int mode, unsigned max_att) {
+  chain_wait();
   map_block<D, R>(c, b, counts, lhmax, mode, max_att, blockIdx.x);
 }
 
@@ -779,6 +782,7 @@ __device__ inline void brick_of(const CellGeo& g, long long t, int& L, int* q) {
 // one thread per brick: its particles, from the start table
 template <int D>
 __global__ void __launch_bounds__(256) k_brick_count(KCtx c, const int* __restrict__ cstart, int* __restrict__ bcount) {
+  chain_wait();
   const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= c.geo.boff[c.geo.ncl]) return;
   int L, q[3], n = 0;
@@ -799,6 +803,7 @@ template <int D>
 __global__ void __launch_bounds__(256) k_brick_order(KCtx c, const int* __restrict__ cstart,
                                                      const int* __restrict__ bcount, const int* __restrict__ bstart,
                                                      int* __restrict__ order) {
+  chain_wait();
   const int lane = threadIdx.x & 31;
   const long long base = ((long long)blockIdx.x * blockDim.x + threadIdx.x) & ~31ll, nb = c.geo.boff[c.geo.ncl];
   const long long mine = base + lane;
@@ -988,10 +993,10 @@ __device__ inline void reorder_block(const Buf<R>& src, const Buf<R>& dst, const
   const long long n = c.n;
   if (t >= n) return;
   const int o = w.perm[t];
-  const int ck = src.cellkey[o], id = src.id[o];
+  const int ck = src.cellkey[o], id = w.pid[t];
   const int c0 = LD::ld(&w.cstart[ck]), c1 = LD::ld(&w.cstart[ck + 1]);
   long long s = c0;
-  for (int u = c0; u < c1; u++) s += src.id[w.perm[u]] < id ? 1 : 0;
+  for (int u = c0; u < c1; u++) s += w.pid[u] < id ? 1 : 0;
   const auto p = src.posh[o];
   const int key = src.key ? src.key[o] : 0;
   const auto nr = src.nr[o];
@@ -1022,6 +1027,7 @@ __device__ inline void reorder_block(const Buf<R>& src, const Buf<R>& dst, const
 
 template <int D, class R>
 __global__ void k_reorder(Buf<R> src, Buf<R> dst, KCtx c, Work<R> w, int partial) {
+  chain_wait();
   reorder_block<D, R>(src, dst, c, w, partial, blockIdx.x);
 }
 
@@ -1589,11 +1595,13 @@ __device__ inline void density_warp_block(const KCtx& c, const Buf<float>& b, co
 constexpr int kDensityThreads = 128;
 template <int D, class R>
 __global__ void __launch_bounds__(kDensityThreads, 10) k_density_group(KCtx c, Buf<R> b, Work<R> w) {
+  chain_wait();
   __shared__ RowTile tiles[kDensityThreads / kG];
   density_group_block<D, R>(c, b, w, tiles, (long long)blockIdx.x * (kDensityThreads / kG));
 }
 template <int D>
 __global__ void __launch_bounds__(kDensityThreads, MRSPH_DENSITY_MIN_BLOCKS) k_density(KCtx c, Buf<float> b, Work<float> w) {
+  chain_wait();
   __shared__ WarpTile tiles[kDensityThreads / 32];
   density_warp_block<D>(c, b, w, tiles, (long long)blockIdx.x * kDensityThreads);
 }
@@ -1983,6 +1991,7 @@ __device__ inline void force_block(const KCtx& c, const Buf<R>& b, const Work<R>
 
 template <int D, class R, int STAGE, int KK>
 __global__ void __launch_bounds__(256, (std::is_same<R, float>::value ? (STAGE == 1 ? MRSPH_FORCE_MIN_BLOCKS : MRSPH_FORCE2_MIN_BLOCKS) : 1)) k_force(KCtx c, Buf<R> b, Work<R> w) {
+  chain_wait();
   if (STAGE < 2 && blockIdx.x == 0 && threadIdx.x == 0) accum_pairs_body(c.sc);
   force_block<D, R, STAGE, KK, 1>(c, b, w, nullptr, (long long)blockIdx.x * 256);
 }
@@ -1990,6 +1999,7 @@ __global__ void __launch_bounds__(256, (std::is_same<R, float>::value ? (STAGE =
 constexpr int kGroupThreads = 128;
 template <int D, class R, int STAGE, int KK>
 __global__ void __launch_bounds__(kGroupThreads, std::is_same<R, float>::value ? 8 : 1) k_force_group(KCtx c, Buf<R> b, Work<R> w) {
+  chain_wait();
   __shared__ GroupTile<R> gt[kGroupThreads / kG];
   if (STAGE < 2 && blockIdx.x == 0 && threadIdx.x == 0) accum_pairs_body(c.sc);
   force_block<D, R, STAGE, KK, kG>(c, b, w, gt, (long long)blockIdx.x * (kGroupThreads / kG));
@@ -2015,6 +2025,7 @@ __device__ inline void force_spill_items(const KCtx& c, const Buf<R>& b, const W
 
 template <int D, class R, int STAGE, int KK>
 __global__ void __launch_bounds__(kGroupThreads) k_force_spill(KCtx c, Buf<R> b, Work<R> w) {
+  chain_wait();
   __shared__ GroupTile<R> gt[kGroupThreads / kG];
   force_spill_items<D, R, STAGE, KK>(c, b, w, gt, blockIdx.x, gridDim.x);
 }
@@ -2593,21 +2604,21 @@ class Engine : public EngineBase {
   // map (mode) + counting sort + reorder; swaps cur_.
   int run_map_and_bin(int mode) {
     const long long n = n_;
-    k_map<D, R><<<grid(n), 256, 0, st_>>>(kc_, buf_[cur_], w_.counts, w_.lhmax, mode, 1000000u);
+    launch_chained(k_map<D, R>, grid(n), 256, st_, kc_, buf_[cur_], w_.counts, w_.lhmax, mode, 1000000u);
     MR_CK(cudaGetLastError());
     return bin(1);
   }
 
   void begin_step(int inc) {
     const long long nl = kc_.geo.nc0 * kc_.geo.ncl;
-    k_begin_step<<<grid(nl), 256, 0, st_>>>(kc_.sc, inc, w_.lhmax, nl);
+    launch_chained(k_begin_step, grid(nl), 256, st_, kc_.sc, inc, w_.lhmax, nl);
   }
 
   int bin(int partial) {
     const long long n = n_;
     cell_scan(w_.counts, w_.cstart, w_.blocksums, ncells_, (int)n, st_);
-    cell_scatter(buf_[cur_].cellkey, w_.counts, w_.cstart, w_.perm, n, st_);
-    k_reorder<D, R><<<grid(n), 256, 0, st_>>>(buf_[cur_], buf_[cur_ ^ 1], kc_, w_, partial);
+    cell_scatter(buf_[cur_].cellkey, buf_[cur_].id, w_.counts, w_.cstart, w_.perm, w_.pid, n, st_);
+    launch_chained(k_reorder<D, R>, grid(n), 256, st_, buf_[cur_], buf_[cur_ ^ 1], kc_, w_, partial);
     MR_CK(cudaGetLastError());
     cur_ ^= 1;
     return 0;
@@ -2621,21 +2632,21 @@ class Engine : public EngineBase {
     if constexpr (std::is_same<R, float>::value) {
       if (n > kListGroupMax) {
         const long long nb = kc_.geo.boff[kc_.geo.ncl];
-        k_brick_count<D><<<grid(nb), 256, 0, st_>>>(kc_, w_.cstart, w_.bcount);
+        launch_chained(k_brick_count<D>, grid(nb), 256, st_, kc_, w_.cstart, w_.bcount);
         cell_scan(w_.bcount, w_.bstart, w_.blocksums, nb, (int)n, st_);
-        k_brick_order<D><<<grid(nb), 256, 0, st_>>>(kc_, w_.cstart, w_.bcount, w_.bstart, w_.order);
-        k_density<D><<<(int)((n + kDensityThreads - 1) / kDensityThreads), kDensityThreads, 0, st_>>>(kc_, buf_[cur_], w_);
+        launch_chained(k_brick_order<D>, grid(nb), 256, st_, kc_, w_.cstart, w_.bcount, w_.bstart, w_.order);
+        launch_chained(k_density<D>, (unsigned)((n + kDensityThreads - 1) / kDensityThreads), kDensityThreads, st_, kc_, buf_[cur_], w_);
         grouped = false;
       }
     }
-    if (grouped) k_density_group<D, R><<<ggrid(kDensityThreads), kDensityThreads, 0, st_>>>(kc_, buf_[cur_], w_);
+    if (grouped) launch_chained(k_density_group<D, R>, ggrid(kDensityThreads), kDensityThreads, st_, kc_, buf_[cur_], w_);
   }
 
   template <int STAGE, int KK>
   void launch_force_kind() {
-    if (n_ <= kGroupMax) k_force_group<D, R, STAGE, KK><<<ggrid(kGroupThreads), kGroupThreads, 0, st_>>>(kc_, buf_[cur_], w_);
-    else k_force<D, R, STAGE, KK><<<grid(n_), 256, 0, st_>>>(kc_, buf_[cur_], w_);
-    k_force_spill<D, R, STAGE, KK><<<qgrid(), kGroupThreads, 0, st_>>>(kc_, buf_[cur_], w_);
+    if (n_ <= kGroupMax) launch_chained(k_force_group<D, R, STAGE, KK>, ggrid(kGroupThreads), kGroupThreads, st_, kc_, buf_[cur_], w_);
+    else launch_chained(k_force<D, R, STAGE, KK>, grid(n_), 256, st_, kc_, buf_[cur_], w_);
+    launch_chained(k_force_spill<D, R, STAGE, KK>, qgrid(), kGroupThreads, st_, kc_, buf_[cur_], w_);
   }
   template <int STAGE>
   void launch_force() {
@@ -2651,7 +2662,7 @@ class Engine : public EngineBase {
     auto mark = [&](int k) { if (ev) cudaEventRecord(ev[k], st_); };
     mark(0);
     begin_step(1);
-    k_map<D, R><<<grid(n), 256, 0, st_>>>(kc_, buf_[cur_], w_.counts, w_.lhmax, MAP_STEP, 1000000u);
+    launch_chained(k_map<D, R>, grid(n), 256, st_, kc_, buf_[cur_], w_.counts, w_.lhmax, (int)MAP_STEP, 1000000u);
     MR_CK(cudaGetLastError());
     mark(1);
     if (phase < MRSPH_PHASE_BIN) {  // the histogram is not consumed by a scatter: clear it
@@ -2660,9 +2671,9 @@ class Engine : public EngineBase {
     }
     cell_scan(w_.counts, w_.cstart, w_.blocksums, ncells_, (int)n, st_);
     mark(2);
-    cell_scatter(buf_[cur_].cellkey, w_.counts, w_.cstart, w_.perm, n, st_);
+    cell_scatter(buf_[cur_].cellkey, buf_[cur_].id, w_.counts, w_.cstart, w_.perm, w_.pid, n, st_);
     mark(3);
-    k_reorder<D, R><<<grid(n), 256, 0, st_>>>(buf_[cur_], buf_[cur_ ^ 1], kc_, w_, phase < MRSPH_PHASE_FORCE2 ? 1 : 0);
+    launch_chained(k_reorder<D, R>, grid(n), 256, st_, buf_[cur_], buf_[cur_ ^ 1], kc_, w_, phase < MRSPH_PHASE_FORCE2 ? 1 : 0);
     MR_CK(cudaGetLastError());
     cur_ ^= 1;
     mark(4);
@@ -2823,6 +2834,7 @@ class Engine : public EngineBase {
       rc |= A((void**)&w_.rlev, sizeof(float) * kc_.geo.ncl * n);
       rc |= A((void**)&w_.cstart, sizeof(int) * (ncells_ + 1));
       rc |= A((void**)&w_.perm, sizeof(int) * n);
+      rc |= A((void**)&w_.pid, sizeof(int) * n);
       rc |= A((void**)&w_.blocksums, sizeof(int) * scan_blocksums_size(ncells_));
       rc |= A((void**)&w_.slot_of_id, sizeof(int) * n);
       rc |= A((void**)&w_.spillq, sizeof(int) * n);

@@ -88,7 +88,8 @@ cudaError_t ls_volume_mass(const LsSet& ls, int level, int D, double* cvol, doub
 
 // sort / scan primitives (mrsph_sort.cu)
 void cell_scan(int* counts, int* cstart, int* blocksums, long long ncells, int ntotal, cudaStream_t s);
-void cell_scatter(const int* cellkey, int* cursor, const int* cstart, int* perm, long long n, cudaStream_t s);
+void cell_scatter(const int* cellkey, const int* id, int* cursor, const int* cstart, int* perm, int* pid, long long n,
+                  cudaStream_t s);
 long long scan_blocksums_size(long long ncells);
 
 }  // namespace mrsph

@@ -132,6 +132,29 @@ __host__ __device__ inline double u53(uint32_t a, uint32_t b) {
   return ((double)(a >> 5) * 67108864.0 + (double)(b >> 6)) * (1.0 / 9007199254740992.0);
 }
 
+// ---------------------------------------------------------------- launches
+// The kernels of a step are launched as programmatic dependents of one another:
+// a kernel's launch is prepared while the one before it runs, and begins with
+// chain_wait(), which returns once that kernel has finished and its writes are
+// visible (launched any other way, it does nothing).  8 steps of 8,745
+// particles take 430 us, 443 with plain launches; letting a kernel's blocks in
+// as soon as the one before has placed its own cost more than it gave (496 us,
+// and 20.2 against 18.8 ms for 2.4 M particles).
+__device__ __forceinline__ void chain_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+template <class... P, class... A>
+inline cudaError_t launch_chained(void (*kernel)(P...), unsigned grid, unsigned block, cudaStream_t s, A... args) {
+  cudaLaunchAttribute at{};
+  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(grid);
+  cfg.blockDim = dim3(block);
+  cfg.stream = s;
+  cfg.attrs = &at;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
+}
+
 // ---------------------------------------------------------------- helpers
 template <class R> struct V4;
 template <> struct V4<double> { using T = double4; };

@@ -177,7 +177,7 @@ __device__ inline void run_item_d(const BatchSlot& S, int ph, long long blk, lon
     case BP_SCAN_REDUCE: scan_reduce_block(S.w.counts, S.ncells, S.w.blocksums, blk); break;
     case BP_SCAN_TOP: scan_top_block(S.w.blocksums, (S.ncells + kBatchScanCells - 1) / kBatchScanCells); break;
     case BP_SCAN_DOWN: scan_down_block(S.w.counts, S.ncells, S.w.blocksums, S.w.cstart, (int)S.c.n, blk); break;
-    case BP_SCATTER: scatter_block(b0.cellkey, S.w.counts, S.w.cstart, S.w.perm, S.c.n, blk); break;
+    case BP_SCATTER: scatter_block(b0.cellkey, b0.id, S.w.counts, S.w.cstart, S.w.perm, S.w.pid, S.c.n, blk); break;
     case BP_REORDER: reorder_block<D, float, LD>(b0, b1, S.c, S.w, 0, blk); break;
     case BP_DENSITY: density_warp_block<D, LD>(S.c, b1, S.w, sm.tile, blk * kBatchThreads); break;
     case BP_FORCE1:

@@ -7,7 +7,7 @@
 //
 //   counts[key]++            (atomic, inside the map kernel)
 //   cstart = exclusive_scan(counts), cstart[ncells] = n
-//   perm[cstart[key] + --counts[key]] = i   (atomic; leaves counts at zero)
+//   perm[cstart[key] + --counts[key]] = i, its id beside it   (atomic; leaves counts at zero)
 //   reorder (engine.cuh): rank inside each cell by particle id (canonical, deterministic)
 //
 // cstart doubles as the dense lower-bound table used by the neighbour scan:
@@ -110,15 +110,26 @@ __device__ inline void scan_top_block(int* blocksums, long long nb) {
   }
 }
 
+// where a block's exclusive prefix comes from: its entry of the scanned block
+// totals; the sum of the raw totals before it, which the block adds up itself
+// (one launch fewer); nowhere (a single block)
+enum { SCAN_PREFIX = 0, SCAN_TOTALS = 1, SCAN_SINGLE = 2 };
 __device__ inline void scan_down_block(const int* counts, long long n, const int* blocksums, int* cstart, int ntotal,
-                                       long long blk) {
+                                       long long blk, int from = SCAN_PREFIX) {
+  int before = 0;
+  if (from == SCAN_PREFIX) before = blocksums[blk];
+  if (from == SCAN_TOTALS) {
+    int t = 0;
+    for (long long k = threadIdx.x; k < blk; k += blockDim.x) t += blocksums[k];
+    block_excl_scan(t, &before);
+  }
   long long base = blk * (long long)(blockDim.x * SCAN_ITEMS) + (long long)threadIdx.x * SCAN_ITEMS;
   int v[SCAN_ITEMS];
   load16(counts, base, n, v);
   int s = 0;
 #pragma unroll
   for (int k = 0; k < SCAN_ITEMS; k++) s += v[k];
-  int off = block_excl_scan(s, nullptr) + blocksums[blk];
+  int off = block_excl_scan(s, nullptr) + before;
   if (base + SCAN_ITEMS <= n) {
     int4* p = reinterpret_cast<int4*>(cstart + base);
 #pragma unroll
@@ -142,13 +153,16 @@ __device__ inline void scan_down_block(const int* counts, long long n, const int
 }
 
 // 256-thread block blk of particles
-__device__ inline void scatter_block(const int* cellkey, int* cursor, const int* cstart, int* perm, long long n,
-                                     long long blk) {
+__device__ inline void scatter_block(const int* cellkey, const int* id, int* cursor, const int* cstart, int* perm,
+                                     int* pid, long long n, long long blk) {
   long long i = blk * blockDim.x + threadIdx.x;
   if (i >= n) return;
   int c = cellkey[i];
   int slot = cstart[c] + atomicSub(&cursor[c], 1) - 1;
-  if (slot >= 0 && slot < n) perm[slot] = (int)i;  // a histogram out of step with the keys cannot write outside
+  if (slot >= 0 && slot < n) {  // a histogram out of step with the keys cannot write outside
+    perm[slot] = (int)i;
+    pid[slot] = id[i];
+  }
 }
 
 }  // namespace mrsph
