@@ -2158,6 +2158,23 @@ __global__ void k_sample_points(KCtx c, long long n, const double* __restrict__ 
   out[6 * i + 5] = (double)ls_tag<D, R>(c.ls, x);
 }
 
+// the same into separate arrays
+template <int D, class R>
+__global__ void k_sample_arrays(KCtx c, long long n, const double* __restrict__ xyz, double* __restrict__ phi,
+                                double* __restrict__ norm, double* __restrict__ curv, int* __restrict__ tag) {
+  const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  const double x[3] = {xyz[3 * i], xyz[3 * i + 1], xyz[3 * i + 2]};
+  R ph, nn[3], cv;
+  ls_sample<D, R>(c.ls, x, ph, nn, cv);
+  phi[i] = ph;
+  norm[3 * i] = nn[0];
+  norm[3 * i + 1] = nn[1];
+  norm[3 * i + 2] = nn[2];
+  curv[i] = cv;
+  tag[i] = ls_tag<D, R>(c.ls, x);
+}
+
 // ---------------------------------------------------------------------------
 // host engine
 // ---------------------------------------------------------------------------
@@ -2505,23 +2522,26 @@ class Engine : public EngineBase {
   }
 
   int sample(long long n, const double* xyz, double* phi, double* norm, double* curv, int* tag) override {
-    double *din = nullptr, *dout = nullptr;
-    MR_CK(cudaMalloc(&din, sizeof(double) * 3 * n));
-    MR_CK(cudaMalloc(&dout, sizeof(double) * 6 * n));
-    MR_CK(cudaMemcpyAsync(din, xyz, sizeof(double) * 3 * n, cudaMemcpyHostToDevice, st_));
-    k_sample_points<D, R><<<grid(n), 256, 0, st_>>>(kc_, n, din, dout);
-    std::vector<double> h((size_t)6 * n);
-    cudaError_t e = cudaMemcpyAsync(h.data(), dout, sizeof(double) * 6 * n, cudaMemcpyDeviceToHost, st_);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(st_);
-    cudaFree(din);
-    cudaFree(dout);
-    if (e != cudaSuccess) { err = cudaGetErrorString(e); return MRSPH_ERR_CUDA; }
-    for (long long i = 0; i < n; i++) {
-      if (phi) phi[i] = h[6 * i];
-      if (norm) for (int d = 0; d < 3; d++) norm[3 * i + d] = h[6 * i + 1 + d];
-      if (curv) curv[i] = h[6 * i + 4];
-      if (tag) tag[i] = (int)h[6 * i + 5];
+    // xyz, then the results as the caller's arrays want them: phi, normals, curvature, tags
+    double* d = nullptr;
+    MR_CK(cudaMallocAsync(&d, (sizeof(double) * 8 + sizeof(int)) * n, st_));
+    double *dphi = d + 3 * n, *dnorm = d + 4 * n, *dcurv = d + 7 * n;
+    int* dtag = reinterpret_cast<int*>(d + 8 * n);
+    cudaError_t e = cudaMemcpyAsync(d, xyz, sizeof(double) * 3 * n, cudaMemcpyHostToDevice, st_);
+    if (e == cudaSuccess) {
+      k_sample_arrays<D, R><<<grid(n), 256, 0, st_>>>(kc_, n, d, dphi, dnorm, dcurv, dtag);
+      e = cudaGetLastError();
     }
+    auto out = [&](void* to, const void* from, size_t bytes) {
+      if (to && e == cudaSuccess) e = cudaMemcpyAsync(to, from, bytes, cudaMemcpyDeviceToHost, st_);
+    };
+    out(phi, dphi, sizeof(double) * n);
+    out(norm, dnorm, sizeof(double) * 3 * n);
+    out(curv, dcurv, sizeof(double) * n);
+    out(tag, dtag, sizeof(int) * n);
+    cudaFreeAsync(d, st_);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(st_);
+    if (e != cudaSuccess) { err = cudaGetErrorString(e); return MRSPH_ERR_CUDA; }
     return 0;
   }
 

@@ -238,26 +238,35 @@ int mrsph_set_levelset(mrsph_handle* h, int nlevels, const mrsph_levelset_level*
     float* c32 = nullptr;
     uint8_t* tag = nullptr;
     uint8_t* act = nullptr;
-    API_CK(h, cudaMalloc(&d_phi, sizeof(double) * ntot));
-    h->ls_allocs.push_back(d_phi);
-    API_CK(h, cudaMalloc(&g64, sizeof(double4) * ntot));
-    h->ls_allocs.push_back(g64);
-    API_CK(h, cudaMalloc(&c64, sizeof(double) * ntot));
-    h->ls_allocs.push_back(c64);
-    API_CK(h, cudaMalloc(&g32, sizeof(float4) * ntot));
-    h->ls_allocs.push_back(g32);
-    API_CK(h, cudaMalloc(&c32, sizeof(float) * ntot));
-    h->ls_allocs.push_back(c32);
-    API_CK(h, cudaMalloc(&tag, ntot));
-    h->ls_allocs.push_back(tag);
-    API_CK(h, cudaMemcpyAsync(d_phi, in.phi, sizeof(double) * ntot, cudaMemcpyHostToDevice, h->stream));
+    long long np = 0;  // package mask, bytes
     if (in.active) {
-      long long np = 1;
+      np = 1;
       for (int d = 0; d < D; d++) np *= (in.num_pkg[d] + 2 * in.margin);
-      API_CK(h, cudaMalloc(&act, np));
-      h->ls_allocs.push_back(act);
-      API_CK(h, cudaMemcpyAsync(act, in.active, np, cudaMemcpyHostToDevice, h->stream));
     }
+    {
+      // one allocation for the level's arrays, each 256-byte aligned
+      size_t off = 0;
+      auto take = [&](size_t bytes) {
+        const size_t o = off;
+        off += (bytes + 255) & ~(size_t)255;
+        return o;
+      };
+      const size_t o_phi = take(sizeof(double) * ntot), o_g64 = take(sizeof(double4) * ntot);
+      const size_t o_c64 = take(sizeof(double) * ntot), o_g32 = take(sizeof(float4) * ntot);
+      const size_t o_c32 = take(sizeof(float) * ntot), o_tag = take(ntot), o_act = take(np);
+      char* base = nullptr;
+      API_CK(h, cudaMalloc(&base, off));
+      h->ls_allocs.push_back(base);
+      d_phi = reinterpret_cast<double*>(base + o_phi);
+      g64 = reinterpret_cast<double4*>(base + o_g64);
+      c64 = reinterpret_cast<double*>(base + o_c64);
+      g32 = reinterpret_cast<float4*>(base + o_g32);
+      c32 = reinterpret_cast<float*>(base + o_c32);
+      tag = reinterpret_cast<uint8_t*>(base + o_tag);
+      if (np) act = reinterpret_cast<uint8_t*>(base + o_act);
+    }
+    API_CK(h, cudaMemcpyAsync(d_phi, in.phi, sizeof(double) * ntot, cudaMemcpyHostToDevice, h->stream));
+    if (np) API_CK(h, cudaMemcpyAsync(act, in.active, np, cudaMemcpyHostToDevice, h->stream));
     API_CK(h, ls_build_level(bd, d_phi, g64, c64, g32, c32, tag, d_max, h->stream));
     L.g64 = g64;
     L.c64 = c64;
@@ -349,12 +358,29 @@ int mrsph_get_levelset(mrsph_handle* h, int level, double* nx, double* ny, doubl
   API_CK(h, cudaSetDevice(h->prm.device));
   const LsLevel& L = h->ls.lv[level];
   long long ntot = h->ls_ntot[level];
-  std::vector<double4> g(ntot);
-  API_CK(h, cudaMemcpy(g.data(), L.g64, sizeof(double4) * ntot, cudaMemcpyDeviceToHost));
-  for (long long a = 0; a < ntot; a++) {
-    if (nx) nx[a] = g[a].y;
-    if (ny) ny[a] = g[a].z;
-    if (nz) nz[a] = g[a].w;
+  if (nx || ny || nz) {
+    // split on the device, so that each component is one copy into the caller's
+    // array (a host buffer of the interleaved field and its de-interleaving took
+    // half of the call)
+    double* const out[3] = {nx, ny, nz};
+    double* d = nullptr;
+    if (cudaMallocAsync(&d, 3 * sizeof(double) * ntot, h->stream) == cudaSuccess) {
+      cudaError_t e = ls_split_normals(ntot, L.g64, d, h->stream);
+      for (int k = 0; k < 3 && e == cudaSuccess; k++)
+        if (out[k]) e = cudaMemcpyAsync(out[k], d + k * ntot, sizeof(double) * ntot, cudaMemcpyDeviceToHost, h->stream);
+      cudaFreeAsync(d, h->stream);
+      if (e == cudaSuccess) e = cudaStreamSynchronize(h->stream);
+      API_CK(h, e);
+    } else {  // no room on the device: through the host
+      cudaGetLastError();
+      std::vector<double4> g(ntot);
+      API_CK(h, cudaMemcpy(g.data(), L.g64, sizeof(double4) * ntot, cudaMemcpyDeviceToHost));
+      for (long long a = 0; a < ntot; a++) {
+        if (nx) nx[a] = g[a].y;
+        if (ny) ny[a] = g[a].z;
+        if (nz) nz[a] = g[a].w;
+      }
+    }
   }
   if (curv) API_CK(h, cudaMemcpy(curv, L.c64, sizeof(double) * ntot, cudaMemcpyDeviceToHost));
   if (tag) API_CK(h, cudaMemcpy(tag, L.tag, ntot, cudaMemcpyDeviceToHost));
