@@ -8,7 +8,7 @@
 //   Graphmeshcls::Reconstruct_tris (graph_mesh.cpp:37-409)
 //     -> k_tri_pass1 (3-cycles i > j > k, longest-edge deletion for all-boundary
 //        triangles whose centroid phi <= 1e-4 of the vertex mean), k_tri_alive
-//        (rebuild from the kept triangles), k_tri_pass2 (final 3-cycles,
+//        (rebuild from the kept triangles), k_tri_mirror, k_tri_pass2 (final 3-cycles,
 //        non-manifold and crossing checks)
 //   Tri_quality_statistics (graph_mesh.cpp:411-670) -> k_tri_quality
 // Exact predicate signs make the edge set independent of evaluation order, so
@@ -17,6 +17,7 @@
 
 #include <algorithm>
 #include <cstring>
+#include <initializer_list>
 #include <vector>
 
 #include "handle.h"
@@ -225,7 +226,7 @@ __device__ inline int row_find(const TriIn& T, int a, int b) {
 // 8 e |e_j||w| and the dot product w . (w - e_j) by 10 e (|w|^2 + |w||e_j|) (each
 // position rounded once); the constants below are larger.  All of this in FP64
 // (rate 1/60), an incircle determinant per point, took 9.9 ms for 77,551
-// particles; now 0.18 ms.
+// particles; now 0.16 ms.
 constexpr float kTE = 0x1p-24f;
 __host__ __device__ inline size_t mark_smem(int cap) { return (sizeof(float4) + 2 * sizeof(int)) * (size_t)cap; }  // per warp
 __global__ void k_tri_mark(TriIn T, unsigned char* mark, long long* queue, unsigned long long* nqueue) {
@@ -360,19 +361,27 @@ __global__ void __launch_bounds__(256) k_tri_adj(TriIn T, const unsigned char* m
   if (lane == 0) T.deg[i] = n;
 }
 
-// position of edge (a, b) in a's list, -1 if there is none
+// position of edge (a, b) in a's list, -1 if there is none; eight entries are in
+// flight at a time (lists have about six)
 __device__ inline long long edge_find(const TriIn& T, int a, int b) {
   const long long o = (long long)a * T.cap;
   const int n = T.deg[a];
-  for (int q = 0; q < n; q++)
-    if (T.adj[o + q] == b) return o + q;
+  for (int q0 = 0; q0 < n; q0 += 8) {
+    int v[8], hit = -1;
+#pragma unroll
+    for (int u = 0; u < 8; u++) v[u] = T.adj[o + min(q0 + u, n - 1)];
+#pragma unroll
+    for (int u = 7; u >= 0; u--)
+      if (v[u] == b) hit = min(q0 + u, n - 1);
+    if (hit >= 0) return o + hit;
+  }
   return -1;
 }
 
-// deletion rule of Reconstruct_tris (graph_mesh.cpp:144-205); returns true when kept,
-// else *ea/*eb = longest edge
-__device__ bool tri_rule(const TriIn& T, const LsSet& ls, int I, int j, int k, int* ea, int* eb) {
-  if (T.type[I] == REAL_P || T.type[j] == REAL_P || T.type[k] == REAL_P) return true;
+// deletion rule of Reconstruct_tris (graph_mesh.cpp:144-205): -1 when kept, else
+// the longest edge: 0 (I, j), 1 (j, k), 2 (I, k)
+__device__ int tri_rule(const TriIn& T, const LsSet& ls, int I, int j, int k) {
+  if (T.type[I] == REAL_P || T.type[j] == REAL_P || T.type[k] == REAL_P) return -1;
   const double* p1 = T.xyz + 3 * (long long)I;
   const double* p2 = T.xyz + 3 * (long long)j;
   const double* p3 = T.xyz + 3 * (long long)k;
@@ -381,65 +390,97 @@ __device__ bool tri_rule(const TriIn& T, const LsSet& ls, int I, int j, int k, i
   double pc, nn[3], cv;
   ls_sample<2, double>(ls, cen, pc, nn, cv);
   double phi_size = 1. / 3. * (T.phi[I] + T.phi[j] + T.phi[k]);
-  if (pc > 0.0001 * phi_size) return true;
+  if (pc > 0.0001 * phi_size) return -1;
   double v1[2] = {p2[0] - p1[0], p2[1] - p1[1]};
   double v2[2] = {p3[0] - p2[0], p3[1] - p2[1]};
   double v3[2] = {p1[0] - p3[0], p1[1] - p3[1]};
   double d = sqrt(v1[0] * v1[0] + v1[1] * v1[1]);
-  *ea = I; *eb = j;
+  int e = 0;
   double d2 = sqrt(v2[0] * v2[0] + v2[1] * v2[1]);
-  if (d2 > d) { d = d2; *ea = j; *eb = k; }
+  if (d2 > d) { d = d2; e = 1; }
   double d3 = sqrt(v3[0] * v3[0] + v3[1] * v3[1]);
-  if (d3 > d) { d = d3; *ea = I; *eb = k; }
-  return false;
+  if (d3 > d) { d = d3; e = 2; }
+  return e;
 }
 
-__device__ inline void set_flag(const TriIn& T, unsigned* fl, int a, int b) {
-  long long p = edge_find(T, a, b);
-  if (p >= 0) atomicOr(&fl[p], 1u);
-  p = edge_find(T, b, a);
-  if (p >= 0) atomicOr(&fl[p], 1u);
-}
+// The passes over the triangles i > j > k run on kTG lanes per particle, which
+// share its pairs of edges; flags of an edge are kept at its larger end while
+// they are formed, where a triangle already knows their places.  One thread per
+// particle left each SM a chain of dependent loads: 231 (k_tri_pass1), 347
+// (k_tri_alive), 136 and 120 us (k_tri_pass2) for 77,551 particles; now 125, 54,
+// 60 and 45, and 25 for k_tri_mirror.
+constexpr int kTG = 8;
 
 // pass 1a: deleted edges
-__global__ void k_tri_pass1(TriIn T, LsSet ls, unsigned* del) {
-  long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= T.n) return;
-  const int* A = T.adj + i * T.cap;
-  const int c = T.deg[i];
-  for (int a = 0; a < c; a++) {
-    int j = A[a];
-    if (j >= i) break;
-    for (int b = 0; b < a; b++) {
-      int k = A[b];
-      if (edge_find(T, j, k) < 0) continue;
-      int ea, eb;
-      if (!tri_rule(T, ls, (int)i, j, k, &ea, &eb)) set_flag(T, del, ea, eb);
-    }
-  }
-}
-
-// pass 1b: edges of kept triangles without a deleted edge are alive
-__global__ void k_tri_alive(TriIn T, LsSet ls, const unsigned* del, unsigned* alive) {
-  long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+__global__ void __launch_bounds__(256) k_tri_pass1(TriIn T, LsSet ls, unsigned* del) {
+  const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x, i = t / kTG;
+  const int g = (int)(t % kTG);
   if (i >= T.n) return;
   const long long o = i * T.cap;
   const int* A = T.adj + o;
   const int c = T.deg[i];
+  int p = 0;
   for (int a = 0; a < c; a++) {
-    int j = A[a];
+    const int j = A[a];
     if (j >= i) break;
-    for (int b = 0; b < a; b++) {
-      int k = A[b];
+    for (int b = 0; b < a; b++, p++) {
+      if (p % kTG != g) continue;
+      const int k = A[b];
       const long long jk = edge_find(T, j, k);
       if (jk < 0) continue;
-      int ea, eb;
-      if (!tri_rule(T, ls, (int)i, j, k, &ea, &eb)) continue;
-      if (del[o + a] || del[o + b] || del[jk]) continue;
-      set_flag(T, alive, (int)i, j);
-      set_flag(T, alive, (int)i, k);
-      set_flag(T, alive, j, k);
+      const int e = tri_rule(T, ls, (int)i, j, k);
+      if (e >= 0) del[e == 0 ? o + a : (e == 1 ? jk : o + b)] = 1u;
     }
+  }
+}
+
+// pass 1b: edges of kept triangles without a deleted edge are alive.  A triangle
+// that the rule does not keep has its longest edge deleted, so the rule is not
+// asked again.
+__global__ void __launch_bounds__(256) k_tri_alive(TriIn T, const unsigned* del, unsigned* alive) {
+  const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x, i = t / kTG;
+  const int g = (int)(t % kTG);
+  if (i >= T.n) return;
+  const long long o = i * T.cap;
+  const int* A = T.adj + o;
+  const int c = T.deg[i];
+  int p = 0;
+  for (int a = 0; a < c; a++) {
+    const int j = A[a];
+    if (j >= i) break;
+    for (int b = 0; b < a; b++, p++) {
+      if (p % kTG != g || del[o + a] || del[o + b]) continue;
+      const long long jk = edge_find(T, j, A[b]);
+      if (jk < 0 || del[jk]) continue;
+      alive[o + a] = 1u;
+      alive[o + b] = 1u;
+      alive[jk] = 1u;
+    }
+  }
+}
+
+// the alive flags of the smaller ends; edges and deleted edges of the first pass
+__global__ void __launch_bounds__(256) k_tri_mirror(TriIn T, const unsigned* del, unsigned* alive,
+                                                    unsigned long long* stats) {
+  const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x, i = t / kTG;
+  unsigned e1 = 0, nd = 0;
+  if (i < T.n) {
+    const long long o = i * T.cap;
+    const int c = T.deg[i];
+    for (int a = (int)(t % kTG); a < c; a += kTG) {
+      const int j = T.adj[o + a];
+      if (j < i) continue;
+      const long long p = edge_find(T, j, (int)i);
+      e1++;
+      if (p >= 0 && del[p]) nd++;
+      if (p >= 0 && alive[p]) alive[o + a] = 1u;
+    }
+  }
+  e1 = __reduce_add_sync(0xffffffffu, e1);
+  nd = __reduce_add_sync(0xffffffffu, nd);
+  if ((threadIdx.x & 31) == 0) {
+    if (e1) atomicAdd(&stats[2], (unsigned long long)e1);
+    if (nd) atomicAdd(&stats[3], (unsigned long long)nd);
   }
 }
 
@@ -448,73 +489,55 @@ __device__ inline bool is_alive(const TriIn& T, const unsigned* alive, int a, in
   return p >= 0 && alive[p];
 }
 
-// pass 2: final triangles (count or fill) and edge checks (graph_mesh.cpp:300-365)
+// pass 2: final triangles (count or fill) and edge checks (graph_mesh.cpp:300-365).
+// The lanes of a particle test the third vertices of one edge together; ballots
+// give their order.
 template <bool FILL>
-__global__ void k_tri_pass2(TriIn T, const unsigned* alive, int* count, const int* offset, int* tris,
-                            unsigned long long* stats) {
-  long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  unsigned long long nerr = 0, nedge = 0;
+__global__ void __launch_bounds__(256) k_tri_pass2(TriIn T, const unsigned* alive, int* count, const int* offset,
+                                                   int* tris, unsigned long long* stats) {
+  const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x, i = t / kTG;
+  const int g = (int)(t % kTG), lane = threadIdx.x & 31, g0 = lane - g;
+  const unsigned gm = ((1u << kTG) - 1u) << g0;
+  unsigned nerr = 0, nedge = 0;
   if (i < T.n) {
     const int* S = T.adj + i * T.cap;
     const unsigned* A = alive + i * T.cap;
     const int c = T.deg[i];
     int ntri = 0;
-    int base = FILL ? offset[i] : 0;
+    const int base = FILL ? offset[i] : 0;
     for (int a = 0; a < c; a++) {
-      int j = S[a];
+      const int j = S[a];
       if (j >= i) break;
       if (!A[a]) continue;
       nedge++;
-      int common = 0, c0 = -1, c1 = -1;
-      for (int b = 0; b < c; b++) {
-        int k = S[b];
-        if (k == j || !A[b]) continue;
-        if (!is_alive(T, alive, j, k)) continue;
-        if (common == 0) c0 = k; else if (common == 1) c1 = k;
-        common++;
-        if (k < j) {
-          if (FILL) {
-            int* o = tris + 3 * (long long)(base + ntri);
-            o[0] = (int)i; o[1] = j; o[2] = k;
-          }
-          ntri++;
+      int total = 0, c0 = -1, c1 = -1;  // third vertices, the first two of them
+      for (int b0 = 0; b0 < c; b0 += kTG) {
+        const int b = b0 + g;
+        const int k = b < c ? S[b] : j;
+        const bool hit = k != j && A[b] && is_alive(T, alive, j, k);
+        const unsigned all = __ballot_sync(gm, hit) >> g0;
+        const unsigned low = __ballot_sync(gm, hit && k < j) >> g0;
+        int seen = total;
+        for (unsigned m = all; m && seen < 2; m &= m - 1u, seen++) (seen ? c1 : c0) = S[b0 + __ffs(m) - 1];
+        if (FILL && hit && k < j) {
+          int* o = tris + 3 * (long long)(base + ntri + __popc(low & ((1u << g) - 1u)));
+          o[0] = (int)i; o[1] = j; o[2] = k;
         }
+        ntri += __popc(low);
+        total += __popc(all);
       }
-      if (!FILL && (common > 2 || (common == 2 && is_alive(T, alive, c0, c1)))) nerr++;
+      if (!FILL && g == 0 && (total > 2 || (total == 2 && is_alive(T, alive, c0, c1)))) nerr++;
     }
-    if (!FILL) count[i] = ntri;
+    if (!FILL && g == 0) count[i] = ntri;
+    if (g) nedge = 0;
   }
-  if (!FILL && stats) {
-    for (int o = 16; o > 0; o >>= 1) {
-      nerr += __shfl_xor_sync(0xffffffffu, nerr, o);
-      nedge += __shfl_xor_sync(0xffffffffu, nedge, o);
+  if (!FILL) {
+    nerr = __reduce_add_sync(0xffffffffu, nerr);
+    nedge = __reduce_add_sync(0xffffffffu, nedge);
+    if (lane == 0) {
+      if (nerr) atomicAdd(&stats[0], (unsigned long long)nerr);
+      if (nedge) atomicAdd(&stats[1], (unsigned long long)nedge);
     }
-    if ((threadIdx.x & 31) == 0) {
-      if (nerr) atomicAdd(&stats[0], nerr);
-      if (nedge) atomicAdd(&stats[1], nedge);
-    }
-  }
-}
-
-__global__ void k_tri_count_first(TriIn T, const unsigned* del, unsigned long long* stats) {
-  long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  unsigned long long e1 = 0, nd = 0;
-  if (i < T.n) {
-    const long long o = i * T.cap;
-    const int c = T.deg[i];
-    for (int a = 0; a < c; a++) {
-      if (T.adj[o + a] <= i) continue;
-      e1++;
-      if (del[o + a]) nd++;
-    }
-  }
-  for (int o = 16; o > 0; o >>= 1) {
-    e1 += __shfl_xor_sync(0xffffffffu, e1, o);
-    nd += __shfl_xor_sync(0xffffffffu, nd, o);
-  }
-  if ((threadIdx.x & 31) == 0) {
-    if (e1) atomicAdd(&stats[2], e1);
-    if (nd) atomicAdd(&stats[3], nd);
   }
 }
 
@@ -639,9 +662,19 @@ extern "C" int mrsph_triangulate(mrsph_handle* h, int* tris, long long cap, long
   cudaStream_t s = h->stream;
   std::vector<void*> mem;
   int rc = 0;
-  auto A = [&](void** p, size_t bytes) -> bool {
-    if (cudaMalloc(p, bytes) != cudaSuccess) return false;
-    mem.push_back(*p);
+  // one allocation for the buffers of known size (each 256-byte aligned), one for
+  // those of the mesh
+  struct Part { void** p; size_t bytes; };
+  auto A = [&](std::initializer_list<Part> parts) -> bool {
+    size_t all = 0;
+    for (const Part& q : parts) all += (q.bytes + 255) & ~(size_t)255;
+    char* base = nullptr;
+    if (cudaMalloc(&base, all) != cudaSuccess) return false;
+    mem.push_back(base);
+    for (const Part& q : parts) {
+      *q.p = base;
+      base += (q.bytes + 255) & ~(size_t)255;
+    }
     return true;
   };
   double *d_xyz = nullptr, *d_phi = nullptr;
@@ -656,26 +689,27 @@ extern "C" int mrsph_triangulate(mrsph_handle* h, int* tris, long long cap, long
   double* d_scratch = nullptr;
   constexpr size_t kMarkSmem = 200 * 1024;
   int wpb = 0;
-  const int XB = 152 * 4, XT = 64;  // exact-predicate launch: four blocks per SM
+  const int XB = 152, XT = 64;  // exact-predicate launch: a block per SM, 40 MB of scratch
   const size_t NC = (size_t)n * rowcap;
   long long ntri = 0;
   unsigned flags = 0;
   unsigned long long st[4] = {0, 0, 0, 0}, hist[45];
   TriStat tq;
   std::memset(&tq, 0, sizeof(tq));
-  if (!A((void**)&d_xyz, sizeof(double) * 3 * n) || !A((void**)&d_phi, sizeof(double) * n) ||
-      !A((void**)&d_type, sizeof(int) * n) || !A((void**)&d_rows, sizeof(int) * NC) ||
-      !A((void**)&d_cnt, sizeof(int) * n) || !A((void**)&d_count, sizeof(int) * (n + 1)) ||
-      !A((void**)&d_off, sizeof(int) * (n + 1)) || !A((void**)&d_blk, sizeof(int) * scan_blocksums_size(n)) ||
-      !A((void**)&d_mark, NC) || !A((void**)&d_adj, sizeof(int) * NC) || !A((void**)&d_deg, sizeof(int) * n) ||
-      !A((void**)&d_queue, sizeof(long long) * NC) || !A((void**)&d_del, sizeof(unsigned) * NC) ||
-      !A((void**)&d_alive, sizeof(unsigned) * NC) || !A((void**)&d_flags, sizeof(unsigned)) ||
-      !A((void**)&d_stats, sizeof(unsigned long long) * 5) ||
-      !A((void**)&d_hist, sizeof(unsigned long long) * 45) ||
-      !A((void**)&d_scratch, sizeof(double) * 2 * XCAP * XB * XT)) {
+  if (!A({{(void**)&d_xyz, sizeof(double) * 3 * n}, {(void**)&d_phi, sizeof(double) * n},
+          {(void**)&d_type, sizeof(int) * n}, {(void**)&d_rows, sizeof(int) * NC}, {(void**)&d_cnt, sizeof(int) * n},
+          {(void**)&d_count, sizeof(int) * (n + 1)}, {(void**)&d_off, sizeof(int) * (n + 1)},
+          {(void**)&d_blk, sizeof(int) * scan_blocksums_size(n)}, {(void**)&d_mark, NC},
+          {(void**)&d_adj, sizeof(int) * NC}, {(void**)&d_deg, sizeof(int) * n},
+          {(void**)&d_queue, sizeof(long long) * NC}, {(void**)&d_flags, sizeof(unsigned)},
+          {(void**)&d_stats, sizeof(unsigned long long) * 5}, {(void**)&d_hist, sizeof(unsigned long long) * 45},
+          {(void**)&d_scratch, sizeof(double) * 2 * XCAP * XB * XT}})) {
     rc = tfail(h, MRSPH_ERR_OOM, "cudaMalloc failed");
     goto done;
   }
+  // the flags of the edge lists take the queue's place: it is spent by then
+  d_del = reinterpret_cast<unsigned*>(d_queue);
+  d_alive = d_del + NC;
   cudaMemsetAsync(d_flags, 0, sizeof(unsigned), s);
   cudaMemsetAsync(d_stats, 0, sizeof(unsigned long long) * 5, s);
   cudaMemsetAsync(d_hist, 0, sizeof(unsigned long long) * 45, s);
@@ -688,7 +722,7 @@ extern "C" int mrsph_triangulate(mrsph_handle* h, int* tris, long long cap, long
     TriIn T;
     T.n = n; T.cap = rowcap; T.xyz = d_xyz; T.type = d_type; T.phi = d_phi; T.rows = d_rows; T.cnt = d_cnt;
     T.deg = d_deg; T.adj = d_adj;
-    const int nbE = (int)((NC + 255) / 256), nbN = (int)((n + 255) / 256);
+    const int nbE = (int)((NC + 255) / 256), nbN = (int)((n * kTG + 255) / 256);
     if (wpb > 0) {
       const size_t sm = wpb * mark_smem(rowcap);
       cudaFuncSetAttribute(k_tri_mark, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMarkSmem);
@@ -699,8 +733,8 @@ extern "C" int mrsph_triangulate(mrsph_handle* h, int* tris, long long cap, long
     k_tri_mark_exact<<<XB, XT, 0, s>>>(T, d_mark, d_queue, d_stats + 4, d_flags, d_scratch);
     k_tri_adj<<<(unsigned)((n + 7) / 8), 256, 0, s>>>(T, d_mark, d_del, d_alive);
     k_tri_pass1<<<nbN, 256, 0, s>>>(T, h->ls, d_del);
-    k_tri_alive<<<nbN, 256, 0, s>>>(T, h->ls, d_del, d_alive);
-    k_tri_count_first<<<nbN, 256, 0, s>>>(T, d_del, d_stats);
+    k_tri_alive<<<nbN, 256, 0, s>>>(T, d_del, d_alive);
+    k_tri_mirror<<<nbN, 256, 0, s>>>(T, d_del, d_alive, d_stats);
     k_tri_pass2<false><<<nbN, 256, 0, s>>>(T, d_alive, d_count, nullptr, nullptr, d_stats);
     cell_scan(d_count, d_off, d_blk, n, 0, s);
     int tot = 0;
@@ -716,13 +750,13 @@ extern "C" int mrsph_triangulate(mrsph_handle* h, int* tris, long long cap, long
     if (flags & 4u) { rc = tfail(h, MRSPH_ERR_RANGE, "neighbour list spilled; raise neighbor_cap"); goto done; }
     if (flags) { rc = tfail(h, MRSPH_ERR_DEVICE, "exact predicate accumulator overflow"); goto done; }
     if (ntri > 0) {
-      if (!A((void**)&d_tris, sizeof(int) * 3 * ntri)) { rc = tfail(h, MRSPH_ERR_OOM, "cudaMalloc failed"); goto done; }
-      k_tri_pass2<true><<<nbN, 256, 0, s>>>(T, d_alive, nullptr, d_off, d_tris, nullptr);
       const int nbT = (int)((ntri + 255) / 256);
-      if (!A((void**)&d_part, sizeof(TriStat) * nbT) || !A((void**)&d_tq, sizeof(TriStat))) {
+      if (!A({{(void**)&d_tris, sizeof(int) * 3 * ntri}, {(void**)&d_part, sizeof(TriStat) * nbT},
+              {(void**)&d_tq, sizeof(TriStat)}})) {
         rc = tfail(h, MRSPH_ERR_OOM, "cudaMalloc failed");
         goto done;
       }
+      k_tri_pass2<true><<<nbN, 256, 0, s>>>(T, d_alive, nullptr, d_off, d_tris, nullptr);
       k_tri_quality<<<nbT, 256, 0, s>>>(d_xyz, ntri, d_tris, d_part, d_hist);
       k_tri_quality_fold<<<1, 256, 0, s>>>(d_part, nbT, d_tq);
       cudaMemcpyAsync(&tq, d_tq, sizeof(TriStat), cudaMemcpyDeviceToHost, s);
