@@ -624,9 +624,12 @@ __global__ void __launch_bounds__(128) k_vm_walk(const int* __restrict__ item_ce
 // full, E empty, P leaves of positive and N of negative corner sum a column
 // counts 4 F + 3 (P - F) + (N - E) + 2 (64 - P - N) = F - E + P - N + 128, so
 // it costs one root per line and one for the sum instead of a visit of the
-// 8^6 tree's cut nodes (some 12,000 per sub-cube): 8.7 ms for the 517,000 cut
-// sub-cubes of the benchmark torus, where visiting the tree breadth-first by
-// one warp each took 46.2 ms.  Both are bound by FP32 and integer issue.  In
+// 8^6 tree's cut nodes (some 12,000 per sub-cube).  Rows of columns are taken
+// along the axis of the largest mean slope, and a row whose eight corners have
+// one sign is counted as a whole: on average more than half of the rows.  The
+// 517,000 cut sub-cubes of the benchmark torus take 4.9 ms, 8.7 with every row and
+// 46.2 when one warp each visited the tree breadth-first; FP32 and integer
+// issue bound all three.  In
 // 2D a sub-square has 64 columns only and the walk (k_vm_walk) stays.
 //
 // Signs are those of the reference's FP64 refinement.  With M the largest
@@ -691,12 +694,29 @@ __global__ void __launch_bounds__(32 * kVmWarps) k_vm_columns(const int* __restr
                                                               const double* __restrict__ item_cor, long long nitem,
                                                               unsigned* __restrict__ units) {
   constexpr unsigned FULL = 0xffffffffu;
-  __shared__ double s_cor[kVmWarps][8];
+  __shared__ double s_org[kVmWarps][8], s_cor[kVmWarps][8];
   const int wid = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const long long it = (long long)blockIdx.x * kVmWarps + wid;
   if (it >= nitem) return;  // whole warps
-  double* cor = s_cor[wid];
-  if (lane < 8) cor[lane] = item_cor[it * 8 + lane];  // [x][y][z]
+  double *org = s_org[wid], *cor = s_cor[wid];  // corners [x][y][z], as given and with the rows' axis as y
+  if (lane < 8) org[lane] = item_cor[it * 8 + lane];
+  __syncwarp();
+  int axis = 1;  // the axis of the largest mean slope becomes y
+  {
+    float sx = 0.f, sy = 0.f, sz = 0.f;
+    for (int q = 0; q < 8; q++) {
+      const float v = (float)org[q];
+      sx += (q & 4) ? v : -v;
+      sy += (q & 2) ? v : -v;
+      sz += (q & 1) ? v : -v;
+    }
+    if (fabsf(sx) > fabsf(sy) && fabsf(sx) >= fabsf(sz)) axis = 0;
+    else if (fabsf(sz) > fabsf(sy)) axis = 2;
+  }
+  if (lane < 8) {
+    const int x = lane >> 2, y = (lane >> 1) & 1, z = lane & 1;
+    cor[lane] = org[axis == 0 ? y * 4 + x * 2 + z : (axis == 2 ? x * 4 + z * 2 + y : lane)];
+  }
   __syncwarp();
   float c[8], M = 0.f;
   for (int q = 0; q < 8; q++) {
@@ -718,10 +738,36 @@ __global__ void __launch_bounds__(32 * kVmWarps) k_vm_columns(const int* __restr
     b0[i] = v00; d0[i] = v10 - v00;
     b1[i] = v01; d1[i] = v11 - v01;
   }
+  // Rows (leaves y to y + 1) whose corners have one sign beyond the band hold only
+  // leaves of that sign; lane l tests rows 2l and 2l + 1.
+  int acc = 0;
+  unsigned mixed[2], row_full = 0;
+  for (int i = 0; i < 2; i++) {
+    bool full = true, empty = true;
+    for (int f = 0; f < 2; f++) {
+      const float ty = (float)(2 * lane + i + f) * 0x1p-6f;
+      for (int q = 0; q < 4; q++) {
+        const int u = (q & 2) * 2 + (q & 1);  // x, z
+        const float v = fmaf(ty, c[u + 2] - c[u], c[u]);
+        full = full && v > th;
+        empty = empty && v < -th;
+      }
+    }
+    mixed[i] = __ballot_sync(FULL, !full && !empty);
+    if (full) row_full |= 1 << i;
+  }
+  const unsigned any = mixed[0] | mixed[1];
+  int y0 = 0, y1 = -1;  // the rows between the first and the last mixed one
+  if (any) {
+    const int l0 = __ffs(any) - 1, l1 = 31 - __clz(any);
+    y0 = 2 * l0 + ((mixed[0] >> l0) & 1 ? 0 : 1);
+    y1 = 2 * l1 + ((mixed[1] >> l1) & 1 ? 1 : 0);
+  }
+  for (int i = 0; i < 2; i++)
+    if (((row_full >> i) & 1) && (2 * lane + i < y0 || 2 * lane + i > y1)) acc += 256 * 64;
   VmLine prev[3];
   unsigned prev_bad = 0;  // bit i: line i of the previous row is not decided
-  int acc = 0;
-  for (int y = 0; y <= 64; y++) {
+  for (int y = y0; y <= y1 + 1; y++) {
     const float ty = (float)y * 0x1p-6f;
     VmLine cur[3];
     unsigned bad = 0;
@@ -749,7 +795,7 @@ __global__ void __launch_bounds__(32 * kVmWarps) k_vm_columns(const int* __restr
       cur[i].P = pos ? w0 : w1;
       cur[i].N = pos ? w1 : w0;
     }
-    if (y > 0) {
+    if (y > y0) {
       bool exact[2];
 #pragma unroll
       for (int i = 0; i < 2; i++) {
@@ -789,11 +835,12 @@ __global__ void __launch_bounds__(32 * kVmWarps) k_vm_columns(const int* __restr
           const int x = 2 * (__ffs(todo) - 1) + i, yy = y - 1;
           todo &= todo - 1u;
           for (int k = lane; k < 64; k += 32) {
+            const int ox = axis == 0 ? yy : x, oy = axis == 0 ? x : (axis == 2 ? k : yy), oz = axis == 2 ? yy : k;
             int path[6];
             for (int l = 0; l < 6; l++)
-              path[l] = (((x >> (5 - l)) & 1) << 2) | (((yy >> (5 - l)) & 1) << 1) | ((k >> (5 - l)) & 1);
+              path[l] = (((ox >> (5 - l)) & 1) << 2) | (((oy >> (5 - l)) & 1) << 1) | ((oz >> (5 - l)) & 1);
             double leaf[8];
-            gc_path64<3>(cor, path, 6, leaf);
+            gc_path64<3>(org, path, 6, leaf);
             const int f = gc_mark(leaf, 8);
             double cv = 0.0;
             for (int q = 0; q < 8; q++) cv += leaf[q];
