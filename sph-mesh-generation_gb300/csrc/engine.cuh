@@ -1731,7 +1731,7 @@ __device__ inline void force_particle(const KCtx& c, const Buf<R>& b, const Work
   // kernel-sum term of a pair at distance r in dim dimensions
   auto W = [&](int dim, R r) -> R {
     if constexpr (F32) return kernel_W_fast(kind, dim, (float)r, (float)inv_h);
-    else return dim == D ? kernel_W_C<R>(kind, dim, r, h, CW) : kernel_W<R>(kind, dim, r, h);
+    else return dim == D ? kernel_W_C<R>(kind, dim, quot(r, h, inv_h), CW) : kernel_W<R>(kind, dim, r, h);
   };
   // pair (i, j): the skip rules of :717-759, :904-920 and :1019-1031; its
   // kernel-sum term wt (true when it counts), and the pair coefficient cij and
@@ -1876,17 +1876,27 @@ __device__ inline void force_particle(const KCtx& c, const Buf<R>& b, const Work
           ncount += __popc(g.ballot(counts));
         }
         __syncwarp(g.mask);
-        if (STAGE > 0 && g.gl < D) {
-          const R* v = gt->term[g.gl];
-          for (int k = 0; k < 4; k++) accum(0, v[k]);
-          flush(0);
-          if (q0 + 4 < cnt) {
-            for (int k = 4; k < kG; k++) accum(0, v[k]);
-            flush(0);
+        if constexpr (!F32 && STAGE == 1) {  // plain sums of all four components at once
+          if (g.gl < 4) {
+            const R* v = gt->term[g.gl];
+            R acc = g.gl == 3 ? sum : F[0];
+            for (int k = 0; k < kG; k++) acc = acc + v[k];
+            if (g.gl == 3) sum = acc;
+            else F[0] = acc;
           }
+        } else {
+          if (STAGE > 0 && g.gl < D) {
+            const R* v = gt->term[g.gl];
+            for (int k = 0; k < 4; k++) accum(0, v[k]);
+            flush(0);
+            if (q0 + 4 < cnt) {
+              for (int k = 4; k < kG; k++) accum(0, v[k]);
+              flush(0);
+            }
+          }
+          if (STAGE < 2 && g.gl == 3)
+            for (int k = 0; k < kG; k++) sum = radd(sum, gt->term[3][k]);
         }
-        if (STAGE < 2 && g.gl == 3)
-          for (int k = 0; k < kG; k++) sum = radd(sum, gt->term[3][k]);
         __syncwarp(g.mask);
       };
       if constexpr (!SPILL) {
