@@ -945,7 +945,7 @@ __device__ inline void level_position(const KCtx& c, int L, const SOrigin<D, flo
 template <int D>
 __device__ inline void level_box(const KCtx& c, int L, float R, const int* q, const float* fr, int* lo, int* up) {
   for (int d = 0; d < D; d++) {
-    const float rr = R / c.geo.hs_f[L][d];
+    const float rr = R * c.geo.ihs_f[L][d];
     lo[d] = max(q[d] + (int)floorf(fr[d] - rr), 0);
     up[d] = min(q[d] + (int)floorf(fr[d] + rr), c.geo.hn[L][d] - 1);
   }
@@ -970,7 +970,7 @@ __device__ inline bool row_range(const KCtx& c, const int* __restrict__ cstart, 
   gy *= c.geo.hs_f[L][1];
   const float rem = R * R - gy * gy - gz * gz;
   if (rem < 0.f) return false;
-  const float w = sqrtf(rem) / c.geo.hs_f[L][0];
+  const float w = sqrtf(rem) * c.geo.ihs_f[L][0];
   const int xl = max(q[0] + (int)floorf(fr[0] - w), 0);
   const int xh = min(q[0] + (int)floorf(fr[0] + w), hn[0] - 1);
   if (xl > xh) return false;
