@@ -4,8 +4,8 @@
 // reference's operation order) and mrsph_fp32.cu.
 //
 // One step (SPH_mesh_generation::SPH_run_mesh_generation,
-// sph_mesh_generation.cpp:1371-1463) is 11 launches on one stream (15 for a
-// large FP32-split handle), replayed as a CUDA graph:
+// sph_mesh_generation.cpp:1371-1463) is 11 launches on one stream (9 for a
+// small handle, 15 for a large FP32-split one in 3D), replayed as a CUDA graph:
 //   k_begin_step   scalars of the step
 //   k_map          A1 advect + A2 sample + A3 surface map/re-seed + A4 spacing
 //                  + scale/level refresh + cell key + cell histogram
@@ -13,7 +13,7 @@
 //   k_reorder      rank inside the cell, gather of the persistent state into the
 //                  sorted order, search radii
 //   k_brick_*      the work order of a large handle's list builder
-//   k_density(_group)  A6 neighbour search over the cell table: the neighbour lists
+//   k_density(_group, _lane)  A6 neighbour search over the cell table: the neighbour lists
 //   k_force<1>     A7 kernel sum + A8 stage 1 + A9 dt/max|v| grid reduction (FP64
 //                  bit atomics), k_force_spill for particles whose list spilled
 //   k_force<2>     A8 stage 2 + A9 + A10 (stage-1 kick folded in; the stage-2
@@ -138,14 +138,18 @@ struct BatchSlot {
 enum { MAP_STEP = 0, MAP_PRE = 1 };
 
 // Particles up to which a handle's own neighbour passes take kG lanes per
-// particle (force_particle, list_group) instead of one lane of a full warp
-// (force_particle, list_warp).  Below these counts the chip is not full and a
-// particle's chain of gathers bounds the kernel, above them the instructions do.
-// Measured, group against lane: stage 1 of 20,000 particles in 3D 37 against 67
-// us, of 77,551 in 2D 39 against 26; lists of 77,551 in 2D 71 against 135 us, of
-// 301,270 in 3D (uniform positions, 281 neighbours) 2.12 against 1.16 ms.
+// particle (force_particle, list_group).  Below these counts the chip is not
+// full and a particle's chain of gathers bounds the kernel, above them the
+// instructions do.  Larger handles take one lane per particle in the force
+// passes, and in the FP32-split lists one lane in 2D (list_lane: short rows,
+// about 60 candidates) and a shared tile per warp in 3D (list_warp).  Measured, us:
+// stage 1 of 20,000 in 3D 37 by groups, 67 by lanes, of 77,551 in 2D 39 and 26;
+// lists in 2D of 77,551 70 by groups, 95 by lanes, 127 by warp tiles, of 150,000
+// 73, 42 and 74; in 3D of 60,000 250 by groups and 440 by tiles, of 100,000 366
+// and 461 (two levels) or 806 and 711 (281 neighbours), of 130,000 483 and 426,
+// of 200,000 258 and 216 (by lanes 347).
 constexpr long long kGroupMax = 40960;
-constexpr long long kListGroupMax = 131072;
+constexpr long long kListGroupMax2 = 98304, kListGroupMax3 = 114688;
 
 // Tuning of the FP32 map and neighbour passes: resident blocks per SM the
 // register allocation must allow (density: of kDensityThreads threads, else 256).
@@ -1189,6 +1193,23 @@ template <int D> struct PairTest<D, float> {
     if (d2 > Rm * kD2Accept) return false;
     return d2 < Rm * kD2Sure || exact_neighbor<D>(c, a0, a1, b0, b1);
   }
+  // in FP32 alone: accepts the band, and notes in close that a pair lies in it
+  __device__ bool near32(const KCtx& c, const float4& b0, const float4& b1, bool& close) const {
+    float dr[3];
+    RecOps<D, float>::rel(c, a0, a1, b0, b1, dr);
+    const float d2 = d2_of(dr, D);
+    const float rj = b0.w * cut;
+    const float Rm = fmaxf(R2i, rj * rj);
+    if (d2 > Rm * kD2Accept) return false;
+    close = close || !(d2 < Rm * kD2Sure);
+    return true;
+  }
+  template <class LD>
+  __device__ bool near32(const KCtx& c, const float4* rec, int j, bool& close) const {
+    float4 b0, b1;
+    LD::rec(rec, j, b0, b1);
+    return near32(c, b0, b1, close);
+  }
 };
 template <int D>
 __device__ __noinline__ bool exact_neighbor64(const KCtx& c, const double4* rec, long long i, int j) {
@@ -1220,21 +1241,34 @@ template <int D> struct PairTest<D, double> {
 // Neighbour list of particle i by its group of kG lanes, in the fixed scan
 // order.  Returns the number of neighbours (itself included); the list keeps the
 // first cap.
-template <int D, class R, class LD>
+// FP32-split decides in FP32; when a pair lies in the criterion's band it returns
+// -1 and the list is taken again with the whole test (EXACT), whose FP64 path the
+// hot loop has no registers for.
+template <int D, class R, bool EXACT, class LD>
 __device__ inline int list_group(const KCtx& c, const Buf<R>& b, const Work<R>& w, const GroupLanes& g, RowTile& rt,
                                  long long i) {
   const PairTest<D, R> pt(c, b.rec, i);
   const SOrigin<D, R> so(c, b.posh[i], b.key ? b.key[i] : 0);
   int* row = w.nbl + nb_slot(i, 0, w.cap);  // entry q at row[(q >> 3) * 256 + (q & 7)]
   int cnt = 0;
+  bool close = false;
   group_scan<D, R, LD>(c, w, g, rt, i, so, [&](int j, bool in) {
-    const bool ok = in && pt.template near<LD>(c, b.rec, j);
+    bool ok;
+    if constexpr (EXACT) ok = in && pt.template near<LD>(c, b.rec, j);
+    else ok = in && pt.template near32<LD>(c, b.rec, j, close);
     const unsigned m = g.ballot(ok);
     const int pos = cnt + __popc(m & g.below);
     if (ok && pos < w.cap) row[((pos >> 3) << 8) + (pos & 7)] = j;
     cnt += __popc(m);
   });
+  if constexpr (!EXACT)
+    if (g.ballot(close)) return -1;
   return cnt;
+}
+template <int D, class LD>
+__device__ __noinline__ int list_group_exact(const KCtx& c, const Buf<float>& b, const Work<float>& w,
+                                             const GroupLanes& g, RowTile& rt, long long i) {
+  return list_group<D, float, true, LD>(c, b, w, g, rt, i);
 }
 
 // Neighbour lists of 32 particles by one warp (FP32-split), lane l's particle i.
@@ -1553,6 +1587,54 @@ __device__ inline int list_warp(const KCtx& c, const Buf<float>& b, const Work<f
   return cnt;
 }
 
+// Neighbour list of particle i by one lane (FP32-split), its rows one after the
+// other, two candidates in flight.  EXACT = false decides in FP32 and returns -1
+// when a pair lies in the criterion's band; the list is then taken again with
+// the whole test, which the hot loop has no registers for.
+template <int D, bool EXACT, class LD>
+__device__ inline int list_lane(const KCtx& c, const Buf<float>& b, const Work<float>& w, long long i) {
+  const PairTest<D, float> pt(c, b.rec, i);
+  const SOrigin<D, float> so(c, b.posh[i], b.key[i]);
+  const int cap = w.cap;
+  int* row = w.nbl + nb_slot(i, 0, cap);  // entry q at row[(q >> 3) * 256 + (q & 7)]
+  int cnt = 0;
+  bool close = false;
+  auto take = [&](int j) {
+    if (cnt < cap) row[((cnt >> 3) << 8) + (cnt & 7)] = j;
+    cnt++;
+  };
+  for (int L = 0; L < c.geo.ncl; L++) {
+    const float R_ = LD::ld(&w.rlev[(long long)L * c.n + i]);
+    if (!(R_ > 0.f)) continue;
+    int q[3] = {0, 0, 0}, lo[3] = {0, 0, 0}, up[3] = {0, 0, 0};
+    float fr[3] = {0.f, 0.f, 0.f};
+    level_position<D>(c, L, so, q, fr);
+    level_box<D>(c, L, R_, q, fr, lo, up);
+    for (int z = lo[2]; z <= up[2]; z++)
+      for (int y = lo[1]; y <= up[1]; y++) {
+        int s0, e0;
+        if (!row_range<D, LD>(c, w.cstart, L, R_, q, fr, z, y, s0, e0)) continue;
+        if constexpr (EXACT) {
+          for (int j = s0; j < e0; j++)
+            if (pt.template near<LD>(c, b.rec, j)) take(j);
+        } else {
+          for (int j = s0; j < e0; j += 2) {
+            float4 b0, b1, c0, c1;
+            LD::rec(b.rec, j, b0, b1);
+            LD::rec(b.rec, min(j + 1, e0 - 1), c0, c1);
+            if (pt.near32(c, b0, b1, close)) take(j);
+            if (j + 1 < e0 && pt.near32(c, c0, c1, close)) take(j + 1);
+          }
+        }
+      }
+  }
+  return close ? -1 : cnt;
+}
+template <int D, class LD>
+__device__ __noinline__ int list_lane_exact(const KCtx& c, const Buf<float>& b, const Work<float>& w, long long i) {
+  return list_lane<D, true, LD>(c, b, w, i);
+}
+
 // what follows a list: its length, the spill queue, the step's totals
 template <int D, class R>
 __device__ inline void list_done(const KCtx& c, const Work<R>& w, long long i, int cnt, bool lead) {
@@ -1576,7 +1658,14 @@ __device__ inline void density_group_block(const KCtx& c, const Buf<R>& b, const
   const GroupLanes g;
   const long long i = first + threadIdx.x / kG;
   int cnt = 0;
-  if (i < c.n) cnt = list_group<D, R, LD>(c, b, w, g, tiles[threadIdx.x / kG], i);
+  if (i < c.n) {
+    if constexpr (std::is_same<R, float>::value) {
+      cnt = list_group<D, R, false, LD>(c, b, w, g, tiles[threadIdx.x / kG], i);
+      if (cnt < 0) cnt = list_group_exact<D, LD>(c, b, w, g, tiles[threadIdx.x / kG], i);
+    } else {
+      cnt = list_group<D, R, true, LD>(c, b, w, g, tiles[threadIdx.x / kG], i);
+    }
+  }
   __syncwarp();
   list_done<D, R>(c, w, i, cnt, i < c.n && g.gl == 0);
 }
@@ -1593,6 +1682,15 @@ __device__ inline void density_warp_block(const KCtx& c, const Buf<float>& b, co
 }
 
 constexpr int kDensityThreads = 128;
+template <int D>
+__global__ void __launch_bounds__(kDensityThreads, 8) k_density_lane(KCtx c, Buf<float> b, Work<float> w) {
+  chain_wait();
+  const long long i = (long long)blockIdx.x * kDensityThreads + threadIdx.x;
+  int cnt = i < c.n ? list_lane<D, false, LdNC>(c, b, w, i) : 0;
+  if (cnt < 0) cnt = list_lane_exact<D, LdNC>(c, b, w, i);
+  __syncwarp();
+  list_done<D, float>(c, w, i, cnt, i < c.n);
+}
 template <int D, class R>
 __global__ void __launch_bounds__(kDensityThreads, 10) k_density_group(KCtx c, Buf<R> b, Work<R> w) {
   chain_wait();
@@ -2007,15 +2105,7 @@ __global__ void __launch_bounds__(256, (std::is_same<R, float>::value ? (STAGE =
 }
 
 constexpr int kGroupThreads = 128;
-template <int D, class R, int STAGE, int KK>
-__global__ void __launch_bounds__(kGroupThreads, std::is_same<R, float>::value ? 8 : 1) k_force_group(KCtx c, Buf<R> b, Work<R> w) {
-  chain_wait();
-  __shared__ GroupTile<R> gt[kGroupThreads / kG];
-  if (STAGE < 2 && blockIdx.x == 0 && threadIdx.x == 0) accum_pairs_body(c.sc);
-  force_block<D, R, STAGE, KK, kG>(c, b, w, gt, (long long)blockIdx.x * (kGroupThreads / kG));
-}
-
-// The force stage of the particles whose list spilled (queued by the density
+// The force stage of the particles whose list spilled (queued by the list
 // pass; grid-stride over groups), re-scanning their cells.
 template <int D, class R, int STAGE, int KK, class LD = LdNC>
 __device__ inline void force_spill_items(const KCtx& c, const Buf<R>& b, const Work<R>& w, GroupTile<R>* gt,
@@ -2031,6 +2121,19 @@ __device__ inline void force_spill_items(const KCtx& c, const Buf<R>& b, const W
   }
   __syncwarp();
   force_reduce<STAGE>(c, my_dt, my_v);
+}
+
+// A small handle's force stage, listed and spilled particles in one launch: the
+// first nq blocks take the spill queue (they leave at once when it is empty, as it
+// nearly always is), the others the listed particles.  A launch of its own for
+// the queue took 2.5 us beside the stage's 10.5 for 8,745 particles in 2D.
+template <int D, class R, int STAGE, int KK>
+__global__ void __launch_bounds__(kGroupThreads, std::is_same<R, float>::value ? 8 : 1) k_force_group(KCtx c, Buf<R> b, Work<R> w, int nq) {
+  chain_wait();
+  __shared__ GroupTile<R> gt[kGroupThreads / kG];
+  if (STAGE < 2 && blockIdx.x == 0 && threadIdx.x == 0) accum_pairs_body(c.sc);
+  if ((int)blockIdx.x < nq) force_spill_items<D, R, STAGE, KK>(c, b, w, gt, blockIdx.x, nq);
+  else force_block<D, R, STAGE, KK, kG>(c, b, w, gt, (long long)(blockIdx.x - nq) * (kGroupThreads / kG));
 }
 
 template <int D, class R, int STAGE, int KK>
@@ -2367,6 +2470,13 @@ class Engine : public EngineBase {
     w_.pc = pc;
     w_.cap = (int)want;
     drop_graphs();
+    // the lists of the state they belong to, now whole: whoever reads them next
+    // (taps, meshes) finds them in the new arrays
+    MR_CK(cudaMemsetAsync(&kc_.sc->pairs, 0, sizeof(kc_.sc->pairs), st_));
+    MR_CK(cudaMemsetAsync(&kc_.sc->nspill, 0, sizeof(kc_.sc->nspill), st_));
+    launch_lists();
+    MR_CK(cudaGetLastError());
+    MR_CK(cudaStreamSynchronize(st_));  // a batch steps the handle on another stream
     return 0;
   }
 
@@ -2534,7 +2644,7 @@ class Engine : public EngineBase {
   int sample(long long n, const double* xyz, double* phi, double* norm, double* curv, int* tag) override {
     // xyz, then the results as the caller's arrays want them: phi, normals, curvature, tags
     double* d = nullptr;
-    MR_CK(cudaMallocAsync(&d, (sizeof(double) * 8 + sizeof(int)) * n, st_));
+    MR_CK(cudaMalloc(&d, (sizeof(double) * 8 + sizeof(int)) * n));
     double *dphi = d + 3 * n, *dnorm = d + 4 * n, *dcurv = d + 7 * n;
     int* dtag = reinterpret_cast<int*>(d + 8 * n);
     cudaError_t e = cudaMemcpyAsync(d, xyz, sizeof(double) * 3 * n, cudaMemcpyHostToDevice, st_);
@@ -2549,8 +2659,8 @@ class Engine : public EngineBase {
     out(norm, dnorm, sizeof(double) * 3 * n);
     out(curv, dcurv, sizeof(double) * n);
     out(tag, dtag, sizeof(int) * n);
-    cudaFreeAsync(d, st_);
     if (e == cudaSuccess) e = cudaStreamSynchronize(st_);
+    cudaFree(d);
     if (e != cudaSuccess) { err = cudaGetErrorString(e); return MRSPH_ERR_CUDA; }
     return 0;
   }
@@ -2658,24 +2768,32 @@ class Engine : public EngineBase {
 
   void launch_lists() {
     const long long n = n_;
-    bool grouped = true;
     if constexpr (std::is_same<R, float>::value) {
-      if (n > kListGroupMax) {
+      if (D == 2 && n > kListGroupMax2) {
+        launch_chained(k_density_lane<D>, (unsigned)((n + kDensityThreads - 1) / kDensityThreads), kDensityThreads, st_, kc_, buf_[cur_], w_);
+        return;
+      }
+    }
+    if constexpr (D == 3 && std::is_same<R, float>::value) {
+      if (n > kListGroupMax3) {
         const long long nb = kc_.geo.boff[kc_.geo.ncl];
         launch_chained(k_brick_count<D>, grid(nb), 256, st_, kc_, w_.cstart, w_.bcount);
         cell_scan(w_.bcount, w_.bstart, w_.blocksums, nb, (int)n, st_);
         launch_chained(k_brick_order<D>, grid(nb), 256, st_, kc_, w_.cstart, w_.bcount, w_.bstart, w_.order);
         launch_chained(k_density<D>, (unsigned)((n + kDensityThreads - 1) / kDensityThreads), kDensityThreads, st_, kc_, buf_[cur_], w_);
-        grouped = false;
+        return;
       }
     }
-    if (grouped) launch_chained(k_density_group<D, R>, ggrid(kDensityThreads), kDensityThreads, st_, kc_, buf_[cur_], w_);
+    launch_chained(k_density_group<D, R>, ggrid(kDensityThreads), kDensityThreads, st_, kc_, buf_[cur_], w_);
   }
 
   template <int STAGE, int KK>
   void launch_force_kind() {
-    if (n_ <= kGroupMax) launch_chained(k_force_group<D, R, STAGE, KK>, ggrid(kGroupThreads), kGroupThreads, st_, kc_, buf_[cur_], w_);
-    else launch_chained(k_force<D, R, STAGE, KK>, grid(n_), 256, st_, kc_, buf_[cur_], w_);
+    if (n_ <= kGroupMax) {
+      launch_chained(k_force_group<D, R, STAGE, KK>, ggrid(kGroupThreads) + qgrid(), kGroupThreads, st_, kc_, buf_[cur_], w_, qgrid());
+      return;
+    }
+    launch_chained(k_force<D, R, STAGE, KK>, grid(n_), 256, st_, kc_, buf_[cur_], w_);
     launch_chained(k_force_spill<D, R, STAGE, KK>, qgrid(), kGroupThreads, st_, kc_, buf_[cur_], w_);
   }
   template <int STAGE>
@@ -2710,14 +2828,8 @@ class Engine : public EngineBase {
     if (phase < MRSPH_PHASE_DENSITY) return 0;
     launch_lists();
     if (settle) {
-      const int cap = w_.cap;
       int rc = maybe_grow_cap();
       if (rc) return rc;
-      if (w_.cap != cap) {  // the same lists again, now whole
-        MR_CK(cudaMemsetAsync(&kc_.sc->pairs, 0, sizeof(kc_.sc->pairs), st_));
-        MR_CK(cudaMemsetAsync(&kc_.sc->nspill, 0, sizeof(kc_.sc->nspill), st_));
-        launch_lists();
-      }
     }
     have_work_ = true;
     mark(5);
@@ -2872,7 +2984,7 @@ class Engine : public EngineBase {
       rc |= A((void**)&kc_.sc, sizeof(DevScalars));
     }
     w_.bcount = w_.bstart = w_.order = nullptr;
-    if (!rc && std::is_same<R, float>::value && n > kListGroupMax) {
+    if (!rc && D == 3 && std::is_same<R, float>::value && n > kListGroupMax3) {
       const long long nb = kc_.geo.boff[kc_.geo.ncl];
       rc |= A((void**)&w_.bcount, sizeof(int) * nb);
       rc |= A((void**)&w_.bstart, sizeof(int) * (nb + 1));

@@ -364,12 +364,12 @@ int mrsph_get_levelset(mrsph_handle* h, int level, double* nx, double* ny, doubl
     // half of the call)
     double* const out[3] = {nx, ny, nz};
     double* d = nullptr;
-    if (cudaMallocAsync(&d, 3 * sizeof(double) * ntot, h->stream) == cudaSuccess) {
+    if (cudaMalloc(&d, 3 * sizeof(double) * ntot) == cudaSuccess) {
       cudaError_t e = ls_split_normals(ntot, L.g64, d, h->stream);
       for (int k = 0; k < 3 && e == cudaSuccess; k++)
         if (out[k]) e = cudaMemcpyAsync(out[k], d + k * ntot, sizeof(double) * ntot, cudaMemcpyDeviceToHost, h->stream);
-      cudaFreeAsync(d, h->stream);
       if (e == cudaSuccess) e = cudaStreamSynchronize(h->stream);
+      cudaFree(d);
       API_CK(h, e);
     } else {  // no room on the device: through the host
       cudaGetLastError();

@@ -1,6 +1,6 @@
 """The neighbour passes on both sides of their dispatch lines (particles per
 handle up to which a group of lanes takes one particle: 40,960 in the force
-passes, 131,072 in the list builder) and the cell scan with more than 2048
+passes, 98,304 in 2D and 114,688 in 3D in the list builder) and the cell scan with more than 2048
 blocks: one step against the oracle, and a handle alone against the persistent
 batch kernel, which has one form for every size."""
 import numpy as np
@@ -13,7 +13,7 @@ from test_gpu_parity import _gpu_step_taps, check_fp32_single_step
 
 pytestmark = pytest.mark.gpu
 
-EDGES = [40960, 40961, 131072, 131073]
+EDGES = [40960, 40961, 98304, 98305, 114688, 114689]
 
 
 def sized_star(dim, n, n_target=None):
