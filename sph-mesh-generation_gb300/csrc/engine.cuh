@@ -4,8 +4,8 @@
 // reference's operation order) and mrsph_fp32.cu.
 //
 // One step (SPH_mesh_generation::SPH_run_mesh_generation,
-// sph_mesh_generation.cpp:1371-1463) is 11 launches on one stream (9 for a
-// small handle, 15 for a large FP32-split one in 3D), replayed as a CUDA graph:
+// sph_mesh_generation.cpp:1371-1463) is 11 launches on one stream (15 for a
+// large FP32-split handle in 3D), replayed as a CUDA graph:
 //   k_begin_step   scalars of the step
 //   k_map          A1 advect + A2 sample + A3 surface map/re-seed + A4 spacing
 //                  + scale/level refresh + cell key + cell histogram
@@ -1204,12 +1204,6 @@ template <int D> struct PairTest<D, float> {
     close = close || !(d2 < Rm * kD2Sure);
     return true;
   }
-  template <class LD>
-  __device__ bool near32(const KCtx& c, const float4* rec, int j, bool& close) const {
-    float4 b0, b1;
-    LD::rec(rec, j, b0, b1);
-    return near32(c, b0, b1, close);
-  }
 };
 template <int D>
 __device__ __noinline__ bool exact_neighbor64(const KCtx& c, const double4* rec, long long i, int j) {
@@ -1241,34 +1235,21 @@ template <int D> struct PairTest<D, double> {
 // Neighbour list of particle i by its group of kG lanes, in the fixed scan
 // order.  Returns the number of neighbours (itself included); the list keeps the
 // first cap.
-// FP32-split decides in FP32; when a pair lies in the criterion's band it returns
-// -1 and the list is taken again with the whole test (EXACT), whose FP64 path the
-// hot loop has no registers for.
-template <int D, class R, bool EXACT, class LD>
+template <int D, class R, class LD>
 __device__ inline int list_group(const KCtx& c, const Buf<R>& b, const Work<R>& w, const GroupLanes& g, RowTile& rt,
                                  long long i) {
   const PairTest<D, R> pt(c, b.rec, i);
   const SOrigin<D, R> so(c, b.posh[i], b.key ? b.key[i] : 0);
   int* row = w.nbl + nb_slot(i, 0, w.cap);  // entry q at row[(q >> 3) * 256 + (q & 7)]
   int cnt = 0;
-  bool close = false;
   group_scan<D, R, LD>(c, w, g, rt, i, so, [&](int j, bool in) {
-    bool ok;
-    if constexpr (EXACT) ok = in && pt.template near<LD>(c, b.rec, j);
-    else ok = in && pt.template near32<LD>(c, b.rec, j, close);
+    const bool ok = in && pt.template near<LD>(c, b.rec, j);
     const unsigned m = g.ballot(ok);
     const int pos = cnt + __popc(m & g.below);
     if (ok && pos < w.cap) row[((pos >> 3) << 8) + (pos & 7)] = j;
     cnt += __popc(m);
   });
-  if constexpr (!EXACT)
-    if (g.ballot(close)) return -1;
   return cnt;
-}
-template <int D, class LD>
-__device__ __noinline__ int list_group_exact(const KCtx& c, const Buf<float>& b, const Work<float>& w,
-                                             const GroupLanes& g, RowTile& rt, long long i) {
-  return list_group<D, float, true, LD>(c, b, w, g, rt, i);
 }
 
 // Neighbour lists of 32 particles by one warp (FP32-split), lane l's particle i.
@@ -1658,14 +1639,7 @@ __device__ inline void density_group_block(const KCtx& c, const Buf<R>& b, const
   const GroupLanes g;
   const long long i = first + threadIdx.x / kG;
   int cnt = 0;
-  if (i < c.n) {
-    if constexpr (std::is_same<R, float>::value) {
-      cnt = list_group<D, R, false, LD>(c, b, w, g, tiles[threadIdx.x / kG], i);
-      if (cnt < 0) cnt = list_group_exact<D, LD>(c, b, w, g, tiles[threadIdx.x / kG], i);
-    } else {
-      cnt = list_group<D, R, true, LD>(c, b, w, g, tiles[threadIdx.x / kG], i);
-    }
-  }
+  if (i < c.n) cnt = list_group<D, R, LD>(c, b, w, g, tiles[threadIdx.x / kG], i);
   __syncwarp();
   list_done<D, R>(c, w, i, cnt, i < c.n && g.gl == 0);
 }
@@ -2123,17 +2097,12 @@ __device__ inline void force_spill_items(const KCtx& c, const Buf<R>& b, const W
   force_reduce<STAGE>(c, my_dt, my_v);
 }
 
-// A small handle's force stage, listed and spilled particles in one launch: the
-// first nq blocks take the spill queue (they leave at once when it is empty, as it
-// nearly always is), the others the listed particles.  A launch of its own for
-// the queue took 2.5 us beside the stage's 10.5 for 8,745 particles in 2D.
 template <int D, class R, int STAGE, int KK>
-__global__ void __launch_bounds__(kGroupThreads, std::is_same<R, float>::value ? 8 : 1) k_force_group(KCtx c, Buf<R> b, Work<R> w, int nq) {
+__global__ void __launch_bounds__(kGroupThreads, std::is_same<R, float>::value ? 8 : 1) k_force_group(KCtx c, Buf<R> b, Work<R> w) {
   chain_wait();
   __shared__ GroupTile<R> gt[kGroupThreads / kG];
   if (STAGE < 2 && blockIdx.x == 0 && threadIdx.x == 0) accum_pairs_body(c.sc);
-  if ((int)blockIdx.x < nq) force_spill_items<D, R, STAGE, KK>(c, b, w, gt, blockIdx.x, nq);
-  else force_block<D, R, STAGE, KK, kG>(c, b, w, gt, (long long)(blockIdx.x - nq) * (kGroupThreads / kG));
+  force_block<D, R, STAGE, KK, kG>(c, b, w, gt, (long long)blockIdx.x * (kGroupThreads / kG));
 }
 
 template <int D, class R, int STAGE, int KK>
@@ -2789,11 +2758,8 @@ class Engine : public EngineBase {
 
   template <int STAGE, int KK>
   void launch_force_kind() {
-    if (n_ <= kGroupMax) {
-      launch_chained(k_force_group<D, R, STAGE, KK>, ggrid(kGroupThreads) + qgrid(), kGroupThreads, st_, kc_, buf_[cur_], w_, qgrid());
-      return;
-    }
-    launch_chained(k_force<D, R, STAGE, KK>, grid(n_), 256, st_, kc_, buf_[cur_], w_);
+    if (n_ <= kGroupMax) launch_chained(k_force_group<D, R, STAGE, KK>, ggrid(kGroupThreads), kGroupThreads, st_, kc_, buf_[cur_], w_);
+    else launch_chained(k_force<D, R, STAGE, KK>, grid(n_), 256, st_, kc_, buf_[cur_], w_);
     launch_chained(k_force_spill<D, R, STAGE, KK>, qgrid(), kGroupThreads, st_, kc_, buf_[cur_], w_);
   }
   template <int STAGE>
