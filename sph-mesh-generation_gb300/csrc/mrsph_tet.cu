@@ -303,6 +303,10 @@ constexpr unsigned kFull = 0xffffffffu;
 // once, kept in shared memory for the whole star), with an error bound beside
 // every value: a decision is taken from FP32 only when it clears its bound, and
 // from the exact predicates otherwise, so every decision equals the exact one.
+// Lengths are taken in units of the power of two at the radius of i's ball: up
+// to six of them are multiplied, and in the body's own units a spacing of 3e-8
+// would already leave FP32's range.  Points far closer to one another than to
+// the ball's size can still do so: what has come below 1e-30 decides nothing.
 // FP64 runs at 1/60 of the FP32 rate on this part: with the candidates' FP64
 // differences, an FP64 circumcentre per tet and a second scan of the row per
 // tet the pass took 142.9 ms for 150,001 particles (830,000 tets); in this
@@ -331,11 +335,12 @@ struct StarRow {
   const int* S;  // the row's ids
   int i, m;
   Pt pi;
+  float sc;  // the unit of length, inverted
   const Star& sm;
   __device__ float4 make(int q) const {
     const int j = S[q];
     const Pt p = load_pt(T, j);
-    const float x = (float)(p.x - pi.x), y = (float)(p.y - pi.y), z = (float)(p.z - pi.z);
+    const float x = (float)(p.x - pi.x) * sc, y = (float)(p.y - pi.y) * sc, z = (float)(p.z - pi.z) * sc;
     return make_float4(j == i ? __int_as_float(0x7fffffff) : x, y, z, sqrtf(fmaf(z, z, fmaf(y, y, x * x))));
   }
   __device__ float4 at(int q) const { return q < kRowS ? sm.w[q] : make(q); }
@@ -347,6 +352,11 @@ __device__ inline int ford(float v) {
   const int b = __float_as_int(v);
   return b >= 0 ? b : b ^ 0x7fffffff;
 }
+// 2^-k for v in [2^k, 2^(k + 1)); 1 where FP32 has no such number
+__device__ inline float inv_pow2(float v) {
+  const int e = (__float_as_int(v) >> 23) & 0xff;
+  return e >= 1 && e <= 253 ? __int_as_float((254 - e) << 23) : 1.f;
+}
 __device__ inline float funord(int b) { return __int_as_float(b >= 0 ? b : b ^ 0x7fffffff); }
 
 struct Face {  // the pencil of spheres through i, u, v: centres c0 + sigma t n
@@ -356,7 +366,10 @@ struct Face {  // the pencil of spheres through i, u, v: centres c0 + sigma t n
 // Bounds, with e = 2^-24, k = |A||B| / |n| and L = |A| + |B|: n is off by at most
 // 4 e |A||B|, c0 by 22 e k^2 L (its formula's rounding 14, the rounding of A and
 // B 8), n . w by 8 e |A||B||w|, the power |w|^2 - 2 w . c0 by e (8 |w|^2 + 48 k^2 L |w|).
-// The constants below are at least a third larger.
+// The constants below are at least a third larger.  They are relative to the
+// products they bound, so a face whose products come near FP32's smallest numbers
+// has no bound.
+constexpr float kTiny = 1.e-30f;
 __device__ inline Face face_of(const float4& A4, const float4& B4, float sigma) {
   Face F;
   const V3 A{A4.x, A4.y, A4.z}, B{B4.x, B4.y, B4.z};
@@ -372,6 +385,7 @@ __device__ inline Face face_of(const float4& A4, const float4& B4, float sigma) 
   F.cO = 16.f * kE * ab;
   F.cP = 64.f * kE * k * k * F.L;
   F.dc0 = 32.f * kE * k * k * F.L;
+  if (!(n2 > kTiny) || !(fminf(A4.w, B4.w) > 1.e-12f)) F.cO = F.cP = F.dc0 = __int_as_float(0x7f800000);
   return F;
 }
 
@@ -553,9 +567,10 @@ __global__ void __launch_bounds__(32 * kStarWarps, 4) k_tet_star(TetIn T, int* _
   const long long nwarps = (long long)gridDim.x * kStarWarps;
   for (long long i64 = (long long)blockIdx.x * kStarWarps + wib; i64 < T.n; i64 += nwarps) {
     const int i = (int)i64;
-    const StarRow R{T, T.rows + i64 * T.cap, i, T.cnt[i], load_pt(T, i), sm};
+    const float sc = inv_pow2(T.rf[i]);
+    const StarRow R{T, T.rows + i64 * T.cap, i, T.cnt[i], load_pt(T, i), sc, sm};
     const int m = R.m;
-    const float Ri = T.rf[i];
+    const float Ri = T.rf[i] * sc;
     bool degen = false, open = false, trunc = false;
     int ns = 0, nl = 0;
     for (int q = lane; q < min(m, kRowS); q += 32) sm.w[q] = R.make(q);
@@ -602,11 +617,12 @@ __global__ void __launch_bounds__(32 * kStarWarps, 4) k_tet_star(TetIn T, int* _
         const V3 x = vcross(u3, v3);
         const float xx = vdot(x, x), dd = vdot(d3, d3), vv = w.w * w.w, uu = u4.w * u4.w;
         const float floor_ = 0.25f * fmaxf(vv, fmaxf(uu, dd)) * (1.f - 0x1p-16f);
-        const float r2 = uu * vv * dd / (4.f * xx), rel = 64.f * kE * u4.w * w.w / sqrtf(xx);
+        const float top = uu * vv * dd, r2 = top / (4.f * xx), rel = 64.f * kE * u4.w * w.w / sqrtf(xx);
         // |v - u| relative to its own rounding: d3 is off by at most 3 e (|u| + |v|)
         const float rd = 8.f * kE * (u4.w + w.w) / sqrtf(dd);
         const float er = rel + 2.f * rd;
-        if (!(er < 0.25f) || !(r2 < 3.e38f)) { lo = floor_; hi = INF; }
+        const bool tiny = !(xx > kTiny) || !(uu * vv > kTiny) || !(top > kTiny);
+        if (tiny || !(er < 0.25f) || !(r2 < 3.e38f) || !(xx < 3.e38f)) { lo = floor_; hi = INF; }
         else { lo = fmaxf(r2 * (1.f - 2.f * er), floor_); hi = r2 * (1.f + 2.f * er); }
         return true;
       };
@@ -764,7 +780,7 @@ __global__ void __launch_bounds__(32 * kStarWarps, 4) k_tet_star(TetIn T, int* _
         int owner = -1;
         bool sure = band < INF;
         for (int k = 0; k < 4 && owner < 0 && sure; k++) {
-          const float Rk = T.rf[v[k]];
+          const float Rk = T.rf[v[k]] * sc;
           if (v[k] == i || rc2 + band < Rk) owner = v[k];
           else if (!(rc2 - band > Rk)) sure = false;
         }
