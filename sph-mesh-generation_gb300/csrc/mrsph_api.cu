@@ -367,7 +367,7 @@ int mrsph_get_levelset(mrsph_handle* h, int level, double* nx, double* ny, doubl
     if (cudaMalloc(&d, 3 * sizeof(double) * ntot) == cudaSuccess) {
       cudaError_t e = ls_split_normals(ntot, L.g64, d, h->stream);
       for (int k = 0; k < 3 && e == cudaSuccess; k++)
-        if (out[k]) e = cudaMemcpyAsync(out[k], d + k * ntot, sizeof(double) * ntot, cudaMemcpyDeviceToHost, h->stream);
+        if (out[k]) e = copy_home(out[k], d + k * ntot, sizeof(double) * ntot, h->stream);
       if (e == cudaSuccess) e = cudaStreamSynchronize(h->stream);
       cudaFree(d);
       API_CK(h, e);
@@ -382,8 +382,9 @@ int mrsph_get_levelset(mrsph_handle* h, int level, double* nx, double* ny, doubl
       }
     }
   }
-  if (curv) API_CK(h, cudaMemcpy(curv, L.c64, sizeof(double) * ntot, cudaMemcpyDeviceToHost));
-  if (tag) API_CK(h, cudaMemcpy(tag, L.tag, ntot, cudaMemcpyDeviceToHost));
+  if (curv) API_CK(h, copy_home(curv, L.c64, sizeof(double) * ntot, h->stream));
+  if (tag) API_CK(h, copy_home(tag, L.tag, ntot, h->stream));
+  API_CK(h, cudaStreamSynchronize(h->stream));
   if (max_phi) *max_phi = h->ls.max_phi;
   return 0;
 }
