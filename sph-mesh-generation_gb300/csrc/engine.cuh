@@ -4,16 +4,16 @@
 // reference's operation order) and mrsph_fp32.cu.
 //
 // One step (SPH_mesh_generation::SPH_run_mesh_generation,
-// sph_mesh_generation.cpp:1371-1463) is 11 launches on one stream (15 for a
-// large FP32-split handle in 3D), replayed as a CUDA graph:
+// sph_mesh_generation.cpp:1371-1463) is 11 launches on one stream (15 where the
+// lists are made in brick order), replayed as a CUDA graph:
 //   k_begin_step   scalars of the step
 //   k_map          A1 advect + A2 sample + A3 surface map/re-seed + A4 spacing
 //                  + scale/level refresh + cell key + cell histogram
 //   scan, scatter  A5 counting sort into (level, cell) order
 //   k_reorder      rank inside the cell, gather of the persistent state into the
 //                  sorted order, search radii
-//   k_brick_*      the work order of a large handle's list builder
-//   k_density(_group, _lane)  A6 neighbour search over the cell table: the neighbour lists
+//   k_brick_*      the work order of a large graded 3D handle's list builder
+//   k_density_(group, lane, tile)  A6 neighbour search over the cell table: the neighbour lists
 //   k_force<1>     A7 kernel sum + A8 stage 1 + A9 dt/max|v| grid reduction (FP64
 //                  bit atomics), k_force_spill for particles whose list spilled
 //   k_force<2>     A8 stage 2 + A9 + A10 (stage-1 kick folded in; the stage-2
@@ -137,19 +137,55 @@ struct BatchSlot {
 
 enum { MAP_STEP = 0, MAP_PRE = 1 };
 
-// Particles up to which a handle's own neighbour passes take kG lanes per
-// particle (force_particle, list_group).  Below these counts the chip is not
-// full and a particle's chain of gathers bounds the kernel, above them the
-// instructions do.  Larger handles take one lane per particle in the force
-// passes, and in the FP32-split lists one lane in 2D (list_lane: short rows,
-// about 60 candidates) and a shared tile per warp in 3D (list_warp).  Measured, us:
-// stage 1 of 20,000 in 3D 37 by groups, 67 by lanes, of 77,551 in 2D 39 and 26;
-// lists in 2D of 77,551 70 by groups, 95 by lanes, 127 by warp tiles, of 150,000
-// 73, 42 and 74; in 3D of 60,000 250 by groups and 440 by tiles, of 100,000 366
-// and 461 (two levels) or 806 and 711 (281 neighbours), of 130,000 483 and 426,
-// of 200,000 258 and 216 (by lanes 347).
+// The forms of the neighbour passes.  All give the same lists and the same bits.
+enum ListForm {
+  LIST_GROUP,  // kG lanes per particle (list_group)
+  LIST_LANE,   // one lane per particle (list_lanes), FP32-split
+  LIST_TILE,   // a tile per warp, particles in storage order (list_warp), FP32-split in 3D
+  LIST_BRICK   // the same in brick order
+};
+struct Forms {
+  ListForm list = LIST_GROUP;
+  bool force_group = true;  // kG lanes per particle in the force passes, else one
+  bool operator==(const Forms& o) const { return list == o.list && force_group == o.force_group; }
+};
+// A group shortens the chain of gathers that bounds a pass while the chip is not
+// full, at three times the instructions; so what counts is total, the particles of
+// all handles that step at the same time (n: this handle's).  Force passes: stage
+// 1 of 20,000 in 3D 37 us by groups, 67 by lanes, of 77,551 in 2D 39 and 26.
+// Lists, by levels of the cell list and by row length (dense: more than kDenseRow
+// neighbours on average, as uniformly seeded bodies have), us of 4 steps with
+// upload and download, groups / lanes / tiles / tiles in brick order:
+//   2D, one level    20,000 363/387, 30,000 449/444, 97,000 597/505
+//   2D, graded       60,000 625/672, 85,000 -/681, 110,000 799/734
+//   3D, one level    50,000 937/967/1018/1043, 60,000 992/974/1013/-,
+//                    150,000 1641/1320/1506/1482, 1,000,000 -/6671/6683/6726
+//   3D, graded       90,000 2389/2600/2594/2744, 111,500 2743/-/2600/2430,
+//                    165,000 3598/2906/2704/3385, 200,000 4207/3034/3749/3202,
+//                    600,000 10434/6802/5863/5622, 2,410,164 34445/-/18862/18848
+//   3D, graded dense 30,000 3197/4831/3384/3594, 60,000 5212/6430/4971/5137,
+//                    160,000 7953/7079/6084/7052, 301,270 13017/-/8262/8626
+// Graded bodies want tiles because the candidates of coarse particles near fine
+// ones are many; brick order saves a quarter of the instructions there but makes
+// the longest warps longer, which shows until some 200,000 particles hide them.
+// Many handles side by side (24 bodies of 2,000 to 60,000 particles on streams of
+// their own, 4 steps): 1608 us in 2D and 3076 in 3D chosen by their total, 2515
+// and 5156 each by its own number.
 constexpr long long kGroupMax = 40960;
-constexpr long long kListGroupMax2 = 98304, kListGroupMax3 = 114688;
+constexpr int kDenseRow = 160;
+inline Forms choose_forms(int D, bool fp32, int ncl, bool dense, long long n, long long total) {
+  Forms f;
+  f.force_group = total <= kGroupMax;
+  if (!fp32) return f;
+  if (D == 2) {
+    if (total > (ncl == 1 ? 24576 : 73728)) f.list = LIST_LANE;
+  } else if (ncl == 1) {
+    if (total > 57344) f.list = LIST_LANE;
+  } else if (total > (dense ? 49152 : 98304)) {
+    f.list = dense || n <= 196608 ? LIST_TILE : LIST_BRICK;
+  }
+  return f;
+}
 
 // Tuning of the FP32 map and neighbour passes: resident blocks per SM the
 // register allocation must allow (density: of kDensityThreads threads, else 256).
@@ -771,7 +807,7 @@ __device__ __noinline__ bool exact_cos(const KCtx& c, const float* ni, const flo
 // Storage is by rows of half cells, so the 32 particles of a warp lie along a
 // row, and where rows are short (a shell of one level, the end of a body) in
 // several of them: 2.2 segments per level on a relaxed torus.  The list builder
-// of a large handle therefore takes its particles in another order, by bricks
+// of a large graded handle therefore takes its particles in another order, by bricks
 // of 4 half cells per axis and by Z-order of the half cells inside a brick; what
 // is computed for a particle does not depend on it.
 __device__ inline void brick_of(const CellGeo& g, long long t, int& L, int* q) {
@@ -783,7 +819,7 @@ __device__ inline void brick_of(const CellGeo& g, long long t, int& L, int* q) {
   q[1] = (int)(r % g.bn[L][1]);
   q[2] = (int)(r / g.bn[L][1]);
 }
-// one thread per brick: its particles, from the start table
+// one thread per brick: its particles, from the start table (D = 3)
 template <int D>
 __global__ void __launch_bounds__(256) k_brick_count(KCtx c, const int* __restrict__ cstart, int* __restrict__ bcount) {
   chain_wait();
@@ -794,7 +830,7 @@ __global__ void __launch_bounds__(256) k_brick_count(KCtx c, const int* __restri
   if (c.sc->lcount[L]) {
     const int* hn = c.geo.hn[L];
     const int x0 = 4 * q[0], x1 = min(x0 + 4, hn[0]);
-    for (int z = 4 * q[2]; z < (D == 3 ? min(4 * q[2] + 4, hn[2]) : 1); z++)
+    for (int z = 4 * q[2]; z < min(4 * q[2] + 4, hn[2]); z++)
       for (int y = 4 * q[1]; y < min(4 * q[1] + 4, hn[1]); y++) {
         const long long rb = c.geo.hoff[L] + ((long long)z * hn[1] + y) * hn[0];
         n += cstart[rb + x1] - cstart[rb + x0];
@@ -802,16 +838,20 @@ __global__ void __launch_bounds__(256) k_brick_count(KCtx c, const int* __restri
   }
   bcount[t] = n;
 }
-// one warp per brick with particles: its half cells' particles in Z-order
+// A warp takes per (1 to 32) bricks one after the other, those with particles:
+// their half cells' particles in Z-order.  A brick is a chain of some 1.4 us, so
+// few bricks are spread over many warps: 32 to a warp take 47 us for the 27,000
+// of a one-level body of 150,000 particles, one or two to a warp 10 us for those of
+// a graded one of 200,000.
 template <int D>
 __global__ void __launch_bounds__(256) k_brick_order(KCtx c, const int* __restrict__ cstart,
                                                      const int* __restrict__ bcount, const int* __restrict__ bstart,
-                                                     int* __restrict__ order) {
+                                                     int* __restrict__ order, int per) {
   chain_wait();
   const int lane = threadIdx.x & 31;
-  const long long base = ((long long)blockIdx.x * blockDim.x + threadIdx.x) & ~31ll, nb = c.geo.boff[c.geo.ncl];
+  const long long base = (((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5) * per, nb = c.geo.boff[c.geo.ncl];
   const long long mine = base + lane;
-  unsigned todo = __ballot_sync(0xffffffffu, mine < nb && bcount[mine] > 0);
+  unsigned todo = __ballot_sync(0xffffffffu, lane < per && mine < nb && bcount[mine] > 0);
   while (todo) {
     const long long t = base + __ffs(todo) - 1;
     todo &= todo - 1u;
@@ -819,12 +859,13 @@ __global__ void __launch_bounds__(256) k_brick_order(KCtx c, const int* __restri
     brick_of(c.geo, t, L, q);
     const int* hn = c.geo.hn[L];
     int at = bstart[t];
-    for (int z0 = 0; z0 < (D == 3 ? 64 : 16); z0 += 32) {
+#pragma unroll
+    for (int z0 = 0; z0 < 64; z0 += 32) {
       const int zc = z0 + lane;  // Z-order index of the half cell
       int h[3];
-      bool ok = zc < (D == 3 ? 64 : 16);
+      bool ok = true;
       for (int d = 0; d < 3; d++) {
-        h[d] = d < D ? 4 * q[d] + (((zc >> d) & 1) | (((zc >> (D + d)) & 1) << 1)) : 0;
+        h[d] = 4 * q[d] + (((zc >> d) & 1) | (((zc >> (3 + d)) & 1) << 1));
         ok = ok && h[d] < hn[d];
       }
       int s0 = 0, s1 = 0;
@@ -1252,7 +1293,7 @@ __device__ inline int list_group(const KCtx& c, const Buf<R>& b, const Work<R>& 
   return cnt;
 }
 
-// Neighbour lists of 32 particles by one warp (FP32-split), lane l's particle i.
+// Neighbour lists of 32 particles by one warp (FP32-split, 3D), lane l's particle i.
 // The lanes that sit in neighbouring half cells (a segment: all 32 in the work
 // order, a few groups in storage order) reach nearly the same rows of the
 // sort table.  The lanes take one row each of the segment's bounding box, the
@@ -1269,13 +1310,14 @@ __device__ inline int list_group(const KCtx& c, const Buf<R>& b, const Work<R>& 
 // levels, so its words are full.  Lanes walking their own rows (430 candidates
 // for 86 neighbours in the relaxed state) ran at a third of the warp's width.
 constexpr int kTile = MRSPH_TILE_SIZE, kTileRows = 64, kSegX = MRSPH_TILE_SPAN_X, kSegYZ = MRSPH_TILE_SPAN_YZ;
-static_assert(kTile % 64 == 0 && kTile <= 1024, "whole mask words, at most 32 of them");
+template <int TILE>
 struct WarpTile {
-  float4 xy[kTile / 2];  // (x0, x1, y0, y1) of two candidates
-  float4 zq[kTile / 2];  // (z0, z1, |c|^2_0, |c|^2_1)
-  float2 nr2[kTile / 2];  // squared cut-off radii, negated
-  int id[kTile];
-  unsigned mask[kTile / 32][32];
+  static_assert(TILE % 64 == 0 && TILE <= 1024, "whole mask words, at most 32 of them");
+  float4 xy[TILE / 2];  // (x0, x1, y0, y1) of two candidates
+  float4 zq[TILE / 2];  // (z0, z1, |c|^2_0, |c|^2_1)
+  float2 nr2[TILE / 2];  // squared cut-off radii, negated
+  int id[TILE];
+  unsigned mask[TILE / 32][32];
   int off[kTileRows], end[kTileRows];
 };
 __device__ __forceinline__ unsigned long long pack2(float a, float b) {
@@ -1302,9 +1344,10 @@ __device__ inline float warp_fmax(float v) {
   return v;
 }
 
-template <int D, class LD>
-__device__ inline int list_warp(const KCtx& c, const Buf<float>& b, const Work<float>& w, WarpTile& wt, long long i,
+template <class LD, int TILE>
+__device__ inline int list_warp(const KCtx& c, const Buf<float>& b, const Work<float>& w, WarpTile<TILE>& wt, long long i,
                                 bool act) {
+  constexpr int D = 3;
   const unsigned FULL = 0xffffffffu;
   const int lane = threadIdx.x & 31, BIG = 0x3fffffff;
   float4 a0 = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -1329,7 +1372,7 @@ __device__ inline int list_warp(const KCtx& c, const Buf<float>& b, const Work<f
     int ks[3];
     for (int d = 0; d < 3; d++) {
       ks[d] = __shfl_sync(FULL, k[d], seed);
-      if (d < D) in = in && abs(k[d] - ks[d]) <= (d == 0 ? span : span1);
+      in = in && abs(k[d] - ks[d]) <= (d == 0 ? span : span1);
     }
     rem &= ~__ballot_sync(FULL, in);
     // frame: the middle anchor in x, the seed's in y and z; bounding box
@@ -1375,7 +1418,7 @@ __device__ inline int list_warp(const KCtx& c, const Buf<float>& b, const Work<f
           const ulonglong2 zq = *reinterpret_cast<const ulonglong2*>(&wt.zq[v * 16 + t]);
           const float2 nr = wt.nr2[v * 16 + t];
           unsigned long long s = add2(zq.y, pp2);
-          if (D == 3) s = fma2(zq.x, mz, s);
+          s = fma2(zq.x, mz, s);
           s = fma2(xy.y, my, s);
           s = fma2(xy.x, mx, s);
           s = add2(s, pack2(fminf(nR2i, nr.x), fminf(nR2i, nr.y)));
@@ -1440,7 +1483,7 @@ __device__ inline int list_warp(const KCtx& c, const Buf<float>& b, const Work<f
           LD::rec(b.rec, j, b0, b1);
           e[0] = fmaf(b1.x - fk[0], c.geo.Af[0], b0.x);
           e[1] = fmaf(b1.y - fk[1], c.geo.Af[1], b0.y);
-          if (D == 3) e[2] = fmaf(b1.z - fk[2], c.geo.Af[2], b0.z);
+          e[2] = fmaf(b1.z - fk[2], c.geo.Af[2], b0.z);
           const float rj = b0.w * cut;
           rr = rj * rj;
           float d2 = 0.f;
@@ -1466,7 +1509,7 @@ __device__ inline int list_warp(const KCtx& c, const Buf<float>& b, const Work<f
           rmax = fmaxf(rmax, rr);
         }
         tn += __popc(m);
-        if (tn > kTile - 32) drain();
+        if (tn > TILE - 32) drain();
       }
       __syncwarp();
       nrow = 0;
@@ -1510,24 +1553,20 @@ __device__ inline int list_warp(const KCtx& c, const Buf<float>& b, const Work<f
         ymin = __reduce_min_sync(FULL, ymin);
         r0[1] = max(r0[1], 4 * ymin);
         r1[1] = min(r1[1], 4 * ymax + 3);
-        if (D == 3) {
-          r0[2] = max(r0[2], 4 * __reduce_min_sync(FULL, zmin));
-          r1[2] = min(r1[2], 4 * __reduce_max_sync(FULL, zmax) + 3);
-        }
+        r0[2] = max(r0[2], 4 * __reduce_min_sync(FULL, zmin));
+        r1[2] = min(r1[2], 4 * __reduce_max_sync(FULL, zmax) + 3);
       }
       const int ny = r1[1] - r0[1] + 1, nr = ny * (r1[2] - r0[2] + 1);
       for (int rb = 0; rb < nr; rb += 32) {
         const int rr = rb + lane;
         int s0 = 0, e0 = 0;
         if (rr < nr) {
-          const int iz = D == 3 ? rr / ny : 0;
+          const int iz = rr / ny;
           const int z = r0[2] + iz, y = r0[1] + rr - iz * ny;
           float gz = 0.f, gy = 0.f;
-          if (D == 3) {
-            const float zl = fmaf((float)(z - h0[2]), c.geo.hs_f[L][2], -f0[2]);
-            if (z > 0) gz = fmaxf(gz, zl - hi[2]);
-            if (z < c.geo.hn[L][2] - 1) gz = fmaxf(gz, lo[2] - (zl + c.geo.hs_f[L][2]));
-          }
+          const float zl = fmaf((float)(z - h0[2]), c.geo.hs_f[L][2], -f0[2]);
+          if (z > 0) gz = fmaxf(gz, zl - hi[2]);
+          if (z < c.geo.hn[L][2] - 1) gz = fmaxf(gz, lo[2] - (zl + c.geo.hs_f[L][2]));
           const float yl = fmaf((float)(y - h0[1]), c.geo.hs_f[L][1], -f0[1]);
           if (y > 0) gy = fmaxf(gy, yl - hi[1]);
           if (y < c.geo.hn[L][1] - 1) gy = fmaxf(gy, lo[1] - (yl + c.geo.hs_f[L][1]));
@@ -1569,10 +1608,9 @@ __device__ inline int list_warp(const KCtx& c, const Buf<float>& b, const Work<f
 }
 
 // Neighbour list of particle i by one lane (FP32-split), its rows one after the
-// other, two candidates in flight.  EXACT = false decides in FP32 and returns -1
-// when a pair lies in the criterion's band; the list is then taken again with
-// the whole test, which the hot loop has no registers for.
-template <int D, bool EXACT, class LD>
+// other, two candidates in flight, decided in FP32: -1 when a pair lies in the
+// criterion's band (the hot loop has no registers for the exact test).
+template <int D, class LD>
 __device__ inline int list_lane(const KCtx& c, const Buf<float>& b, const Work<float>& w, long long i) {
   const PairTest<D, float> pt(c, b.rec, i);
   const SOrigin<D, float> so(c, b.posh[i], b.key[i]);
@@ -1595,25 +1633,43 @@ __device__ inline int list_lane(const KCtx& c, const Buf<float>& b, const Work<f
       for (int y = lo[1]; y <= up[1]; y++) {
         int s0, e0;
         if (!row_range<D, LD>(c, w.cstart, L, R_, q, fr, z, y, s0, e0)) continue;
-        if constexpr (EXACT) {
-          for (int j = s0; j < e0; j++)
-            if (pt.template near<LD>(c, b.rec, j)) take(j);
-        } else {
-          for (int j = s0; j < e0; j += 2) {
-            float4 b0, b1, c0, c1;
-            LD::rec(b.rec, j, b0, b1);
-            LD::rec(b.rec, min(j + 1, e0 - 1), c0, c1);
-            if (pt.near32(c, b0, b1, close)) take(j);
-            if (j + 1 < e0 && pt.near32(c, c0, c1, close)) take(j + 1);
-          }
+        for (int j = s0; j < e0; j += 2) {
+          float4 b0, b1, c0, c1;
+          LD::rec(b.rec, j, b0, b1);
+          LD::rec(b.rec, min(j + 1, e0 - 1), c0, c1);
+          if (pt.near32(c, b0, b1, close)) take(j);
+          if (j + 1 < e0 && pt.near32(c, c0, c1, close)) take(j + 1);
         }
       }
   }
   return close ? -1 : cnt;
 }
+// Lists of the 32 particles from first, lane l's being first + l.  Those with a
+// pair in the band (one particle in 300 of 74 neighbours, so one warp in ten)
+// are taken again by groups, which decide as the reference does; a lane taking
+// them again made its warp wait for a second whole list.
 template <int D, class LD>
-__device__ __noinline__ int list_lane_exact(const KCtx& c, const Buf<float>& b, const Work<float>& w, long long i) {
-  return list_lane<D, true, LD>(c, b, w, i);
+__device__ inline int list_lanes(const KCtx& c, const Buf<float>& b, const Work<float>& w, RowTile& rt,
+                                 long long first) {
+  const unsigned FULL = 0xffffffffu;
+  const int lane = threadIdx.x & 31;
+  int cnt = first + lane < c.n ? list_lane<D, LD>(c, b, w, first + lane) : 0;
+  unsigned again = __ballot_sync(FULL, cnt < 0);
+  while (again) {
+    const GroupLanes g;
+    unsigned left = again;  // group k takes the k-th of them
+    for (int k = 0; k < lane / kG; k++) left &= left - 1u;
+    const int own = left ? __ffs(left) - 1 : -1;
+    for (int k = 0; k < 32 / kG; k++) again &= again - 1u;
+    int m = 0;
+    if (own >= 0) m = list_group<D, float, LD>(c, b, w, g, rt, first + own);
+    __syncwarp();
+    for (int k = 0; k < 32; k += kG) {
+      const int to = __shfl_sync(FULL, own, k), v = __shfl_sync(FULL, m, k);
+      if (lane == to) cnt = v;
+    }
+  }
+  return cnt;
 }
 
 // what follows a list: its length, the spill queue, the step's totals
@@ -1645,25 +1701,31 @@ __device__ inline void density_group_block(const KCtx& c, const Buf<R>& b, const
 }
 
 // particles [first, first + blockDim.x), one warp per 32
-template <int D, class LD = LdNC>
-__device__ inline void density_warp_block(const KCtx& c, const Buf<float>& b, const Work<float>& w, WarpTile* tiles,
+template <class LD = LdNC, int TILE>
+__device__ inline void density_warp_block(const KCtx& c, const Buf<float>& b, const Work<float>& w, WarpTile<TILE>* tiles,
                                           long long first) {
   const long long t = first + threadIdx.x;
   const bool act = t < c.n;
   const long long i = act && w.order ? w.order[t] : t;
-  const int cnt = list_warp<D, LD>(c, b, w, tiles[threadIdx.x >> 5], i, act);
-  list_done<D, float>(c, w, i, cnt, act);
+  const int cnt = list_warp<LD>(c, b, w, tiles[threadIdx.x >> 5], i, act);
+  list_done<3, float>(c, w, i, cnt, act);
+}
+
+// particles [first, first + blockDim.x), a lane each
+template <int D, class LD = LdNC>
+__device__ inline void density_lane_block(const KCtx& c, const Buf<float>& b, const Work<float>& w, RowTile* tiles,
+                                          long long first) {
+  const long long i = first + threadIdx.x;
+  const int cnt = list_lanes<D, LD>(c, b, w, tiles[threadIdx.x / kG], i - (threadIdx.x & 31));
+  list_done<D, float>(c, w, i, cnt, i < c.n);
 }
 
 constexpr int kDensityThreads = 128;
 template <int D>
-__global__ void __launch_bounds__(kDensityThreads, 8) k_density_lane(KCtx c, Buf<float> b, Work<float> w) {
+__global__ void __launch_bounds__(kDensityThreads, D == 2 ? 8 : 10) k_density_lane(KCtx c, Buf<float> b, Work<float> w) {
   chain_wait();
-  const long long i = (long long)blockIdx.x * kDensityThreads + threadIdx.x;
-  int cnt = i < c.n ? list_lane<D, false, LdNC>(c, b, w, i) : 0;
-  if (cnt < 0) cnt = list_lane_exact<D, LdNC>(c, b, w, i);
-  __syncwarp();
-  list_done<D, float>(c, w, i, cnt, i < c.n);
+  __shared__ RowTile tiles[kDensityThreads / kG];
+  density_lane_block<D>(c, b, w, tiles, (long long)blockIdx.x * kDensityThreads);
 }
 template <int D, class R>
 __global__ void __launch_bounds__(kDensityThreads, 10) k_density_group(KCtx c, Buf<R> b, Work<R> w) {
@@ -1672,10 +1734,10 @@ __global__ void __launch_bounds__(kDensityThreads, 10) k_density_group(KCtx c, B
   density_group_block<D, R>(c, b, w, tiles, (long long)blockIdx.x * (kDensityThreads / kG));
 }
 template <int D>
-__global__ void __launch_bounds__(kDensityThreads, MRSPH_DENSITY_MIN_BLOCKS) k_density(KCtx c, Buf<float> b, Work<float> w) {
+__global__ void __launch_bounds__(kDensityThreads, MRSPH_DENSITY_MIN_BLOCKS) k_density_tile(KCtx c, Buf<float> b, Work<float> w) {
   chain_wait();
-  __shared__ WarpTile tiles[kDensityThreads / 32];
-  density_warp_block<D>(c, b, w, tiles, (long long)blockIdx.x * kDensityThreads);
+  __shared__ WarpTile<kTile> tiles[kDensityThreads / 32];
+  density_warp_block<LdNC>(c, b, w, tiles, (long long)blockIdx.x * kDensityThreads);
 }
 
 __device__ inline void accum_pairs_body(DevScalars* sc) { sc->pairs_total += sc->pairs; }
@@ -2378,7 +2440,7 @@ class Engine : public EngineBase {
       }
       int rc = build_graphs();
       if (rc) return rc;
-      MR_CK(cudaGraphLaunch(graph_[cur_], st_));
+      MR_CK(cudaGraphLaunch(graphs_[0][cur_], st_));
       cur_ ^= 1;
       have_work_ = true;
       if (--countdown_ <= 0) {
@@ -2396,10 +2458,18 @@ class Engine : public EngineBase {
   // beside the current lists, at least 48 GB), or when the caller fixed the
   // cap; a growth that falls short raises MRSPH_FLAG_CAPACITY_CLAMPED in the
   // next stats.
+  // The form of the passes follows the mean row length seen here.
   int maybe_grow_cap() {
-    unsigned mc = 0;
-    MR_CK(cudaMemcpyAsync(&mc, &kc_.sc->maxcnt, sizeof(unsigned), cudaMemcpyDeviceToHost, st_));
+    DevScalars h;
+    MR_CK(cudaMemcpyAsync(&h, kc_.sc, sizeof(h), cudaMemcpyDeviceToHost, st_));
     MR_CK(cudaStreamSynchronize(st_));
+    dense_ = (long long)h.pairs > kDenseRow * n_;
+    const Forms f = choose_forms(n_, n_);
+    if (!(f == alone_)) {
+      drop_graphs(0);
+      alone_ = forms_ = f;
+    }
+    const unsigned mc = h.maxcnt;
     if ((int)mc <= w_.cap || cfg_.neighbor_cap > 0) return 0;
     long long want = ((long long)mc * 5 / 4 + 31) / 32 * 32;
     const long long n32 = (n_ + 31) / 32 * 32;  // nb_slot blocks of 32 particles
@@ -2449,13 +2519,18 @@ class Engine : public EngineBase {
     return 0;
   }
 
-  int build_graphs() {
+  // The step graphs: those of the handle's steps alone, or (set 1) those of its
+  // steps beside other handles' with forms of their own.
+  int build_graphs(int set = 0) {
+    cudaGraphExec_t* const graph_ = graphs_[set];
     for (int p = 0; p < 2; p++) {
       if (!graph_[p]) {
         int saved = cur_;
         cur_ = p;
         MR_CK(cudaStreamBeginCapture(st_, cudaStreamCaptureModeThreadLocal));
+        forms_ = set ? beside_ : alone_;
         int rc = launch_step(MRSPH_PHASE_FORCE2);
+        forms_ = alone_;
         cudaGraph_t g;
         cudaError_t ee = cudaStreamEndCapture(st_, &g);
         cur_ = saved;
@@ -2471,24 +2546,31 @@ class Engine : public EngineBase {
   }
 
   void drop_graphs() {
+    drop_graphs(0);
+    drop_graphs(1);
+  }
+  void drop_graphs(int set) {
     for (int p = 0; p < 2; p++) {
-      if (graph_[p]) { cudaGraphExecDestroy(graph_[p]); graph_[p] = nullptr; }
+      cudaGraphExec_t& g = graphs_[set][p];
+      if (g) { cudaGraphExecDestroy(g); g = nullptr; }
     }
   }
 
   // One step of a batch: the step graph of the current parity launched on the
   // handle's stream, without the periodic capacity check (the batch makes it).
-  int step_batched() override {
+  // total: the particles of all handles that step at the same time.
+  int step_batched(long long total) override {
     if (!n_) { err = "no particles"; return MRSPH_ERR_STATE; }
-    int rc = build_graphs();
+    const int set = graph_set(total);
+    int rc = build_graphs(set);
     if (rc) return rc;
-    MR_CK(cudaGraphLaunch(graph_[cur_], st_));
+    MR_CK(cudaGraphLaunch(graphs_[set][cur_], st_));
     cur_ ^= 1;
     have_work_ = true;
     return 0;
   }
 
-  int prepare_steps() override { return n_ ? build_graphs() : 0; }
+  int prepare_steps(long long total) override { return n_ ? build_graphs(graph_set(total)) : 0; }
 
   int check_capacity() override { return have_work_ ? maybe_grow_cap() : 0; }
 
@@ -2742,24 +2824,49 @@ class Engine : public EngineBase {
     return 0;
   }
 
+  Forms choose_forms(long long n, long long total) const {
+    return mrsph::choose_forms(D, std::is_same<R, float>::value, kc_.geo.ncl, dense_, n, total);
+  }
+  // the graphs that a step beside handles of total particles takes
+  // (half of their number: two handles of 23,000 take 739 us by the forms of 23,000
+  // particles, 827 by those of 46,000)
+  int graph_set(long long total) {
+    const Forms f = choose_forms(n_, std::max(n_, total / 2));
+    if (f == alone_) return 0;
+    if (!(f == beside_) && graphs_[1][0]) {
+      cudaStreamSynchronize(st_);
+      drop_graphs(1);
+    }
+    beside_ = f;
+    return 1;
+  }
+
   int ggrid(int threads) const { return (int)((n_ + threads / kG - 1) / (threads / kG)); }  // kG lanes per particle
 
   void launch_lists() {
-    const long long n = n_;
     if constexpr (std::is_same<R, float>::value) {
-      if (D == 2 && n > kListGroupMax2) {
-        launch_chained(k_density_lane<D>, (unsigned)((n + kDensityThreads - 1) / kDensityThreads), kDensityThreads, st_, kc_, buf_[cur_], w_);
+      const unsigned blocks = (unsigned)((n_ + kDensityThreads - 1) / kDensityThreads);
+      if (forms_.list == LIST_LANE) {
+        launch_chained(k_density_lane<D>, blocks, kDensityThreads, st_, kc_, buf_[cur_], w_);
         return;
       }
-    }
-    if constexpr (D == 3 && std::is_same<R, float>::value) {
-      if (n > kListGroupMax3) {
-        const long long nb = kc_.geo.boff[kc_.geo.ncl];
-        launch_chained(k_brick_count<D>, grid(nb), 256, st_, kc_, w_.cstart, w_.bcount);
-        cell_scan(w_.bcount, w_.bstart, w_.blocksums, nb, (int)n, st_);
-        launch_chained(k_brick_order<D>, grid(nb), 256, st_, kc_, w_.cstart, w_.bcount, w_.bstart, w_.order);
-        launch_chained(k_density<D>, (unsigned)((n + kDensityThreads - 1) / kDensityThreads), kDensityThreads, st_, kc_, buf_[cur_], w_);
-        return;
+      if constexpr (D == 3) {
+        if (forms_.list == LIST_TILE || forms_.list == LIST_BRICK) {
+          Work<R> w = w_;
+          if (forms_.list == LIST_BRICK) {
+            const long long nb = kc_.geo.boff[kc_.geo.ncl];
+            int per = 1;  // bricks per warp: 64 warps per SM or more
+            while (per < 32 && nb > 64ll * sms_ * 2 * per) per *= 2;
+            launch_chained(k_brick_count<D>, grid(nb), 256, st_, kc_, w_.cstart, w_.bcount);
+            cell_scan(w_.bcount, w_.bstart, w_.blocksums, nb, (int)n_, st_);
+            launch_chained(k_brick_order<D>, grid((nb + per - 1) / per * 32), 256, st_, kc_, w_.cstart, w_.bcount, w_.bstart,
+                           w_.order, per);
+          } else {
+            w.order = w.bstart = nullptr;
+          }
+          launch_chained(k_density_tile<D>, blocks, kDensityThreads, st_, kc_, buf_[cur_], w);
+          return;
+        }
       }
     }
     launch_chained(k_density_group<D, R>, ggrid(kDensityThreads), kDensityThreads, st_, kc_, buf_[cur_], w_);
@@ -2767,7 +2874,7 @@ class Engine : public EngineBase {
 
   template <int STAGE, int KK>
   void launch_force_kind() {
-    if (n_ <= kGroupMax) launch_chained(k_force_group<D, R, STAGE, KK>, ggrid(kGroupThreads), kGroupThreads, st_, kc_, buf_[cur_], w_);
+    if (forms_.force_group) launch_chained(k_force_group<D, R, STAGE, KK>, ggrid(kGroupThreads), kGroupThreads, st_, kc_, buf_[cur_], w_);
     else launch_chained(k_force<D, R, STAGE, KK>, grid(n_), 256, st_, kc_, buf_[cur_], w_);
     launch_chained(k_force_spill<D, R, STAGE, KK>, qgrid(), kGroupThreads, st_, kc_, buf_[cur_], w_);
   }
@@ -2959,7 +3066,9 @@ class Engine : public EngineBase {
       rc |= A((void**)&kc_.sc, sizeof(DevScalars));
     }
     w_.bcount = w_.bstart = w_.order = nullptr;
-    if (!rc && D == 3 && std::is_same<R, float>::value && n > kListGroupMax3) {
+    dense_ = false;
+    forms_ = alone_ = choose_forms(n, n);
+    if (!rc && alone_.list == LIST_BRICK) {
       const long long nb = kc_.geo.boff[kc_.geo.ncl];
       rc |= A((void**)&w_.bcount, sizeof(int) * nb);
       rc |= A((void**)&w_.bstart, sizeof(int) * (nb + 1));
@@ -2993,8 +3102,10 @@ class Engine : public EngineBase {
   long long n_ = 0, ncells_ = 0;
   int cur_ = 0;
   bool have_work_ = false;
+  bool dense_ = false;  // rows longer than kDenseRow on average, when the capacity was last checked
   int countdown_ = 0;
-  cudaGraphExec_t graph_[2] = {nullptr, nullptr};
+  Forms forms_, alone_, beside_;  // those of the launches being made, of steps alone, of graph set 1
+  cudaGraphExec_t graphs_[2][2] = {};  // [set][parity]
   std::vector<void*> allocs_;
   std::vector<void*> anc_allocs_;  // anchor tables, kept across re-allocations
   int init_rc_ = 0;

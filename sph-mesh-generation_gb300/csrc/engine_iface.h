@@ -70,11 +70,12 @@ class EngineBase {
                          unsigned* d_flags, double* d_h = nullptr, bool sort_rows = true) = 0;
   virtual int neighbor_capacity() const = 0;
   // Batched stepping: one step launched on the handle's stream without the
-  // periodic capacity check; the step graphs built ahead of a timed region;
+  // periodic capacity check; the step graphs built ahead of a timed region
+  // (total: the particles of all handles that step at the same time);
   // the neighbour-list capacity check a solo step makes every 32 steps (the
   // handle's stream must be idle; the graphs may be rebuilt).
-  virtual int step_batched() = 0;
-  virtual int prepare_steps() = 0;
+  virtual int step_batched(long long total) = 0;
+  virtual int prepare_steps(long long total) = 0;
   virtual int check_capacity() = 0;
   // The batch kernels' view of the handle (FP32-split engines; see BatchSlot)
   // and the bookkeeping after nsteps steps of a batch launch.

@@ -12,7 +12,9 @@
 // * streams: every handle keeps the CUDA graph of its own step and a batch
 //   step launches each handle's graph on the handle's own stream, back to
 //   back from one host thread (about 8.5 ms of host launch cost per step for
-//   512 handles).  FP64-plain handles always step this way.
+//   512 handles).  The graphs are those of the neighbour-pass forms that suit the
+//   batch's particles together (choose_forms, engine.cuh).  FP64-plain handles
+//   always step this way.
 //
 // Either way each handle's results are those of stepping it alone (the same
 // device code on the same state).  Ordering: the batch kernels run on the
@@ -107,11 +109,18 @@ int check_caps(mrsph_batch* b) {
   return 0;
 }
 
+long long particles(const mrsph_batch* b) {
+  long long n = 0;
+  for (auto* e : b->engines) n += e->num_particles();
+  return n;
+}
+
 int run_streams(mrsph_batch* b, int nsteps, bool checks) {
+  const long long total = particles(b);
   for (int s = 0; s < nsteps; s++) {
     for (size_t k = 0; k < b->hs.size(); k++) {
       mrsph::EngineBase* e = b->engines[k];
-      int rc = e->step_batched();
+      int rc = e->step_batched(total);
       if (rc) return bfail(b, rc, "handle " + std::to_string(k) + ": " + e->err);
     }
     if (checks && --b->countdown <= 0) {
@@ -275,7 +284,7 @@ extern "C" int mrsph_batch_step_timed(mrsph_batch* b, int nsteps, double* ms) {
   // settle capacities and build every graph outside the timed region
   int rc = check_caps(b);
   for (size_t k = 0; !rc && k < b->hs.size(); k++) {
-    rc = b->engines[k]->prepare_steps();
+    rc = b->engines[k]->prepare_steps(particles(b));
     if (rc) rc = bfail(b, rc, "handle " + std::to_string(k) + ": " + b->engines[k]->err);
   }
   if (rc) return rc;

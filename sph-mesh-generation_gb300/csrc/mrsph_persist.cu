@@ -38,11 +38,18 @@
 namespace mrsph {
 
 // resident 256-thread blocks per SM of the persistent kernel, i.e. its
-// register budget (2: 128 registers, where the fused phases do not spill;
-// 4: 64, with spills in the rare paths but twice the warps; measured on a
-// GB300 with 512 geometries: 45, 37 and 32 ms per step at 2, 3 and 4)
+// register budget, and the candidates of a warp's tile in the batch kernels (8
+// tiles of 256 take 61 KB of shared memory, so that a fourth block would not be
+// resident whatever the registers; 8 of 128 take 32 KB).  us for 4 steps with
+// upload and download, by tile / blocks:
+//                                       128/3  128/4  192/3  256/3  192/4
+//   24 3D stars of 2,000 to 60,000       5339   5697   5385   5499   6700
+//   24 2D stars                          2578   2681   2614   2666   2939
+//   64 3D stars of 2,000 to 4,000        4347   4693   4420   4441   5482
+//   16 graded tori of 8,000 to 40,000    9024   8377   9176   9339   9969
+// Four blocks spill 796 bytes a thread, three 420.
 #ifndef MRSPH_BATCH_MIN_BLOCKS
-#define MRSPH_BATCH_MIN_BLOCKS 4
+#define MRSPH_BATCH_MIN_BLOCKS 3
 #endif
 constexpr int kBatchThreads = 256;
 constexpr int kBatchScanCells = kBatchThreads * SCAN_ITEMS;  // cells per scan item
@@ -157,10 +164,26 @@ __device__ inline void load_slot(const BatchPlan& P, int g, BatchSlot& s_slot, i
   __syncthreads();
 }
 
+#ifndef MRSPH_BATCH_TILE
+#define MRSPH_BATCH_TILE 128
+#endif
+constexpr int kBatchTile = MRSPH_BATCH_TILE;
+
 union PhaseTiles {  // shared memory of the phases that scan cells
-  WarpTile tile[kBatchThreads / 32];
+  WarpTile<kBatchTile> tile[kBatchThreads / 32];
+  RowTile rows[kBatchThreads / kG];
   GroupTile<float> spill[kBatchThreads / kG];
 };
+
+// The lists of a block's particles: a lane each in 2D, tiles in storage order in
+// 3D.  (24 uniformly seeded 2D stars 2178 us, 2398 by tiles; 16 graded 2D bodies
+// 3457 and 4690.)
+template <int D, class LD>
+__device__ inline void list_item(const KCtx& c, const Buf<float>& b, const Work<float>& w, long long blk,
+                                 PhaseTiles& sm) {
+  if constexpr (D == 2) density_lane_block<D, LD>(c, b, w, sm.rows, blk * kBatchThreads);
+  else density_warp_block<LD>(c, b, w, sm.tile, blk * kBatchThreads);
+}
 
 template <int D, int KK, class LD>
 __device__ inline void run_item_d(const BatchSlot& S, int ph, long long blk, long long nblk, int cur, PhaseTiles& sm) {
@@ -179,7 +202,7 @@ __device__ inline void run_item_d(const BatchSlot& S, int ph, long long blk, lon
     case BP_SCAN_DOWN: scan_down_block(S.w.counts, S.ncells, S.w.blocksums, S.w.cstart, (int)S.c.n, blk); break;
     case BP_SCATTER: scatter_block(b0.cellkey, b0.id, S.w.counts, S.w.cstart, S.w.perm, S.w.pid, S.c.n, blk); break;
     case BP_REORDER: reorder_block<D, float, LD>(b0, b1, S.c, S.w, 0, blk); break;
-    case BP_DENSITY: density_warp_block<D, LD>(S.c, b1, S.w, sm.tile, blk * kBatchThreads); break;
+    case BP_DENSITY: list_item<D, LD>(S.c, b1, S.w, blk, sm); break;
     case BP_FORCE1:
       if (blk == 0 && threadIdx.x == 0) accum_pairs_body(S.c.sc);
       force_block<D, float, 1, KK, 1, LD>(S.c, b1, S.w, nullptr, blk * kBatchThreads);

@@ -5,9 +5,9 @@ candidates; MRSPH_TILE_SPAN_X / _YZ: the spread in half cells within which a
 warp's particles share one) and their resident blocks per SM, i.e. registers per
 thread and work per SM (MRSPH_DENSITY_MIN_BLOCKS, MRSPH_FORCE_MIN_BLOCKS,
 MRSPH_FORCE2_MIN_BLOCKS, MRSPH_MAP_MIN_BLOCKS), as compile-time macros; the
-persistent batch kernel its resident blocks per SM (MRSPH_BATCH_MIN_BLOCKS)
-and the items a block claims at a time from a phase's work queue
-(MRSPH_BATCH_CHUNK), tuned on a batch workload (--workload star_batch_512).  This
+persistent batch kernel its resident blocks per SM (MRSPH_BATCH_MIN_BLOCKS), the
+items a block claims at a time from a phase's work queue (MRSPH_BATCH_CHUNK)
+and the candidates of a warp's tile (MRSPH_BATCH_TILE), tuned on a batch workload (--workload star_batch_512).  This
 tuner builds candidate settings side by side (one build directory each),
 times each on a workload in a fresh process (device-timed steps after a
 warm-up, mrsph_step_timed), searches coordinate by coordinate from the
@@ -31,8 +31,9 @@ from . import build as _build
 # the engine's defaults (csrc/engine.cuh) and the values tried per macro
 DEFAULTS: Dict[str, int] = {"DENSITY_MIN_BLOCKS": 6, "FORCE_MIN_BLOCKS": 5, "FORCE2_MIN_BLOCKS": 6,
                             "MAP_MIN_BLOCKS": 4, "TILE_SIZE": 256, "TILE_SPAN_X": 15, "TILE_SPAN_YZ": 1}
-BATCH_DEFAULTS: Dict[str, int] = {"BATCH_MIN_BLOCKS": 4, "BATCH_CHUNK": 2}
-BATCH_SPACE: Dict[str, List[int]] = {"BATCH_MIN_BLOCKS": [2, 3, 4, 5, 6], "BATCH_CHUNK": [1, 2, 4, 8]}
+BATCH_DEFAULTS: Dict[str, int] = {"BATCH_MIN_BLOCKS": 3, "BATCH_CHUNK": 2, "BATCH_TILE": 128}
+BATCH_SPACE: Dict[str, List[int]] = {"BATCH_MIN_BLOCKS": [2, 3, 4, 5, 6], "BATCH_CHUNK": [1, 2, 4, 8],
+                               "BATCH_TILE": [128, 192, 256]}
 SPACE: Dict[str, List[int]] = {"DENSITY_MIN_BLOCKS": [5, 6, 7], "FORCE_MIN_BLOCKS": [4, 5, 6],
                                "FORCE2_MIN_BLOCKS": [5, 6, 8], "MAP_MIN_BLOCKS": [3, 4],
                                "TILE_SIZE": [128, 192, 256], "TILE_SPAN_X": [7, 15, 31], "TILE_SPAN_YZ": [1, 3]}
