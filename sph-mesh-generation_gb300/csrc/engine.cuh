@@ -2459,7 +2459,9 @@ class Engine : public EngineBase {
   // cap; a growth that falls short raises MRSPH_FLAG_CAPACITY_CLAMPED in the
   // next stats.
   // The form of the passes follows the mean row length seen here.
-  int maybe_grow_cap() {
+  // settle: no force has read the lists yet, so those that spill into a larger
+  // capacity were no spills.
+  int maybe_grow_cap(bool settle = false) {
     DevScalars h;
     MR_CK(cudaMemcpyAsync(&h, kc_.sc, sizeof(h), cudaMemcpyDeviceToHost, st_));
     MR_CK(cudaStreamSynchronize(st_));
@@ -2513,6 +2515,7 @@ class Engine : public EngineBase {
     // (taps, meshes) finds them in the new arrays
     MR_CK(cudaMemsetAsync(&kc_.sc->pairs, 0, sizeof(kc_.sc->pairs), st_));
     MR_CK(cudaMemsetAsync(&kc_.sc->nspill, 0, sizeof(kc_.sc->nspill), st_));
+    if (settle) MR_CK(cudaMemcpyAsync(&kc_.sc->flags, &kc_.sc->flags0, sizeof(unsigned), cudaMemcpyDeviceToDevice, st_));
     launch_lists();
     MR_CK(cudaGetLastError());
     MR_CK(cudaStreamSynchronize(st_));  // a batch steps the handle on another stream
@@ -2908,9 +2911,10 @@ class Engine : public EngineBase {
     cur_ ^= 1;
     mark(4);
     if (phase < MRSPH_PHASE_DENSITY) return 0;
+    if (settle) MR_CK(cudaMemcpyAsync(&kc_.sc->flags0, &kc_.sc->flags, sizeof(unsigned), cudaMemcpyDeviceToDevice, st_));
     launch_lists();
     if (settle) {
-      int rc = maybe_grow_cap();
+      int rc = maybe_grow_cap(true);
       if (rc) return rc;
     }
     have_work_ = true;

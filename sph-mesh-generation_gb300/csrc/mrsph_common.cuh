@@ -100,7 +100,8 @@ struct DevScalars {
   float dt_adv_f, hdt_adv_f;  // FP32 dt_adv and dt_adv / 2 (set with dt_adv at the start of a step)
   unsigned long long pairs;
   unsigned long long pairs_total;
-  unsigned int remap, nsurf, flags, spill;
+  unsigned int remap, nsurf, flags;
+  unsigned int flags0;  // flags before the lists of a step that settles the capacity
   unsigned int step;
   unsigned int maxcnt;  // largest neighbour count of the last density phase
   unsigned int nspill;  // particles whose neighbour list spilled (re-scanned by the force fix-up launches)
