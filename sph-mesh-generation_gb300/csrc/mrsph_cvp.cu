@@ -468,7 +468,9 @@ __global__ void __launch_bounds__(128) k_cvp_face_cull(CvpGeo G, const double* _
   float mag = S;
   for (int q = 0; q < 3; q++) mag += fmaxf(fabsf(lo[q]), fabsf(hi[q]));
   int nv = live ? 4 : 0;
-  bool full = false;  // more vertices than are kept: left to the FP64 pass
+  // left to the FP64 pass: a box whose squares leave FP32's range (S is then 0 or
+  // infinite), or more vertices than are kept
+  bool full = !(mag > 1.e-15f && mag < 1.e15f);
   auto clip = [&](const float* cn, float cd, bool act) {
     const int no = gclip<float>(g, A, act ? nv : 0, cn, cd + kCullMargin * (mag + fabsf(cd)), B, s_s[grp]);
     if (no < 0) return;
