@@ -719,12 +719,16 @@ __global__ void __launch_bounds__(32 * kVmWarps) k_vm_columns(const int* __restr
   }
   __syncwarp();
   float c[8], M = 0.f;
+  bool fits = true;
   for (int q = 0; q < 8; q++) {
     c[q] = (float)cor[q];
     M = fmaxf(M, fabsf(c[q]));
+    fits = fits && fabsf(c[q]) < 1.e35f;
   }
-  // M rounded up, so that the bands hold for the FP64 corners
-  M *= 1.000001f;
+  // M rounded up, so that the bands hold for the FP64 corners; where the products
+  // of the root search (64 times a sum of four) leave FP32's range, and where a
+  // corner is no number, nothing but the refinement decides
+  M = fits ? M * 1.000001f : __int_as_float(0x7f800000);
   const float th = M * 0x1p-20f + 1.e-37f, thc = M * 0x1p-17f + 1.e-37f;
   // (corners near FP32's smallest numbers: no FP64 decision, M being inexact)
   const double th64 = M > 1.e-30f ? (double)M * 0x1p-46 : 1.e300, thc64 = M > 1.e-30f ? (double)M * 0x1p-44 : 1.e300;
