@@ -249,14 +249,19 @@ __global__ void k_tri_mark(TriIn T, unsigned char* mark, long long* queue, unsig
   }
   __syncwarp();
   const double px = T.xyz[3 * i64], py = T.xyz[3 * i64 + 1];
+  // the bounds are relative to products of two lengths: a row whose products leave
+  // FP32's range (a length below 1e-15 or above 1e15) is decided exactly
+  bool fits = true;
   for (int q = lane; q < m; q += 32) {
     const long long j = id[q];
     S[q] = (int)j;
     const float x = (float)(T.xyz[3 * j] - px), y = (float)(T.xyz[3 * j + 1] - py);
     const float n2 = fmaf(y, y, x * x);
     w[q] = make_float4(x, y, n2, sqrtf(n2));
+    if (j != i64) fits = fits && n2 > 1.e-30f && n2 < 1.e30f;
   }
   __syncwarp();
+  fits = __all_sync(0xffffffffu, fits);
   const float INF = __int_as_float(0x7f800000);
   for (int q = lane; q < m; q += 32) {
     unsigned char* out = mark + i64 * T.cap + q;
@@ -267,8 +272,8 @@ __global__ void k_tri_mark(TriIn T, unsigned char* mark, long long* queue, unsig
     const float4 e = w[q];
     const float es0 = 16.f * kTE * e.w, ed0 = 16.f * kTE;
     float loL = INF, hiL = INF, loR = INF, hiR = INF;
-    bool undecided = false, cut = false;
-    for (int k = 0; k < m; k++) {
+    bool undecided = !fits, cut = false;
+    for (int k = 0; fits && k < m; k++) {
       if (k == q || id[k] == i) continue;
       const float4 p = w[k];
       const float s = e.x * p.y - e.y * p.x, d = p.z - fmaf(e.y, p.y, e.x * p.x);
