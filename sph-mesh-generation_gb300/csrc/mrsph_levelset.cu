@@ -430,9 +430,8 @@ __host__ __device__ inline void gc_child32(const float* p, int c, float* out) {
 }
 
 // Shared state of one warp of k_vm_walk.
-template <int D>
 struct VmWarp {
-  static constexpr int NC = D == 3 ? 8 : 4;
+  static constexpr int NC = 4;
   double s1[NC][NC];        // cut level-1 nodes (FP64 corners)
   double anc[NC * NC][NC];  // cut level-2 nodes, the anchors (FP64 corners)
   float th[NC * NC], thc[NC * NC];
@@ -465,16 +464,15 @@ struct VmWarp {
 // the FP64 sum.  A child with a corner (or a corner sum) inside the bound
 // takes its corners from the FP64 refinements along its path from the
 // anchor, as the reference computes them.
-template <int D>
 __global__ void __launch_bounds__(128) k_vm_walk(const int* __restrict__ item_cell, const double* __restrict__ item_cor,
                                                  long long nitem, unsigned* __restrict__ units) {
-  constexpr int NC = D == 3 ? 8 : 4, NR = D == 3 ? 27 : 9, LB = D == 3 ? 3 : 2, NB = 32 / NC;
+  constexpr int D = 2, NC = 4, NR = 9, LB = 2, NB = 32 / NC;
   constexpr unsigned FULL = 0xffffffffu;
-  __shared__ VmWarp<D> smem[4];
+  __shared__ VmWarp smem[4];
   const int wid = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const long long it = (long long)blockIdx.x * 4 + wid;
   if (it >= nitem) return;  // whole warps
-  VmWarp<D>& S = smem[wid];
+  VmWarp& S = smem[wid];
   const unsigned below = (1u << lane) - 1u;
   double root[NC];
   for (int q = 0; q < NC; q++) root[q] = item_cor[it * NC + q];
@@ -650,7 +648,7 @@ struct VmLine {
 };
 
 // direct interpolation at (x, y, z) in units of 1/128 of the sub-cube
-__device__ __noinline__ double vm_point64(const double* c, int x, int y, int z) {
+__host__ __device__ __noinline__ double vm_point64(const double* c, int x, int y, int z) {
   const double tx = x * 0x1p-7, ty = y * 0x1p-7, tz = z * 0x1p-7;
   double v[4];
   for (int q = 0; q < 4; q++) v[q] = c[q] + tx * (c[4 + q] - c[q]);
@@ -1264,7 +1262,7 @@ cudaError_t ls_volume_mass(const LsSet& ls, int level, int D, double* cvol, doub
       if (ni > 0) {
         const long long nbi = ((long long)ni + 3) / 4;  // one warp per cut sub-cube
         if (D == 3) k_vm_columns<<<(unsigned)nbi, 32 * kVmWarps, 0, s>>>(item_cell, item_cor, (long long)ni, units);
-        else k_vm_walk<2><<<(unsigned)nbi, 128, 0, s>>>(item_cell, item_cor, (long long)ni, units);
+        else k_vm_walk<<<(unsigned)nbi, 128, 0, s>>>(item_cell, item_cor, (long long)ni, units);
       }
       k_vm_finish<<<(unsigned)((nl + 255) / 256), 256, 0, s>>>(list, nl, units, mark, dv, cvol);
       e = cudaStreamSynchronize(s);

@@ -293,8 +293,8 @@ __device__ double tet_aspect(const TetGeo& g, const Pt* P) {
 constexpr int kMaxStar = 128;  // tets around one particle
 constexpr int kMaxLink = 224;  // link edges around one particle
 constexpr int kMaxOut = kMaxStar;  // tets emitted by one particle (at most its star)
-// flags: 2 emit overflow, 4 spilled neighbour row (a star that outgrows
-// kMaxStar / kMaxLink stops its walk and is counted in stats[3])
+// flags: 4 spilled neighbour row (a star that outgrows kMaxStar / kMaxLink stops
+// its walk and is counted in stats[3])
 
 constexpr unsigned kFull = 0xffffffffu;
 
@@ -559,8 +559,7 @@ constexpr int kStarWarps = 4;  // warps (particles) per block of k_tet_star
 // Four blocks of four warps per SM (128 registers): 7.5 ms for 150,001
 // particles, 10.6 ms at six blocks (spills), 7.9 ms at three.
 __global__ void __launch_bounds__(32 * kStarWarps, 4) k_tet_star(TetIn T, int* __restrict__ out,
-                                                              int* __restrict__ count, unsigned long long* stats,
-                                                              unsigned* flags) {
+                                                              int* __restrict__ count, unsigned long long* stats) {
   __shared__ Star s_star[kStarWarps];
   const int wib = threadIdx.x >> 5, lane = threadIdx.x & 31;
   Star& sm = s_star[wib];
@@ -1069,7 +1068,7 @@ extern "C" int mrsph_tetrahedralize(mrsph_handle* h, int* tets, long long cap, l
     TetIn T;
     T.n = n; T.cap = rowcap; T.x = d_x; T.type = d_type; T.h = d_h; T.rf = d_rf; T.rows = d_rows; T.cnt = d_cnt;
     T.inv_g = inv_g; T.cutoff = h->prm.cutoff; T.thres = 10.0;
-    k_tet_star<<<nbN, 32 * kStarWarps, 0, s>>>(T, d_out, d_count, d_stats, d_flags);
+    k_tet_star<<<nbN, 32 * kStarWarps, 0, s>>>(T, d_out, d_count, d_stats);
     cell_scan(d_count, d_off, d_blk, n, 0, s);
     int tot = 0, last = 0;
     cudaMemcpyAsync(&tot, d_off + n - 1, sizeof(int), cudaMemcpyDeviceToHost, s);
@@ -1079,7 +1078,6 @@ extern "C" int mrsph_tetrahedralize(mrsph_handle* h, int* tets, long long cap, l
     if (cudaStreamSynchronize(s) != cudaSuccess) { rc = tfail(h, MRSPH_ERR_CUDA, "tetrahedralisation failed"); goto done; }
     ntet = (long long)tot + last;
     if (flags & 4u) { rc = tfail(h, MRSPH_ERR_RANGE, "neighbour list spilled; raise neighbor_cap"); goto done; }
-    if (flags & 2u) { rc = tfail(h, MRSPH_ERR_RANGE, "a particle emits more tets than the kernel keeps"); goto done; }
     if (ntet > 0) {
       if (!A((void**)&d_tets, sizeof(int) * 4 * ntet)) { rc = tfail(h, MRSPH_ERR_OOM, "cudaMalloc failed"); goto done; }
       k_tet_compact<<<(int)((n + 255) / 256), 256, 0, s>>>(n, d_out, d_count, d_off, d_tets);
