@@ -1,7 +1,9 @@
 // engine.cuh — the relaxation step as CUDA kernels, templated on dimension D
 // and arithmetic type R (double: FP64-plain, float: FP32-split).  Included by
-// mrsph_fp64.cu (compiled without FMA contraction so FP64 results follow the
-// reference's operation order) and mrsph_fp32.cu.
+// mrsph_fp64.cu (compiled without FMA contraction: FP64 follows the reference's
+// operation order but for the Wendland gradient and the kernel sum, whose
+// divisions share one reciprocal, kernel_dW and quot, within 1e-12 of the
+// reference's value) and mrsph_fp32.cu.
 //
 // One step (SPH_mesh_generation::SPH_run_mesh_generation,
 // sph_mesh_generation.cpp:1371-1463) is 11 launches on one stream (15 where the

@@ -213,11 +213,12 @@ __device__ inline R kernel_C(int kind, int D, R h) {
   if (D == 2) return (R)1.0 / PI * (R)7. / (R)478. / powern(h, 2);
   return (R)1.0 / PI * (R)3. / (R)359. / powern(h, 3);
 }
-// a / b from an approximation ib of 1 / b, corrected by its residual (within one
-// unit in the last place)
-__device__ inline double quot(double a, double b, double ib) {
+// a / b from ib, 1 / b to a few units in the last place: one Newton step on
+// b q = a, its remainder by a fused multiply-add (P. Markstein, IBM J. Res. Dev.
+// 34, 1990), which leaves q within one unit in the last place
+__host__ __device__ inline double quot(double a, double b, double ib) {
   const double q = a * ib;
-  return __fma_rn(__fma_rn(-b, q, a), ib, q);
+  return fma(fma(-b, q, a), ib, q);
 }
 // W given s = dist / h and C = kernel_C(kind, D, h)
 template <class R>
@@ -455,8 +456,6 @@ __device__ inline float kernel_dW_fast(int kind, int D, float dist, float h) {
 }
 
 // path dispatch: FP64 keeps the reference arithmetic
-__device__ inline double pair_W(int kind, int D, double dist, double h, double) { return kernel_W<double>(kind, D, dist, h); }
-__device__ inline float pair_W(int kind, int D, float dist, float, float inv_h) { return kernel_W_fast(kind, D, dist, inv_h); }
 __device__ inline double pair_dW(int kind, int D, double dist, double h) { return kernel_dW<double>(kind, D, dist, h); }
 __device__ inline float pair_dW(int kind, int D, float dist, float h) { return kernel_dW_fast(kind, D, dist, h); }
 
