@@ -306,7 +306,7 @@ constexpr unsigned kFull = 0xffffffffu;
 // Lengths are taken in units of the power of two at the radius of i's ball: up
 // to six of them are multiplied, and in the body's own units a spacing of 3e-8
 // would already leave FP32's range.  Points far closer to one another than to
-// the ball's size can still do so: what has come below 1e-30 decides nothing.
+// the ball's size can still do so: products that come near it decide nothing.
 // FP64 runs at 1/60 of the FP32 rate on this part: with the candidates' FP64
 // differences, an FP64 circumcentre per tet and a second scan of the row per
 // tet the pass took 142.9 ms for 150,001 particles (830,000 tets); in this
@@ -368,8 +368,9 @@ struct Face {  // the pencil of spheres through i, u, v: centres c0 + sigma t n
 // B 8), n . w by 8 e |A||B||w|, the power |w|^2 - 2 w . c0 by e (8 |w|^2 + 48 k^2 L |w|).
 // The constants below are at least a third larger.  They are relative to the
 // products they bound, so a face whose products come near FP32's smallest numbers
-// has no bound.
-constexpr float kTiny = 1.e-30f;
+// has no bound: |n|^2 above 1e-22 keeps both lengths above 1e-12 (rows reach a few
+// radii of the ball), and no bound on n . w is one on nothing else either.
+constexpr float kTiny = 1.e-22f;
 __device__ inline Face face_of(const float4& A4, const float4& B4, float sigma) {
   Face F;
   const V3 A{A4.x, A4.y, A4.z}, B{B4.x, B4.y, B4.z};
@@ -382,10 +383,9 @@ __device__ inline Face face_of(const float4& A4, const float4& B4, float sigma) 
   F.nn = sqrtf(n2);
   const float ab = A4.w * B4.w, k = ab / F.nn;
   F.L = A4.w + B4.w;
-  F.cO = 16.f * kE * ab;
+  F.cO = n2 > kTiny ? 16.f * kE * ab : __int_as_float(0x7f800000);
   F.cP = 64.f * kE * k * k * F.L;
   F.dc0 = 32.f * kE * k * k * F.L;
-  if (!(n2 > kTiny) || !(fminf(A4.w, B4.w) > 1.e-12f)) F.cO = F.cP = F.dc0 = __int_as_float(0x7f800000);
   return F;
 }
 
@@ -620,8 +620,8 @@ __global__ void __launch_bounds__(32 * kStarWarps, 4) k_tet_star(TetIn T, int* _
         // |v - u| relative to its own rounding: d3 is off by at most 3 e (|u| + |v|)
         const float rd = 8.f * kE * (u4.w + w.w) / sqrtf(dd);
         const float er = rel + 2.f * rd;
-        const bool tiny = !(xx > kTiny) || !(uu * vv > kTiny) || !(top > kTiny);
-        if (tiny || !(er < 0.25f) || !(r2 < 3.e38f) || !(xx < 3.e38f)) { lo = floor_; hi = INF; }
+        // (top above 1e-17 keeps |u||v| above 1e-10, and er below 1/4 then |u x v|^2 above 1e-30)
+        if (!(top > 1.e-17f) || !(er < 0.25f) || !(r2 < 3.e38f)) { lo = floor_; hi = INF; }
         else { lo = fmaxf(r2 * (1.f - 2.f * er), floor_); hi = r2 * (1.f + 2.f * er); }
         return true;
       };
