@@ -486,9 +486,9 @@ def run_mrsph(args, ws, rank, local, dist):
             "traffic": (tr * n if tr is not None else None),
             "issue": {"issue_active_frac": ns.get("issue_active_pct", 0.0) / 100.0 or None,
                       "fp32_fma_pipe_frac": ns.get("fma_pipe_pct", 0.0) / 100.0 or None,
-                      "source": "ncu --set full of the same kernel on the 301,270-particle torus "
-                                "(profiles/density_torus_3d_small.md): the kernel is issue-bound, so its "
-                                "instruction-issue and FP32-pipe fractions bound it, not HBM"},
+                      "source": "ncu of the same kernel on the 301,270-particle torus "
+                                "(profiles/neighbour_passes_torus_3d_small.md): the kernel is bound by issue at "
+                                "the few warps its tiles leave room for, not by HBM"},
             "algorithmic_bytes_per_launch": bytes_[top],
             "step_achieved": step_ach, "step_frac": step_ach / peak,
             "step_bytes_per_particle": roofline.total_bytes_per_particle(dim, "fp32")}
