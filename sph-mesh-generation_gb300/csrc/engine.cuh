@@ -155,6 +155,9 @@ struct Forms {
 // full, at three times the instructions; so what counts is total, the particles of
 // all handles that step at the same time (n: this handle's).  Force passes: stage
 // 1 of 20,000 in 3D 37 us by groups, 67 by lanes, of 77,551 in 2D 39 and 26.
+// In FP64 the line lies higher in 3D (seeded graded bodies, ms: 41,000 3.08 and 4.11,
+// 160,000 8.91 and 10.20) and about there in 2D (50,000 0.299 and 0.315 in stage 1, 0.180
+// and 0.138 in stage 2).
 // Lists, by levels of the cell list and by row length (dense: more than kDenseRow
 // neighbours on average, as uniformly seeded bodies have), us of 4 steps with
 // upload and download, groups / lanes / tiles / tiles in brick order:
